@@ -143,7 +143,7 @@ mts_status mts_get_solution(mts_handle h, double* u);
  *   LOD::Solve_2nd(eq(t_next), inter, uh, beta, 'I'|'C')   lod.cc:44-205
  *   TS::Solve_2nd(eq(t_prev), eq(t_half), eq(t_next), ...)  trapezoidal.cc:46-272
  * t_prev and t_half are read by TS only.  Refresh_Jump (intersection.cc:
- * 2294-2490) runs on the device inside the step.  Asynchronous. */
+ * 2294-2490) is evaluated inside the step's kernels where it is read.  Asynchronous. */
 mts_status mts_solve_2nd(mts_handle h, double t_prev, double t_half, double t_next);
 
 /* nsteps steps of the time loop of src/helper.h:199-238 (t += dt before each
@@ -155,8 +155,8 @@ mts_status mts_advance(mts_handle h, int32_t nsteps);
  * kernel of the step for all of them (each CTA carries its problem and its
  * place in that problem's grid), and so do the mixed-precision Douglas-ADI
  * handles whose lines have at most 160 rows, in a group of their own;
- * handles whose lines fill the GPU (256 per SM in every direction),
- * fast-form handles and longer-line mixed ones step on their own streams
+ * handles whose lines fill the GPU (256 per SM in every direction) or are
+ * longer than a batched tile takes (232 rows), fast-form handles and longer-line mixed ones step on their own streams
  * alongside, and the groups run at once on their own streams.  Each
  * handle's result and time are those of mts_advance(h, nsteps), bit for
  * bit.  Handles must be distinct, on one
@@ -257,16 +257,16 @@ mts_status mts_get_stream(mts_handle h, void** stream);
 
 /* Per-kernel timing with CUDA events recorded on the handle's stream around
  * every launch of a step (negligible overhead; off by default).  Slots, in
- * launch order: Douglas-ADI and LOD {0 jumps, 1 x sweep, 2 y sweep, 3 z sweep};
- * TS {0 jumps, 1 explicit x, 2 explicit y, 3 z sweep, 4 y sweep, 5 x sweep}.
+ * launch order: Douglas-ADI {0 empty, 1 MIB rows (mixed: residual), 2 x sweep,
+ * 3 y sweep, 4 z sweep}; LOD {0 empty, 1 x sweep, 2 y sweep, 3 z sweep}; TS
+ * {0 empty, 1 explicit x, 2 explicit y, 3 z sweep, 4 y sweep, 5 x sweep}.
  * mts_profile_read synchronizes, returns the summed milliseconds and launch
  * counts per slot since the last read, and resets them. */
 mts_status mts_set_profiling(mts_handle h, int32_t on);
 mts_status mts_profile_read(mts_handle h, double ms[8], int64_t launches[8]);
 
-/* Launch shape of the persistent line-sweep kernels (rows staged per chunk,
- * staging-ring depth, threads per CTA), chosen separately for the first,
- * second and third implicit sweep of a step.  Every shape computes the same
+/* Launch shape of the line-sweep kernels (lines per tile, threads per CTA),
+ * chosen separately for the first, second and third implicit sweep of a step.  Every shape computes the same
  * bits; they differ only in speed.  mts_autotune times each compiled shape on
  * the handle's own problem for `steps` steps (the solution and time are
  * restored afterwards) and keeps the fastest per sweep; shapes[3] receives

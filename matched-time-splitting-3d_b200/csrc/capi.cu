@@ -397,13 +397,14 @@ mts_status finish_create(mts_problem* h) {
     h->nblk[d] = (int64_t)blocks[d].size();
   }
   // Thomas factorisation (the factor half of TDMA, douglas_adi.cc:1790-1798:
-  // gam_j = c_{j-1}/bet, bet = b_j - a_j*gam_j, same operations): prefix
-  // tables per direction and row-1 side here; the per-node factors of the
-  // lines that cross the interface, from their first MIB row on, are
-  // computed on the device once the tables are there (launch_factor_lines).
-  std::vector<double> ptab[3][2];
+  // gam_j = c_{j-1}/bet, bet = b_j - a_j*gam_j, same operations): row
+  // tables per direction and row-1 side here; the factors of the lines that
+  // cross the interface are computed on the device (launch_factor_lines).
+  std::vector<double2> tab[3][2];
+  std::vector<double> taba[3][2], tabg[3][2];
+  const int nd[3] = {g.nx, g.ny, g.nz};
   {
-    const int n[3] = {g.nx, g.ny, g.nz};
+    const int* const n = nd;
     std::vector<double> a, b, c;
     auto factor = [&](int len, std::vector<double>& bet_out, std::vector<double>& gam_out) -> bool {
       bet_out.resize(len);
@@ -437,10 +438,13 @@ mts_status finish_create(mts_problem* h) {
         b[len - 1] = 1.0;
         c[len - 1] = 0.0;
         if (!factor(len, lb, lg)) return fail(MTS_ERR_ZERO_PIVOT, "zero pivot in a line factorisation");
-        ptab[d][side].resize(2 * (size_t)len);
+        tab[d][side].resize((size_t)len);
+        tabg[d][side].resize((size_t)len);
+        taba[d][side] = a;
         for (int j = 0; j < len; j++) {
-          ptab[d][side][2 * j] = lb[j];
-          ptab[d][side][2 * j + 1] = lg[j];
+          tab[d][side][j] = make_double2(lb[j], 1.0 / lb[j]);
+          if (!(std::fabs(lb[j]) >= 0x1p-100 && std::fabs(lb[j]) <= 0x1p100)) D.plain_div = 1;
+          tabg[d][side][j] = j + 1 < len ? lg[j + 1] : 0.0;
         }
       }
     }
@@ -466,6 +470,31 @@ mts_status finish_create(mts_problem* h) {
           lside[d][(size_t)i1 * n2 + i2] = (uint8_t)(out_at(0) | (out_at(1) << 1) | (out_at(n[d] - 1) << 2));
         }
     }
+  }
+  // the lines that cross the interface, in memory order (the fast line index
+  // first), and each line's index in that list
+  std::vector<int32_t> clist[3], cline[3], lperm[3];
+  for (int d = 0; d < 3; d++) {
+    const int n1 = d == 0 ? g.ny : g.nx, n2 = d == 2 ? g.ny : g.nz;
+    // (the order of the bit-exact sweeps: crossing, inside, outside)
+    lperm[d].reserve((size_t)(n1 - 2) * (n2 - 2));
+    for (int kind = 0; kind < 3; kind++)
+      for (int i2 = 1; i2 < n2 - 1; i2++)
+        for (int i1 = 1; i1 < n1 - 1; i1++) {
+          const size_t l = (size_t)i1 * n2 + i2;
+          const int kd = bstart[d][l + 1] > bstart[d][l] ? 0 : 1 + ((lside[d][l] >> 1) & 1);
+          if (kd == kind) lperm[d].push_back(i1 + n1 * i2);
+        }
+    if (blocks[d].empty()) continue;
+    cline[d].assign((size_t)line_count(g, d), -1);
+    for (int i2 = 0; i2 < n2; i2++)
+      for (int i1 = 0; i1 < n1; i1++) {
+        const size_t l = (size_t)i1 * n2 + i2;
+        if (bstart[d][l + 1] > bstart[d][l]) {
+          cline[d][(size_t)i1 + (size_t)n1 * i2] = (int32_t)clist[d].size();
+          clist[d].push_back((int32_t)l);
+        }
+      }
   }
   for (size_t i = 0; i < h->cross.size(); i++) {
     const mts_crossing& c = h->cross[i];
@@ -510,34 +539,17 @@ mts_status finish_create(mts_problem* h) {
   int sms = 0;
   CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
   D.sweep_blocks = sms > 0 ? sms : 1;
-  // sweep threads of a launch: one CTA per SM at most and no more CTAs than
-  // the lines of a direction need, so at most max lines + one CTA
   long long maxlines = 0;
   for (int d = 0; d < 3; d++) maxlines = std::max(maxlines, (long long)line_count(g, d));
-  const size_t tmax = std::min((size_t)D.sweep_blocks * (size_t)mts::sweep_shape_max_threads(),
-                               (size_t)maxlines + (size_t)mts::sweep_shape_max_threads());
   const int nmax = std::max(g.nx, std::max(g.ny, g.nz));
-  {
-    // default shapes: when the lines fill the GPU, 4 rows x 4 chunks with 384
-    // threads for x and y lines and 448 for z lines (the shapes mts_autotune
-    // picks at 257^3, 23 % faster per step than 8 x 4 x 256 there); the small
-    // shape 9 (several CTAs per SM, for concurrent small problems) when they
-    // do not; mts_autotune picks per problem.  TS runs its sweeps z, y, x.
-    const bool large = maxlines >= (long long)D.sweep_blocks * 256;
-    const int by_dir[3] = {large ? 6 : 9, large ? 6 : 9, large ? 8 : 9};  // x, y, z
-    const int dir_of_sweep[3] = {p.method == MTS_TS ? 2 : 0, 1, p.method == MTS_TS ? 0 : 2};
-    for (int k = 0; k < 3; k++) {
-      const int want = by_dir[dir_of_sweep[k]];
-      int def = -1;
-      for (int s = mts::sweep_shape_count() - 1; s >= 0; s--)
-        if (mts::sweep_shape_fits(s, nmax) && (def < 0 || s == want)) def = s;
-      if (def < 0) return fail(MTS_ERR_ARG, "grid lines too long for the sweep kernels' shared memory");
-      D.shape[k] = def;
-    }
+  for (int k = 0; k < 3; k++) {
+    // (mts_autotune picks per problem and sweep)
+    D.shape[k] = mts::sweep_shape_default(nmax);
+    if (D.shape[k] < 0) return fail(MTS_ERR_ARG, "grid lines too long for the sweep kernels' shared memory");
   }
   CUDA_TRY(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
-  // row slack of the fields the sweeps stage whole chunks of: kRowPad rows of
-  // the largest stride (an x-y plane)
+  // row slack of the fields that are staged past their last row: kRowPad rows
+  // of the largest stride (an x-y plane)
   const size_t fpad = (size_t)mts::kRowPad * (size_t)g.nx * (size_t)g.ny;
   // nodes that are a MIB row of some block: the pointwise passes leave them
   // to a per-node pass over this list
@@ -552,37 +564,49 @@ mts_status finish_create(mts_problem* h) {
     CUDA_TRY(h->put_padded(&h->u1, (const double*)nullptr, (size_t)N, fpad));
     D.u0 = h->u0;
     D.u1 = h->u1;
-    CUDA_TRY(h->put_padded(&D.dp, (const double*)nullptr, (size_t)nmax * tmax, (size_t)mts::kRowPad * tmax));
     for (int d = 0; d < 3; d++) {
       for (int side = 0; side < 2; side++) {
-        double* pt = nullptr;
-        CUDA_TRY(h->put(&pt, ptab[d][side].data(), ptab[d][side].size()));
-        D.ptab[d][side] = pt;
+        double2* pt = nullptr;
+        double *pa = nullptr, *pg = nullptr;
+        CUDA_TRY(h->put(&pa, taba[d][side].data(), taba[d][side].size()));
+        D.taba[d][side] = pa;
+        CUDA_TRY(h->put(&pt, tab[d][side].data(), tab[d][side].size()));
+        CUDA_TRY(h->put(&pg, tabg[d][side].data(), tabg[d][side].size()));
+        D.tab[d][side] = pt;
+        D.tabg[d][side] = pg;
       }
-      double* rbk = nullptr;
-      CUDA_TRY(h->put(&rbk, (const double*)nullptr, 3 * blocks[d].size()));
-      D.rblk[d] = rbk;
       D.nblk[d] = (int)blocks[d].size();
-      // per-node factor fields of the crossing lines (zero elsewhere), FP64
-      // and, for the mixed form, FP32 (1/bet and gam): filled on the device
-      double *fb = nullptr, *fg = nullptr;
+      // the crossing lines' factors, filled on the device; for the mixed
+      // form's ring sweeps 1/bet and gam per node in FP32 too
       float *fb32 = nullptr, *fg32 = nullptr;
       if (!blocks[d].empty()) {
-        CUDA_TRY(h->put_padded(&fb, (const double*)nullptr, (size_t)N, fpad));
-        CUDA_TRY(h->put_padded(&fg, (const double*)nullptr, (size_t)N, fpad));
-        CUDA_TRY(h->put_padded(&fb32, (const float*)nullptr, (size_t)N, fpad));
-        CUDA_TRY(h->put_padded(&fg32, (const float*)nullptr, (size_t)N, fpad));
+        int32_t *dl = nullptr, *dc = nullptr;
+        double *ca = nullptr, *cg = nullptr;
+        double2* cb = nullptr;
+        CUDA_TRY(h->put(&dl, clist[d].data(), clist[d].size()));
+        CUDA_TRY(h->put(&dc, cline[d].data(), cline[d].size()));
+        CUDA_TRY(h->put(&ca, (const double*)nullptr, clist[d].size() * (size_t)nd[d]));
+        CUDA_TRY(h->put(&cb, (const double2*)nullptr, clist[d].size() * (size_t)nd[d]));
+        CUDA_TRY(h->put(&cg, (const double*)nullptr, clist[d].size() * (size_t)nd[d]));
+        D.fcross[d] = dl;
+        D.cline[d] = dc;
+        D.ca[d] = ca;
+        D.cb[d] = cb;
+        D.cg[d] = cg;
+        if (!mts::mixed_segments_fit(nmax)) {
+          CUDA_TRY(h->put_padded(&fb32, (const float*)nullptr, (size_t)N, fpad));
+          CUDA_TRY(h->put_padded(&fg32, (const float*)nullptr, (size_t)N, fpad));
+        }
       }
-      D.fbet[d] = fb;
-      D.fgam[d] = fg;
+      D.nfcross[d] = (int)clist[d].size();
       D.fib32[d] = fb32;
       D.fgam32[d] = fg32;
       // the same factors in FP32 for the mixed-precision sweeps, as 1/bet and gam
       for (int side = 0; side < 2; side++) {
-        std::vector<float> p32(ptab[d][side].size());
-        for (size_t j = 0; j + 1 < p32.size(); j += 2) {
-          p32[j] = (float)(1.0 / ptab[d][side][j]);
-          p32[j + 1] = (float)ptab[d][side][j + 1];
+        std::vector<float> p32(2 * tab[d][side].size());
+        for (size_t j = 0; j < tab[d][side].size(); j++) {
+          p32[2 * j] = (float)tab[d][side][j].y;
+          p32[2 * j + 1] = (float)(j ? tabg[d][side][j - 1] : 0.0);
         }
         float* pt = nullptr;
         CUDA_TRY(h->put(&pt, p32.data(), p32.size()));
@@ -609,11 +633,17 @@ mts_status finish_create(mts_problem* h) {
       CUDA_TRY(h->put(&dm, mibn.empty() ? nullptr : mibn.data(), mibn.size()));
       D.mibnode = dm;
       D.nmibnode = (int)mibn.size();
+      int4* ref = nullptr;
+      if (p.method == MTS_ADI && !mibn.empty()) CUDA_TRY(h->put(&ref, (const int4*)nullptr, mibn.size()));
+      D.mibref = ref;
     }
     for (int d = 0; d < 3; d++) {
       uint8_t* ls = nullptr;
       CUDA_TRY(h->put(&ls, lside[d].data(), lside[d].size()));
       D.lside[d] = ls;
+      int32_t* lp = nullptr;
+      CUDA_TRY(h->put(&lp, lperm[d].data(), lperm[d].size()));
+      D.lperm[d] = lp;
     }
     for (int d = 0; d < 3; d++) {
       double *a = nullptr, *s = nullptr, *c = nullptr;
@@ -633,7 +663,6 @@ mts_status finish_create(mts_problem* h) {
     mts::CrossConst* dcc = nullptr;
     CUDA_TRY(h->put(&dcc, cc.empty() ? nullptr : cc.data(), cc.size()));
     D.cc = dcc;
-    CUDA_TRY(h->put(&D.jv, (const double2*)nullptr, h->cross.size()));
     CUDA_TRY(h->put(&D.status, (const int*)nullptr, 1));
     CUDA_TRY(h->put(&h->norm_part, (const double*)nullptr, (size_t)3 * h->norm_nb));
     CUDA_TRY(h->put(&h->norm_out, (const double*)nullptr, 3));
@@ -649,13 +678,14 @@ mts_status finish_create(mts_problem* h) {
   if (placed) return placed;
   CUDA_TRY(cudaMemsetAsync(D.status, 0, sizeof(int), h->stream));
   {
-    // the crossing lines' per-node factors; a zero pivot raises D.status
+    // the crossing lines' factors
     mts::launch_factor_lines(D, D.status, h->stream);
     CUDA_TRY(cudaGetLastError());
-    int zero_pivot = 0;
-    CUDA_TRY(cudaMemcpyAsync(&zero_pivot, D.status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    int flags = 0;
+    CUDA_TRY(cudaMemcpyAsync(&flags, D.status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     CUDA_TRY(cudaStreamSynchronize(h->stream));
-    if (zero_pivot) return fail(MTS_ERR_ZERO_PIVOT, "zero pivot in a line factorisation");
+    if (flags & 1) return fail(MTS_ERR_ZERO_PIVOT, "zero pivot in a line factorisation");
+    if (flags & 2) D.plain_div = 1;
     CUDA_TRY(cudaMemsetAsync(D.status, 0, sizeof(int), h->stream));
   }
   CUDA_TRY(cudaStreamSynchronize(h->stream));
@@ -727,7 +757,7 @@ mts_status enqueue_step(mts_problem* h, double t_prev, double t_half, double t_n
   else if (h->dev.precision == 1)
     h->launches += mts::launch_step_mixed(h->dev, T, h->u0, h->stream, ev, &h->side);
   else
-    h->launches += mts::launch_step(h->dev, T, h->u0, h->u1, h->stream, ev, &h->side);
+    h->launches += mts::launch_step(h->dev, T, h->u0, h->u1, h->stream, ev);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(MTS_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(e));
   h->t = t_next;
@@ -1007,8 +1037,12 @@ mts_status mts_batch_advance_steps(const mts_handle* hs, const int32_t* counts, 
       if (mts::mixed_batch_class(h->dev, d) < 0) return false;
     return true;
   };
+  // plain ones whose lines' tiles let an SM hold a few
+  auto plain_batchable = [&](const mts_problem* h) {
+    return mts::batch_lines_fit(std::max(h->g.nx, std::max(h->g.ny, h->g.nz)));
+  };
   auto solo = [&](int i) {
-    return fills_gpu(hs[i]) || (hs[i]->dev.precision != 0 && !mixed_batchable(hs[i]));
+    return fills_gpu(hs[i]) || (hs[i]->dev.precision != 0 ? !mixed_batchable(hs[i]) : !plain_batchable(hs[i]));
   };
   // plain handles by method: one batched launch sequence per group
   for (int method = 0; method < 4; method++) {
@@ -1023,7 +1057,7 @@ mts_status mts_batch_advance_steps(const mts_handle* hs, const int32_t* counts, 
     mts::BatchPlan plan{};
     plan.method = method;
     plan.n = (int)mem.size();
-    std::vector<mts::BatchItem> jumps, rows, mib, blk[3], sw[3];
+    std::vector<mts::BatchItem> rows, mib, sw[3];
     auto add = [](std::vector<mts::BatchItem>& v, int p, unsigned ncta) {
       for (unsigned c = 0; c < ncta; c++) v.push_back(mts::BatchItem{p, (int32_t)c, (int32_t)ncta, 0});
     };
@@ -1031,13 +1065,9 @@ mts_status mts_batch_advance_steps(const mts_handle* hs, const int32_t* counts, 
       const mts::Dev& d = hs[mem[(size_t)k]]->dev;
       recs.push_back(d);
       plan.nmax = std::max(plan.nmax, std::max(d.nx, std::max(d.ny, d.nz)));
-      if (d.ncross > 0) add(jumps, k, mts::jumps_grid(d));
-      add(rows, k, mts::pointwise_rows_grid(d));
-      if (d.nmibnode > 0) add(mib, k, mts::mib_grid(d));
-      for (int dd = 0; dd < 3; dd++) {
-        if (d.nblk[dd] > 0) add(blk[dd], k, mts::block_grid(d, dd));
-        add(sw[dd], k, mts::batch_sweep_grid(d, dd));
-      }
+      if (method == MTS_TS) add(rows, k, mts::ts_explicit_grid(d));
+      if (method == MTS_ADI && d.nmibnode > 0) add(mib, k, mts::mib_grid(d));
+      for (int dd = 0; dd < 3; dd++) add(sw[dd], k, mts::batch_sweep_grid(d, dd));
     }
     void* tmp = nullptr;
     BATCH_TRY(dev_upload(recs.data(), recs.size() * sizeof(mts::Dev), q, &tmp));
@@ -1049,13 +1079,9 @@ mts_status mts_batch_advance_steps(const mts_handle* hs, const int32_t* counts, 
       *dst = (const mts::BatchItem*)p;
       return e;
     };
-    BATCH_TRY(up(jumps, &plan.jumps, &plan.njumps));
     BATCH_TRY(up(rows, &plan.rows, &plan.nrows));
     BATCH_TRY(up(mib, &plan.mib, &plan.nmib));
-    for (int dd = 0; dd < 3; dd++) {
-      BATCH_TRY(up(blk[dd], &plan.blk[dd], &plan.nblk[dd]));
-      BATCH_TRY(up(sw[dd], &plan.sw[dd], &plan.nsw[dd]));
-    }
+    for (int dd = 0; dd < 3; dd++) BATCH_TRY(up(sw[dd], &plan.sw[dd], &plan.nsw[dd]));
     // the host vectors must outlive the asynchronous uploads
     BATCH_TRY(cudaStreamSynchronize(q));
     int gsteps = 0;  // the group's longest count: later steps skip finished problems
@@ -1077,14 +1103,13 @@ mts_status mts_batch_advance_steps(const mts_handle* hs, const int32_t* counts, 
       std::vector<mts::Dev> recs;
       mts::MixedBatchPlan plan{};
       plan.n = (int)mem.size();
-      std::vector<mts::BatchItem> jumps, rows, mib, blk[3], line[3][2];
+      std::vector<mts::BatchItem> rows, mib, blk[3], line[3][2];
       auto add = [](std::vector<mts::BatchItem>& v, int p, unsigned ncta) {
         for (unsigned c = 0; c < ncta; c++) v.push_back(mts::BatchItem{p, (int32_t)c, (int32_t)ncta, 0});
       };
       for (int k = 0; k < (int)mem.size(); k++) {
         const mts::Dev& d = hs[mem[(size_t)k]]->dev;
         recs.push_back(d);
-        if (d.ncross > 0) add(jumps, k, mts::jumps_grid(d));
         add(rows, k, mts::pointwise_rows_grid(d));
         if (d.nmibnode > 0) add(mib, k, mts::mib_grid(d));
         for (int dd = 0; dd < 3; dd++) {
@@ -1102,7 +1127,6 @@ mts_status mts_batch_advance_steps(const mts_handle* hs, const int32_t* counts, 
         *dst = (const mts::BatchItem*)p;
         return e;
       };
-      BATCH_TRY(up(jumps, &plan.jumps, &plan.njumps));
       BATCH_TRY(up(rows, &plan.rows, &plan.nrows));
       BATCH_TRY(up(mib, &plan.mib, &plan.nmib));
       for (int dd = 0; dd < 3; dd++) {
@@ -1130,7 +1154,7 @@ mts_status mts_batch_advance_steps(const mts_handle* hs, const int32_t* counts, 
       else if (h->dev.precision == 1)
         h->launches += mts::launch_step_mixed(h->dev, T, h->u0, h->stream, nullptr, &h->side);
       else
-        h->launches += mts::launch_step(h->dev, T, h->u0, h->u1, h->stream, nullptr, &h->side);
+        h->launches += mts::launch_step(h->dev, T, h->u0, h->u1, h->stream, nullptr);
       mts::launch_tick(h->dev, h->stream);
       h->launches++;
     }
@@ -1453,9 +1477,8 @@ mts_status mts_set_precision(mts_handle h, int32_t precision) {
     if (!mts::fast_fits(h->g.nx, h->g.ny, h->g.nz))
       return fail(MTS_ERR_ARG, "grid lines too long for the fast FP64 form (at most 544 nodes per axis)");
     if (!h->fast_built) {
-      // row tables, line flags, the crossing lines' list and coefficients,
-      // the block rows' q and the MIB nodes' block references, once per
-      // handle
+      // row tables, line flags, the crossing lines' coefficients, the block
+      // rows' q, once per handle
       mts::Dev& D = h->dev;
       const int nd[3] = {h->g.nx, h->g.ny, h->g.nz};
       uint8_t* fl[3] = {nullptr, nullptr, nullptr};
@@ -1471,37 +1494,16 @@ mts_status mts_set_precision(mts_handle h, int32_t precision) {
       CUDA_TRY(cudaGetLastError());
       for (int d = 0; d < 3; d++) {
         const size_t R = 32 * (size_t)mts::fast_rows_per_lane(nd[d]);
-        const size_t nl = (size_t)line_count(h->g, d);
-        std::vector<uint8_t> hf(nl);
-        CUDA_TRY(cudaMemcpyAsync(hf.data(), fl[d], nl, cudaMemcpyDeviceToHost, h->stream));
-        CUDA_TRY(cudaStreamSynchronize(h->stream));
-        // listed in memory order (the fast line index first), so that the
-        // warps that take neighbouring entries read neighbouring lines
-        const int n1 = d == 0 ? h->g.ny : h->g.nx, n2 = d == 2 ? h->g.ny : h->g.nz;
-        std::vector<int32_t> list;
-        for (int i2 = 0; i2 < n2; i2++)
-          for (int i1 = 0; i1 < n1; i1++) {
-            const size_t l = (size_t)i1 * n2 + i2;
-            if (hf[l] & 1) list.push_back((int32_t)l);
-          }
-        int32_t* dl = nullptr;
         double *cf = nullptr, *bq = nullptr;
-        if (!list.empty()) {
-          CUDA_TRY(h->put(&dl, list.data(), list.size()));
-          CUDA_TRY(h->put(&cf, (const double*)nullptr, 2 * R * list.size()));
-          CUDA_TRY(cudaMemsetAsync(cf, 0, 2 * R * list.size() * sizeof(double), h->stream));
+        const size_t nc = (size_t)D.nfcross[d];
+        if (nc > 0) {
+          CUDA_TRY(h->put(&cf, (const double*)nullptr, 2 * R * nc));
+          CUDA_TRY(cudaMemsetAsync(cf, 0, 2 * R * nc * sizeof(double), h->stream));
         }
         if (h->nblk[d] > 0) CUDA_TRY(h->put(&bq, (const double*)nullptr, 3 * (size_t)h->nblk[d]));
-        D.fcross[d] = dl;
-        D.nfcross[d] = (int)list.size();
         D.fcoef[d] = cf;
         D.fbq[d] = bq;
-        // the host list must outlive the asynchronous upload
-        CUDA_TRY(cudaStreamSynchronize(h->stream));
       }
-      int4* ref = nullptr;
-      if (D.nmibnode > 0) CUDA_TRY(h->put(&ref, (const int4*)nullptr, (size_t)D.nmibnode));
-      D.mibref = ref;
       mts::build_fast_tables(h->dev, h->stream);
       CUDA_TRY(cudaGetLastError());
       CUDA_TRY(cudaStreamSynchronize(h->stream));

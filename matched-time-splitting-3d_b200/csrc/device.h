@@ -5,22 +5,16 @@
 //   u0, u1   float64[N]   solution ping-pong (state + stage results)
 //   tag      uint8[N]     bit0 outside, bit1/2/3 node is a MIB row of an
 //                         x/y/z crossing block
-//   dp       float64[nmax x T]  partial solutions d'_j of the T = grid
-//                         threads' lines in flight, row-major [row][thread]
-//                         so every access is coalesced whatever the sweep
-//                         direction; reused line after line (L2-resident:
-//                         ~25 MB at 257 nodes and 148 x 256 threads)
-//   fbet, fgam float64[N] per direction that has crossings: Thomas factors
-//                         of crossing lines from their first MIB row on
-//   u0, u1, dp, fbet, fgam carry kRowPad rows of slack (an x-y plane per row
-//                         for the node fields) past their end: the sweeps
-//                         stage whole chunks of rows without bound checks
+//   ca, cb, cg  the Thomas factors of the lines that cross the interface,
+//                         32 B a row, by row and line
+//   u0, u1 and the FP32 fields carry kRowPad rows of slack (x-y planes)
+//                         past their end: the fast form's bulk copies and
+//                         the FP32 ring sweeps may read past the last row
 //   lside    uint8 per line and direction: bit0 node 0, bit1 node 1, bit2
 //                         node n-1 outside (the side changes only at crossings)
 //   per axis: coordinates, sin 2x, cos 2x (exact-solution tables)
 //   per direction: CSR offsets over grid lines -> MIB row blocks
-//   per crossing: time-invariant constants of its jump data, and the
-//                 per-step ([u], [beta u_d]) pair
+//   per crossing: time-invariant constants of its jump data
 #pragma once
 
 #include <cstdint>
@@ -82,28 +76,35 @@ struct Dev {
   const int32_t* bstart[3];
   const MibBlock* blk[3];
   const CrossConst* cc;
-  double2* jv;  // per crossing ([u], u_dir) of the current step
   // Thomas factorisation of every line, computed once (the matrices do not
   // change between steps): bet_j = b_j - a_j*gam_j, gam_j = c_{j-1}/bet_{j-1}.
-  // Up to its first MIB row a line's factors depend only on the side of its
-  // row 1, so they come from the per-direction prefix tables
-  // ptab[d][side][2*j + {0: bet, 1: gam}]; from the first MIB row on they are
-  // stored per node in fbet[d] / fgam[d] (field layout, written only for
-  // lines that cross the interface).
-  const double* ptab[3][2];
-  const double* fbet[3];
-  const double* fgam[3];
-  // Per block, for the sweep in flight: the right-hand sides of its rows after
-  // the jump terms and the Convert2Tri row operations, [3*block + q]
-  // (written by the block pre-pass, read by the sweep).
-  double* rblk[3];
+  // A line that does not cross the interface has the rows of its side (the
+  // side of its row 1): taba[d][side][j] = a_j, tab[d][side][j] = (bet_j,
+  // 1/bet_j), tabg[d][side][j] = gam_{j+1} (0 past the end).  The lines that
+  // cross it (nfcross of them, their ids in fcross in memory order, the index
+  // of a line in that list in cline[i1 + n1 i2], -1: none) have their own, by
+  // row, the lines of a row side by side: ca, cb, cg[d][j nfcross + c].
+  const double* taba[3][2];
+  const double2* tab[3][2];
+  const double* tabg[3][2];
+  const int32_t* fcross[3];
+  int nfcross[3];
+  const int32_t* cline[3];
+  // The interior lines (i1 + n1 i2) in the order of the bit-exact sweeps:
+  // those that cross the interface, then the others inside, then outside.
+  const int32_t* lperm[3];
+  const double* ca[3];
+  const double2* cb[3];
+  const double* cg[3];
+  int plain_div;     // a factor is out of the range of the quotients from reciprocals (kernels.cu)
   int nblk[3];
-  double* dp;        // [nmax][sweep threads of the launch]: forward results d'_j
-  int sweep_blocks;  // one persistent CTA per SM
+  int sweep_blocks;  // SMs
   int shape[3];      // sweep shape of the first, second and third sweep of a step
   // Mixed precision (Douglas-ADI): the step is solved for its increment
   // delta = u^{n+1} - u^n in FP32 (residual in FP64, state accumulated in
-  // FP64).  Factors as 1/bet and gam in FP32, laid out like ptab/fbet/fgam.
+  // FP64).  Factors of the ring sweeps in FP32 (built for grids with a line
+  // too long for the segmented solves): by row per side, and per node from
+  // its first MIB row on for a line that crosses the interface.
   float* r32;                 // residual in, increment out [N + slack]
   float* dp32;                // [nmax + slack][sweep threads]
   const float* ptab32[3][2];  // [2*j + {0: 1/bet, 1: gam}]
@@ -128,17 +129,11 @@ struct Dev {
   // (32 MX each), then 2 x 5 x 32 lane-scan multipliers] of the lines
   // without crossings; per line a flag byte (bit0 the line
   // crosses the interface, bit1 the side of its row 1); the crossing lines'
-  // ids in memory order (fcross, nfcross of them) and their own rows
-  // [c][1/bet, -a/bet][32 MX]; per block the -gam_{j+1} of its rows.  Per
-  // MIB node its block in x, y, z (-1: none); per x block the MIB node
-  // index of each of its rows.
+  // (fcross) own rows [c][1/bet, -a/bet][32 MX]; per block the -gam_{j+1} of its rows.
   const double* ftab[3];
   const uint8_t* fline[3];
-  const int32_t* fcross[3];
-  int nfcross[3];
   const double* fcoef[3];
   const double* fbq[3];
-  const int4* mibref;
   // Replayable steps (batches captured in a CUDA graph): when tsched is set,
   // kernels take the step's exp(-t) factors from tsched[3*(*tstep) + {0: t_prev,
   // 1: t_half, 2: t_next}] instead of their arguments; k_tick advances tstep.
@@ -149,14 +144,15 @@ struct Dev {
   double* u1;  // scratch field
   const long long* mibnode;  // nodes with a MIB flag (any direction), ascending
   int nmibnode;
+  const int4* mibref;        // Douglas-ADI: per listed node its block in x, y, z (16 block + 4 kind + row, -1: none)
   int* status;       // reserved
 };
 
-// Persistent line-sweep shapes (rows per staged chunk, ring depth, threads
-// per CTA); all give bit-identical results, they differ only in speed.
+// Line-sweep shapes (lines per tile, threads per CTA); all give bit-identical
+// results, they differ only in speed.
 int sweep_shape_count();
-int sweep_shape_max_threads();
 bool sweep_shape_fits(int shape, int nmax);  // shared memory of the shape within the limit
+int sweep_shape_default(int nmax);           // -1: no shape takes lines of nmax nodes
 void configure_kernels();
 
 // Per-step exact-solution time factors.
@@ -167,9 +163,10 @@ struct StepTimes {
 // Host-side launchers (kernels.cu).  All enqueue on `stream` and return the
 // number of kernel launches made.
 int launch_initialize(const Dev& P, double E, double* u, cudaStream_t stream);
-// Per-node Thomas factors of the lines with MIB blocks (once, at setup);
-// *zero_pivot is set on a zero pivot.
-int launch_factor_lines(const Dev& P, int* zero_pivot, cudaStream_t stream);
+// Thomas factors of the lines with MIB blocks and the MIB nodes' block
+// references (once, at setup); *flags: bit 0 a zero pivot, bit 1 a factor out
+// of the range of the quotients from reciprocals.
+int launch_factor_lines(const Dev& P, int* flags, cudaStream_t stream);
 // ev: null, or 2 events per kernel slot recorded around each launch.
 // A second stream with its fork and join events (timing off), for work of a
 // step that can run beside the main stream's.
@@ -177,8 +174,7 @@ struct SideStream {
   cudaStream_t stream;
   cudaEvent_t fork, join;
 };
-int launch_step(const Dev& P, const StepTimes& T, double*& u0, double*& u1, cudaStream_t stream,
-                cudaEvent_t* ev, const SideStream* side = nullptr);
+int launch_step(const Dev& P, const StepTimes& T, double* u0, double* u1, cudaStream_t stream, cudaEvent_t* ev);
 // The mixed-precision Douglas-ADI step (mixed.cu), in place on u.
 int launch_step_mixed(const Dev& P, const StepTimes& T, double* u, cudaStream_t stream, cudaEvent_t* ev,
                       const SideStream* side);
@@ -197,7 +193,7 @@ void configure_fast_kernels();
 int fast_rows_per_lane(int n);               // MX of a direction with n rows (0: lines too long)
 bool fast_fits(int nx, int ny, int nz);      // the form takes this grid
 int build_fast_lines(const Dev& P, uint8_t* const fline[3], cudaStream_t stream);  // the line flags
-int build_fast_tables(const Dev& P, cudaStream_t stream);  // fills ftab, fcoef, fbq, mibref (allocated by the caller)
+int build_fast_tables(const Dev& P, cudaStream_t stream);  // fills ftab, fcoef, fbq (allocated by the caller)
 // Batched plain steps (kernels.cu): problems of one method advance together,
 // one launch per kernel of the step for all of them.  A launch's CTAs are
 // listed as items (problem, the CTA's index in that problem's own grid, the
@@ -211,14 +207,10 @@ struct BatchPlan {
   int n;              // problems
   int nmax;           // longest line over the problems
   const Dev* Ps;      // [n] device records (tsched/tstep set)
-  const BatchItem* jumps;
-  int njumps;
-  const BatchItem* rows;  // pointwise passes over grid rows
+  const BatchItem* rows;  // TS explicit half steps
   int nrows;
-  const BatchItem* mib;   // MIB node list passes
+  const BatchItem* mib;   // MIB rows of the Douglas-ADI first right-hand side
   int nmib;
-  const BatchItem* blk[3];  // block pre-pass per direction
-  int nblk[3];
   const BatchItem* sw[3];   // line sweeps per direction
   int nsw[3];
 };
@@ -228,8 +220,6 @@ struct BatchPlan {
 struct MixedBatchPlan {
   int n;
   const Dev* Ps;
-  const BatchItem* jumps;
-  int njumps;
   const BatchItem* rows;
   int nrows;
   const BatchItem* mib;
@@ -243,18 +233,16 @@ int mixed_batch_class(const Dev& P, int d);          // -1: not batchable
 unsigned mixed_line_ctas(const Dev& P, int d);      // CTAs of the line solves of direction d
 int launch_step_batch_mixed(const MixedBatchPlan& plan, cudaStream_t stream);  // one step + tick
 void configure_mixed_batch_kernels();
-int launch_batch_jumps(const Dev* Ps, const BatchItem* items, int nitems, cudaStream_t stream);
 int launch_batch_tick(const Dev* Ps, int n, cudaStream_t stream);
-int batch_sweep_threads();                 // threads per CTA of the batched sweeps
+bool batch_lines_fit(int nmax);            // the batched sweeps take lines of nmax nodes
+unsigned ts_explicit_grid(const Dev& P);
 void configure_batch_kernels();
 int launch_step_batch(const BatchPlan& plan, cudaStream_t stream);  // one step + tick
-unsigned jumps_grid(const Dev& P);
 unsigned mib_grid(const Dev& P);
 unsigned block_grid(const Dev& P, int d);
 unsigned batch_sweep_grid(const Dev& P, int d);
 
 // Shared by both step forms (kernels.cu).
-void launch_jumps(const Dev& P, double E, cudaStream_t stream);
 void launch_tick(const Dev& P, cudaStream_t stream);  // ++(*P.tstep)
 unsigned pointwise_rows_grid(const Dev& P);
 constexpr int kProfileSlots = 8;

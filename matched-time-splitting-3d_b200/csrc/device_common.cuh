@@ -12,8 +12,12 @@ namespace {
 
 constexpr int TPB = 128;                // pointwise kernels and small kernels
 constexpr int kMaxSweepSmem = 232448;  // 227 KB: the sm_100 per-CTA limit
+constexpr int kMaxTileSmem = kMaxSweepSmem - 1024;  // the line tiles keep a few words of static shared memory too
+constexpr int kMaxLineRows = 3245;     // the longest line the bit-exact form takes
+// The batched line tiles: three of them (and their problems' records) to an SM.
+constexpr int kBatchTileSmem = 70 * 1024;
 
-enum Kind { K_COPY = 0, K_STENCIL = 1, K_TS_Z = 2 };
+enum Kind { K_COPY = 0, K_STENCIL = 1, K_TS_Z = 2, K_ADI = 3 };
 
 struct SweepIO {
   const double* stin;  // field the explicit stencil reads
@@ -73,6 +77,16 @@ __device__ __forceinline__ void exact_jumps(const Dev& P, const CrossConst& q, d
     const double xyz[3] = {q.x, q.y, q.z};
     for (int d = 0; d < 3; d++) jb[d] = P.bo * ((2.0 * xyz[d]) * E) - P.bi * (q.D[d] * E);
   }
+}
+
+// Jump data of crossing c (Refresh_Jump, intersection.cc:2294-2490): [u] and
+// u_dir at the step's exp(-t).
+__device__ __forceinline__ double2 jump_at(const Dev& P, int c, double E) {
+  const CrossConst& q = P.cc[c];
+  double ju, jb[3];
+  exact_jumps(P, q, E, ju, jb);
+  const double bxi = q.p[0] * jb[0] + q.p[1] * jb[1] + q.p[2] * jb[2];
+  return make_double2(ju, q.pinv * bxi);
 }
 
 // ---------------------------------------------------------------------------
@@ -164,8 +178,9 @@ __device__ __forceinline__ double corner_jumps(const double* w, double2 l, doubl
 // Explicit 3-point sum of row r of block b with fictitious points, before the
 // dt factor: the MIB branches of douglas_adi.cc:112-210 (jumps = 0) and
 // lod.cc:337-496 (jumps = 1).  U(j) returns the field at row j of the line.
+// Jl, Jr: the jump data of the block's crossings (read when jumps).
 template <class UF>
-__device__ double mib_sum(const MibBlock& b, int r, UF U, const double* vd, bool jumps, const double2* jv) {
+__device__ double mib_sum(const MibBlock& b, int r, UF U, const double* vd, bool jumps, double2 Jl, double2 Jr) {
   const int L = b.L;
   double sum = 0.0;
   if (b.kind == 2) {
@@ -173,25 +188,14 @@ __device__ double mib_sum(const MibBlock& b, int r, UF U, const double* vd, bool
       sum += vd[0] * U(L - 1);
       sum += vd[1] * U(L);
       for (int i = 0; i < 4; i++) sum += vd[2] * U(L - 1 + i) * b.w[1][i];
-      if (jumps) {
-        double2 J = jv[b.c0];
-        sum += vd[2] * (J.x * b.w[1][4] + J.y * b.w[1][5]);
-      }
+      if (jumps) sum += vd[2] * (Jl.x * b.w[1][4] + Jl.y * b.w[1][5]);
     } else {
       sum += vd[1] * U(L + 1);
       sum += vd[2] * U(L + 2);
       for (int i = 0; i < 4; i++) sum += vd[0] * U(L - 1 + i) * b.w[0][i];
-      if (jumps) {
-        double2 J = jv[b.c0];
-        sum += vd[0] * (J.x * b.w[0][4] + J.y * b.w[0][5]);
-      }
+      if (jumps) sum += vd[0] * (Jl.x * b.w[0][4] + Jl.y * b.w[0][5]);
     }
   } else {
-    double2 Jl = make_double2(0, 0), Jr = make_double2(0, 0);
-    if (jumps) {
-      Jl = jv[b.c0];
-      Jr = jv[b.c1];
-    }
     if (r == 0) {
       sum += vd[0] * U(L - 1);
       sum += vd[1] * U(L);
@@ -213,36 +217,17 @@ __device__ double mib_sum(const MibBlock& b, int r, UF U, const double* vd, bool
   return sum;
 }
 
-// Douglas-ADI source jump terms of row r (Src_2nd, douglas_adi.cc:1156-1427).
-__device__ __forceinline__ double adi_src_add(double src, const MibBlock& b, int r, const double* vd,
-                                              const double2* jv) {
-  if (b.kind == 2) {
-    double2 J = jv[b.c0];
-    if (r == 0) return src + vd[2] * (J.x * b.w[1][4] + J.y * b.w[1][5]);
-    return src + vd[0] * (J.x * b.w[0][4] + J.y * b.w[0][5]);
-  }
-  double2 Jl = jv[b.c0], Jr = jv[b.c1];
-  if (r == 0) return src + vd[2] * corner_jumps(b.w[1], Jl, Jr);
-  if (r == 1) {
-    src = src + vd[0] * corner_jumps(b.w[0], Jl, Jr);
-    return src + vd[2] * corner_jumps(b.w[3], Jl, Jr);
-  }
-  return src + vd[0] * corner_jumps(b.w[2], Jl, Jr);
-}
-
 // LOD/TS: jump terms on the right-hand side of the implicit MIB rows
 // (D_xx_l, lod.cc:960-1097), then the Convert2Tri row operations.
 __device__ __forceinline__ void implicit_rows(const Dev& P, const MibBlock& b, double* r,
                                               const double* vd0, const double* vd1, const double* vd2,
-                                              bool jumps, const double2* jv) {
+                                              bool jumps, double2 Jl, double2 Jr) {
   const double cdt = P.cdt;
   if (jumps) {
     if (b.kind == 2) {
-      double2 J = jv[b.c0];
-      r[0] = r[0] + cdt * vd0[2] * (J.x * b.w[1][4] + J.y * b.w[1][5]);
-      r[1] = r[1] + cdt * vd1[0] * (J.x * b.w[0][4] + J.y * b.w[0][5]);
+      r[0] = r[0] + cdt * vd0[2] * (Jl.x * b.w[1][4] + Jl.y * b.w[1][5]);
+      r[1] = r[1] + cdt * vd1[0] * (Jl.x * b.w[0][4] + Jl.y * b.w[0][5]);
     } else {
-      double2 Jl = jv[b.c0], Jr = jv[b.c1];
       r[0] = r[0] + cdt * vd0[2] * corner_jumps(b.w[1], Jl, Jr);
       r[1] = r[1] + cdt * vd1[0] * corner_jumps(b.w[0], Jl, Jr);
       r[1] += cdt * vd1[2] * corner_jumps(b.w[3], Jl, Jr);
@@ -276,6 +261,105 @@ __device__ __forceinline__ const MibBlock* find_block(const Dev& P, int lid, int
   return nullptr;
 }
 
+// The Douglas-ADI data of a MIB node in one direction: the explicit sum of
+// D_dd u there (the MIB sum of douglas_adi.cc:112-210 where the node is a row
+// of a d block, else the three-point sum), and the jump terms that Src_2nd
+// adds (douglas_adi.cc:1156-1427; nt of them, in their order).  ref: the
+// node's block of that direction (Dev::mibref), -1: none.  Every load's
+// address comes from ref alone, so they are in flight together.
+struct MibDir {
+  double sum, t0, t1;
+  int nt;
+};
+__device__ __forceinline__ MibDir mib_direction(const Dev& P, const double* __restrict__ un, double E, long long m,
+                                                int ref, int d, int side) {
+  const long long s = d == 0 ? 1 : d == 1 ? (long long)P.nx : (long long)P.nx * P.ny;
+  const double vd0 = P.vd[d][side][0], vd1 = P.vd[d][side][1], vd2 = P.vd[d][side][2];
+  MibDir r;
+  r.sum = 0.0;
+  r.t0 = r.t1 = 0.0;
+  r.nt = 0;
+  if (ref < 0) {
+    r.sum += un[m - s] * vd0;
+    r.sum += un[m] * vd1;
+    r.sum += un[m + s] * vd2;
+    return r;
+  }
+  const MibBlock& b = (d == 0 ? P.blk[0] : d == 1 ? P.blk[1] : P.blk[2])[ref >> 4];
+  const int kind = (ref >> 2) & 3, row = ref & 3;
+  const double* const p = un + m - (row + 1) * s;  // row L-1
+  double u[5], w[9];
+  for (int i = 0; i < 4; i++) u[i] = p[i * s];
+  u[4] = kind == 3 ? p[4 * s] : 0.0;
+  // the fictitious value's weights: right of the first row, left of the others
+  const double* const wp = b.w[row == 0 ? 1 : row == 1 ? 0 : 2];
+  for (int i = 0; i < 9; i++) w[i] = wp[i];
+  const double2 Jl = jump_at(P, b.c0, E);
+  const double2 Jr = kind == 3 ? jump_at(P, b.c1, E) : Jl;
+  const double vf = row == 0 ? vd2 : vd0;
+  if (kind == 3 && row == 1) {
+    for (int i = 0; i < 5; i++) r.sum += vf * u[i] * w[i];
+    r.sum += vd1 * u[2];
+    const double* const wq = b.w[3];
+    for (int i = 0; i < 5; i++) r.sum += vd2 * u[i] * wq[i];
+    r.t0 = vf * (Jl.x * w[5] + Jl.y * w[6] + Jr.x * w[7] + Jr.y * w[8]);
+    r.t1 = vd2 * (Jl.x * wq[5] + Jl.y * wq[6] + Jr.x * wq[7] + Jr.y * wq[8]);
+    r.nt = 2;
+    return r;
+  }
+  r.sum += row == 0 ? vd0 * u[0] : vd1 * (kind == 2 ? u[2] : u[3]);
+  r.sum += row == 0 ? vd1 * u[1] : vd2 * (kind == 2 ? u[3] : u[4]);
+  for (int i = 0; i < 4; i++) r.sum += vf * u[i] * w[i];
+  if (kind == 3) r.sum += vf * u[4] * w[4];
+  r.t0 = kind == 2 ? vf * (Jl.x * w[4] + Jl.y * w[5]) : vf * (Jl.x * w[5] + Jl.y * w[6] + Jr.x * w[7] + Jr.y * w[8]);
+  r.nt = 1;
+  return r;
+}
+
+// The listed MIB nodes k0 <= k < k1, shared out over nw warps (this one is
+// w): three lanes a node, one per direction.  done(m, ix, iy, iz, sx, sy,
+// sz, src) gets a node's three sums and its source with the jump terms.
+template <class F>
+__device__ __forceinline__ void mib_nodes(const Dev& P, const double* __restrict__ un, double E, int k0, int k1, int w,
+                                          int nw, F done) {
+  constexpr unsigned ALL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int d = lane % 3, g = lane / 3;
+  for (int kb = k0 + 10 * w; kb < k1; kb += 10 * nw) {
+    const int k = kb + g;
+    const bool act = g < 10 && k < k1;
+    MibDir r{0.0, 0.0, 0.0, 0};
+    long long m = 0;
+    int side = 0;
+    if (act) {
+      m = P.mibnode[k];
+      const int ref = reinterpret_cast<const int*>(P.mibref)[4 * (long long)k + d];
+      side = P.tag[m] & TAG_OUT;
+      r = mib_direction(P, un, E, m, ref, d, side);
+    }
+    MibDir q[2];
+    for (int e = 0; e < 2; e++) {
+      q[e].sum = __shfl_down_sync(ALL, r.sum, e + 1);
+      q[e].t0 = __shfl_down_sync(ALL, r.t0, e + 1);
+      q[e].t1 = __shfl_down_sync(ALL, r.t1, e + 1);
+      q[e].nt = __shfl_down_sync(ALL, r.nt, e + 1);
+    }
+    if (act && d == 0) {
+      int ix, iy, iz;
+      node_xyz(P, m, ix, iy, iz);
+      double src = source(P, E, side, ix, iy, iz);
+      if (r.nt > 0) src = src + r.t0;
+      if (r.nt > 1) src = src + r.t1;
+      for (int e = 0; e < 2; e++) {
+        if (q[e].nt > 0) src = src + q[e].t0;
+        if (q[e].nt > 1) src = src + q[e].t1;
+      }
+      done(m, ix, iy, iz, r.sum, q[0].sum, q[1].sum, src);
+    }
+  }
+}
+
+inline unsigned mib_nodes_grid(const Dev& P) { return (unsigned)((P.nmibnode + 10 * (TPB / 32) - 1) / (10 * (TPB / 32))); }
 
 // Rows of the pointwise passes: a warp takes one x-row (iy, iz) at a time and
 // covers it in groups of G x 32 nodes (ROW_G, or 2 for the five-load ADI

@@ -18,7 +18,7 @@
 // same time as the others.  A step is:
 //
 //   kf_mib  the right-hand side of every MIB row (the explicit MIB sums of
-//           all three directions and the jump terms, one thread per node),
+//           all three directions and the jump terms, a lane per direction),
 //           written into d at those nodes;
 //   kf_xw   rho of the regular x lines (and d on the face lines), fused with
 //           their solves: a CTA walks a column of planes for TY lines with
@@ -103,82 +103,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, unsigned parity) {
 // Orders this thread's generic-proxy shared-memory accesses before later
 // bulk copies into the same memory.
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
-
-// ---------------------------------------------------------------------------
-// Jump data on the fly (Refresh_Jump, intersection.cc:2294-2490): [u] and
-// u_dir of crossing c at the step's exp(-t), the values k_jumps stores.
-
-__device__ __forceinline__ double2 jump_at(const Dev& P, int c, double E) {
-  const CrossConst& q = P.cc[c];
-  double ju, jb[3];
-  if (P.eq == 0) {
-    ju = 100.0 - 80.0;
-    for (int d = 0; d < 3; d++) jb[d] = 0.0;
-  } else {
-    ju = q.R2 * E - q.S * E;
-    const double xyz[3] = {q.x, q.y, q.z};
-    for (int d = 0; d < 3; d++) jb[d] = P.bo * ((2.0 * xyz[d]) * E) - P.bi * (q.D[d] * E);
-  }
-  const double bxi = q.p[0] * jb[0] + q.p[1] * jb[1] + q.p[2] * jb[2];
-  return make_double2(ju, q.pinv * bxi);
-}
-
-// Src_2nd's jump terms of row r of block b (douglas_adi.cc:1156-1427).
-__device__ __forceinline__ double src_jumps(const Dev& P, double E, double src, const MibBlock& b, int r,
-                                            const double* vd) {
-  if (b.kind == 2) {
-    const double2 J = jump_at(P, b.c0, E);
-    if (r == 0) return src + vd[2] * (J.x * b.w[1][4] + J.y * b.w[1][5]);
-    return src + vd[0] * (J.x * b.w[0][4] + J.y * b.w[0][5]);
-  }
-  const double2 Jl = jump_at(P, b.c0, E), Jr = jump_at(P, b.c1, E);
-  if (r == 0) return src + vd[2] * corner_jumps(b.w[1], Jl, Jr);
-  if (r == 1) {
-    src = src + vd[0] * corner_jumps(b.w[0], Jl, Jr);
-    return src + vd[2] * corner_jumps(b.w[3], Jl, Jr);
-  }
-  return src + vd[0] * corner_jumps(b.w[2], Jl, Jr);
-}
-
-// rho at a MIB node m = (ix, iy, iz): the explicit MIB sums of
-// douglas_adi.cc:112-210 (no jumps) in every direction the node is a block
-// row of, the regular three-point sums in the others, and the jump terms of
-// Src_2nd.  ref: the node's block in x, y, z (-1: none).
-__device__ __noinline__ double rho_mib(const Dev& P, const double* __restrict__ un, double E, long long m, int ix,
-                                       int iy, int iz, int tg, int4 ref) {
-  const int side = tg & TAG_OUT;
-  const long long sy = P.nx, sz = (long long)P.nx * P.ny;
-  const double* vdx = P.vd[0][side];
-  const double* vdy = P.vd[1][side];
-  const double* vdz = P.vd[2][side];
-  const MibBlock* xb = ref.x >= 0 ? &P.blk[0][ref.x] : nullptr;
-  const MibBlock* yb = ref.y >= 0 ? &P.blk[1][ref.y] : nullptr;
-  const MibBlock* zb = ref.z >= 0 ? &P.blk[2][ref.z] : nullptr;
-  double sx, sy_, sz_;
-  if (xb) {
-    const long long base = m - ix;
-    sx = mib_sum(*xb, ix - xb->L, [&](int j) { return un[base + j]; }, vdx, false, P.jv);
-  } else {
-    sx = (un[m - 1] * vdx[0] + un[m] * vdx[1]) + un[m + 1] * vdx[2];
-  }
-  if (yb) {
-    const long long base = ix + sz * iz;
-    sy_ = mib_sum(*yb, iy - yb->L, [&](int j) { return un[base + (long long)j * sy]; }, vdy, false, P.jv);
-  } else {
-    sy_ = (un[m - sy] * vdy[0] + un[m] * vdy[1]) + un[m + sy] * vdy[2];
-  }
-  if (zb) {
-    const long long base = ix + (long long)P.nx * iy;
-    sz_ = mib_sum(*zb, iz - zb->L, [&](int j) { return un[base + (long long)j * sz]; }, vdz, false, P.jv);
-  } else {
-    sz_ = (un[m - sz] * vdz[0] + un[m] * vdz[1]) + un[m + sz] * vdz[2];
-  }
-  double src = source(P, E, side, ix, iy, iz);
-  if (xb) src = src_jumps(P, E, src, *xb, ix - xb->L, vdx);
-  if (yb) src = src_jumps(P, E, src, *yb, iy - yb->L, vdy);
-  if (zb) src = src_jumps(P, E, src, *zb, iz - zb->L, vdz);
-  return P.dt * (((sx + sy_) + sz_) + src);
-}
 
 // The Convert2Tri row operations of a line's blocks on its right-hand side
 // in shared memory (buf: the line's rows, stride 1), and their rows' own q
@@ -455,15 +379,12 @@ __device__ __forceinline__ void load_tab(double* s, const double* g, int w2) {
 
 __global__ void __launch_bounds__(TPB) kf_mib(const __grid_constant__ Dev P, const double* __restrict__ un,
                                               double* __restrict__ d, double E) {
-  // every MIB row at once, one thread each (the rows of an x block too:
+  // every MIB row at once, three lanes each (the rows of an x block too:
   // kf_xc applies their block's row operations when it solves the line)
-  const long long k = (long long)blockIdx.x * TPB + threadIdx.x;
-  if (k >= P.nmibnode) return;
-  E = step_e(P, E, 2);
-  const long long m = P.mibnode[k];
-  int ix, iy, iz;
-  node_xyz(P, m, ix, iy, iz);
-  d[m] = rho_mib(P, un, E, m, ix, iy, iz, P.tag[m], P.mibref[k]);
+  mib_nodes(P, un, step_e(P, E, 2), 0, P.nmibnode, blockIdx.x * (TPB / 32) + (threadIdx.x >> 5), gridDim.x * (TPB / 32),
+            [&](long long m, int, int, int, double sx, double sy, double sz, double src) {
+              d[m] = P.dt * (((sx + sy) + sz) + src);
+            });
 }
 
 // ---------------------------------------------------------------------------
@@ -1069,8 +990,8 @@ __global__ void __launch_bounds__(32 * CW, 3) kf_yc(const __grid_constant__ Dev 
 // ---------------------------------------------------------------------------
 // Set-up of the form (once per handle).
 
-// Row tables of direction D: [side][TABW]: ib and p by row from the prefix
-// factors of that side (ptab: bet_j, gam_j), zero past the line end.
+// Row tables of direction D: [side][TABW]: ib and p by row from the
+// factors of that side, zero past the line end.
 template <int D>
 __global__ void __launch_bounds__(TPB) kf_tab(const __grid_constant__ Dev P, double* tab, int R) {
   const int n = D == 0 ? P.nx : D == 1 ? P.ny : P.nz;
@@ -1079,10 +1000,9 @@ __global__ void __launch_bounds__(TPB) kf_tab(const __grid_constant__ Dev P, dou
   const int side = i / R, j = i % R;
   double ib = 0.0, p = 0.0;
   if (j < n) {
-    const double bet = P.ptab[D][side][2 * j];
-    const double a = (j == 0 || j == n - 1) ? 0.0 : P.ia[D][side];
-    ib = 1.0 / bet;
-    p = -(a / bet);
+    const double2 b = P.tab[D][side][j];
+    ib = b.y;
+    p = -(P.taba[D][side][j] / b.x);
   }
   double* T = tab + (size_t)side * (2 * R + 320);
   T[j] = ib;
@@ -1136,98 +1056,32 @@ __global__ void __launch_bounds__(TPB) kf_fline(const __grid_constant__ Dev P, u
   fl[L.lid] = v;
 }
 
-// Line geometry from a line id (i1 * n2 + i2) of direction D.
-template <int D>
-__device__ __forceinline__ void line_at(const Dev& P, long long lid, long long& base, long long& s) {
-  const int n2 = D == 2 ? P.ny : P.nz;
-  const int i1 = (int)(lid / n2), i2 = (int)(lid % n2);
-  if (D == 0) {
-    base = (long long)P.nx * (i1 + (long long)P.ny * i2);
-    s = 1;
-  } else if (D == 1) {
-    base = i1 + (long long)P.nx * P.ny * i2;
-    s = P.nx;
-  } else {
-    base = i1 + (long long)P.nx * i2;
-    s = (long long)P.nx * P.ny;
-  }
-}
-
-// Coefficients (ib, p) of the crossing lines, one thread per listed line,
-// walking the line as the sequential sweep does (the factors from the
-// prefix table before the first MIB row and per node from it on; the regular
-// rows' side from the line's start and after each block), into cf[c][2][R].
+// Coefficients (ib, p) of the crossing lines from their factors, one thread
+// per listed line and row, into cf[c][2][R].
 template <int D>
 __global__ void __launch_bounds__(TPB) kf_coef(const __grid_constant__ Dev P, double* cf, int R) {
-  const int c = blockIdx.x * TPB + threadIdx.x;
-  if (c >= P.nfcross[D]) return;
-  const long long lid = P.fcross[D][c];
   const int n = D == 0 ? P.nx : D == 1 ? P.ny : P.nz;
-  long long base, s;
-  line_at<D>(P, lid, base, s);
-  const int bfirst = P.bstart[D][lid], bend = P.bstart[D][lid + 1];
-  const MibBlock* const blk = P.blk[D];
-  const int L1 = blk[bfirst].L;
-  const int side1 = (P.lside[D][lid] >> 1) & 1;
-  const double* const pt = P.ptab[D][side1];
+  const int nc = P.nfcross[D];
+  const long long t = (long long)blockIdx.x * TPB + threadIdx.x;
+  if (t >= (long long)nc * n) return;
+  const int c = (int)(t % nc), j = (int)(t / nc);
+  const double2 b = P.cb[D][t];
   double* const o = cf + (size_t)c * 2 * R;
-  int b = bfirst, side = side1;
-  for (int j = 0; j < n; j++) {
-    const double bet = j >= L1 ? P.fbet[D][base + (long long)j * s] : pt[2 * j];
-    double a;
-    if (j == 0 || j == n - 1) {
-      a = 0.0;
-    } else if (b < bend && j >= blk[b].L) {
-      const int q = j - blk[b].L;
-      a = blk[b].ia[q];
-      if (q == blk[b].kind - 1) {
-        side = (blk[b].sides >> q) & 1;
-        b++;
-      }
-    } else {
-      a = P.ia[D][side];
-    }
-    o[j] = 1.0 / bet;
-    o[R + j] = -(a / bet);
-  }
+  o[j] = b.y;
+  o[R + j] = -(P.ca[D][t] / b.x);
 }
 
 // q = -gam_{j+1} of the rows of each block of direction D (their c is not
-// their a), from the per-node factors: bq[3 k + r].
+// their a): bq[3 k + r].
 template <int D>
 __global__ void __launch_bounds__(TPB) kf_bq(const __grid_constant__ Dev P, double* bq) {
   const int k = blockIdx.x * TPB + threadIdx.x;
   if (k >= P.nblk[D]) return;
   const MibBlock& b = P.blk[D][k];
-  long long base, s;
-  line_at<D>(P, b.line, base, s);
+  const int n1 = D == 0 ? P.ny : P.nx, n2 = D == 2 ? P.ny : P.nz;
+  const int c = P.cline[D][b.line / n2 + n1 * (b.line % n2)];
   for (int r = 0; r < 3; r++)
-    bq[3 * (long long)k + r] = r < b.kind ? -P.fgam[D][base + (long long)(b.L + r + 1) * s] : 0.0;
-}
-
-// Per MIB node: its block in each direction (-1: none).
-__global__ void __launch_bounds__(TPB) kf_mibref(const __grid_constant__ Dev P, int4* ref) {
-  const int k = blockIdx.x * TPB + threadIdx.x;
-  if (k >= P.nmibnode) return;
-  const long long m = P.mibnode[k];
-  const int tg = P.tag[m];
-  int ix, iy, iz;
-  node_xyz(P, m, ix, iy, iz);
-  int4 r = make_int4(-1, -1, -1, 0);
-  int row = 0;
-  if (tg & TAG_MIBX) {
-    const MibBlock* b = find_block<0>(P, iy * P.nz + iz, ix, row);
-    if (b) r.x = (int)(b - P.blk[0]);
-  }
-  if (tg & TAG_MIBY) {
-    const MibBlock* b = find_block<1>(P, ix * P.nz + iz, iy, row);
-    if (b) r.y = (int)(b - P.blk[1]);
-  }
-  if (tg & TAG_MIBZ) {
-    const MibBlock* b = find_block<2>(P, ix * P.ny + iy, iz, row);
-    if (b) r.z = (int)(b - P.blk[2]);
-  }
-  ref[k] = r;
+    bq[3 * (long long)k + r] = r < b.kind ? -P.cg[D][(long long)(b.L + r) * P.nfcross[D] + c] : 0.0;
 }
 
 // ---------------------------------------------------------------------------
@@ -1360,7 +1214,7 @@ int build_fast_tables(const Dev& P, cudaStream_t st) {
     if (P.nblk[d] == 0) continue;
     double* cf = const_cast<double*>(P.fcoef[d]);
     double* bq = const_cast<double*>(P.fbq[d]);
-    const unsigned gc = (unsigned)((P.nfcross[d] + TPB - 1) / TPB);
+    const unsigned gc = (unsigned)(((long long)P.nfcross[d] * nd[d] + TPB - 1) / TPB);
     const unsigned gb = (unsigned)((P.nblk[d] + TPB - 1) / TPB);
     if (d == 0) {
       if (gc) kf_coef<0><<<gc, TPB, 0, st>>>(P, cf, R);
@@ -1375,10 +1229,6 @@ int build_fast_tables(const Dev& P, cudaStream_t st) {
       kf_bq<2><<<gb, TPB, 0, st>>>(P, bq);
     }
     launches += 2;
-  }
-  if (P.nmibnode > 0) {
-    kf_mibref<<<(unsigned)((P.nmibnode + TPB - 1) / TPB), TPB, 0, st>>>(P, const_cast<int4*>(P.mibref));
-    launches++;
   }
   return launches;
 }
@@ -1409,7 +1259,7 @@ int launch_step_fast(const Dev& P, const StepTimes& T, double* u, double* d, cud
   };
   mark(0);
   if (P.nmibnode > 0) {
-    kf_mib<<<(unsigned)((P.nmibnode + TPB - 1) / TPB), TPB, 0, st>>>(P, u, d, T.e_next);
+    kf_mib<<<mib_nodes_grid(P), TPB, 0, st>>>(P, u, d, T.e_next);
     launches++;
   }
 

@@ -1,26 +1,12 @@
 // Time-stepping kernels for sm_100a.
 //
 // Implicit line sweeps (the Thomas solves, douglas_adi.cc:1784-1807 and the
-// LOD/TS copies) run as one persistent CTA of 128-512 threads per SM (the
-// sweep shape); each thread solves one grid line at a time, lines of a warp
-// being consecutive in the fast index.  The Thomas factors (bet, gam) are
-// computed once at setup.  Per line:
-//   * forward: the inputs of the line (and its per-node factors from its
-//     first MIB row on) are staged into a shared-memory ring with cp.async,
-//     chunks ahead of use; each row's right-hand side is built from the ring
-//     (3-point stencil, source terms), the MIB row blocks' right-hand sides
-//     come from the block pre-pass (Convert2Tri row operations replayed on
-//     them), and the elimination recurrence runs over the chunk;
-//   * the partial solutions d'_j go to per-thread scratch laid out
-//     [row][thread] (coalesced in every direction, reused line after line);
-//   * backward: the scratch is staged back through the same ring and the
-//     solution is written once.
-// The inside/outside side of a node, which selects the stencil weights and
-// the source, changes along a line only at its recorded crossings, so it is
-// tracked from the line's block list instead of being read per node.
+// LOD/TS copies): a CTA holds a tile of lines in shared memory, builds their
+// right-hand sides (stencils, sources, MIB rows with their jumps) with all
+// threads, solves them with one warp, a lane per line, and writes them back
+// (k_line).  The Thomas factors (bet, gam) are computed once at setup.
 //
-// Pointwise passes (the Douglas-ADI first right-hand side and the TS explicit
-// half steps) are plain grid-stride kernels.
+// The TS explicit half steps are plain grid-stride kernels.
 //
 // The file is compiled with -fmad=false: every product and sum is rounded on
 // its own, in the operand order of the reference statement it restates, which
@@ -37,9 +23,6 @@ namespace {
 // ---------------------------------------------------------------------------
 // Pointwise passes
 
-// Douglas-ADI first right-hand side (douglas_adi.cc:89-359):
-//   uhs = ((dt*D_yy u + dt*D_zz u) + u) + dt*src,  src = f + x, y, z jump
-// terms; Outer_u(t_next) on the faces.
 // Pointwise kernels run one warp per grid row (iy, iz), lanes over ix.
 #define FOR_EACH_NODE(P)                                                                          \
   for (int row_ = blockIdx.x * (TPB / 32) + (threadIdx.x >> 5); row_ < (P).ny * (P).nz;          \
@@ -47,157 +30,34 @@ namespace {
     for (int ix = threadIdx.x & 31, iy = row_ % (P).ny, iz = row_ / (P).ny; ix < (P).nx; ix += 32) \
       if (long long m = ix + (long long)(P).nx * row_; true)
 
-// RHS1 of a node that is a MIB row of some x, y or z block: the general form.
-__device__ __forceinline__ double adi_rhs_mib(const Dev& P, const double* __restrict__ un, double E, long long m,
-                                              int ix, int iy, int iz, int tg) {
-  const long long sy = P.nx, sz = (long long)P.nx * P.ny;
-  const int side = tg & TAG_OUT;
-  const double dt = P.dt;
-  const double* vdy = P.vd[1][side];
-  const double* vdz = P.vd[2][side];
-  const MibBlock* xb = nullptr;
-  const MibBlock* yb = nullptr;
-  const MibBlock* zb = nullptr;
-  int xr = 0, yr = 0, zr = 0;
-  double sum, ydt, zdt;
-  if (tg & TAG_MIBY) yb = find_block<1>(P, ix * P.nz + iz, iy, yr);
-  if (yb) {
-    const long long base = ix + sz * iz;
-    sum = mib_sum(*yb, yr, [&](int j) { return un[base + (long long)j * sy]; }, vdy, false, P.jv);
-    ydt = sum * dt;
-  } else {
-    sum = 0.0;
-    sum += un[m - sy] * vdy[0];
-    sum += un[m] * vdy[1];
-    sum += un[m + sy] * vdy[2];
-    ydt = dt * sum;
-  }
-  if (tg & TAG_MIBZ) zb = find_block<2>(P, ix * P.ny + iy, iz, zr);
-  if (zb) {
-    const long long base = ix + (long long)P.nx * iy;
-    sum = mib_sum(*zb, zr, [&](int j) { return un[base + (long long)j * sz]; }, vdz, false, P.jv);
-    zdt = sum * dt;
-  } else {
-    sum = 0.0;
-    sum += un[m - sz] * vdz[0];
-    sum += un[m] * vdz[1];
-    sum += un[m + sz] * vdz[2];
-    zdt = dt * sum;
-  }
-  double src = source(P, E, side, ix, iy, iz);
-  if (tg & TAG_MIBX) xb = find_block<0>(P, iy * P.nz + iz, ix, xr);
-  if (xb) src = adi_src_add(src, *xb, xr, P.vd[0][side], P.jv);
-  if (yb) src = adi_src_add(src, *yb, yr, vdy, P.jv);
-  if (zb) src = adi_src_add(src, *zb, zr, vdz, P.jv);
-  double r = ydt + zdt;
-  r += un[m];
-  r += dt * src;
-  return r;
-}
-
-template <int G>
-__device__ __forceinline__ void k_adi_rhs_body(const Dev& P, unsigned cta_, unsigned ncta_,
+// The MIB rows of the Douglas-ADI first right-hand side (douglas_adi.cc:
+// 89-359): uhs = ((dt*D_yy u + dt*D_zz u) + u) + dt*src with src = f + the x,
+// y, z jump terms, into R at those nodes; the x sweep takes them from there.
+// A pass of its own because a node waits on three loads in a row (its block,
+// the block's weights and crossings, the field): all nodes of the grid wait
+// at once here, a tile's would wait in turn.
+__device__ __forceinline__ void k_adi_mib_body(const Dev& P, unsigned cta_, unsigned ncta_,
                                                const double* __restrict__ un, double* __restrict__ R, double E) {
-  E = step_e(P, E, 2);
-  const int lane = threadIdx.x & 31;
-  const int nx = P.nx, nrows = P.ny * P.nz;
-  const long long sy = nx, sz = (long long)nx * P.ny;
   const double dt = P.dt;
-  // a node's side selects one of two specialised bodies (uniform over a warp
-  // away from the interface), whose stencil weights are fixed kernel
-  // parameters (constant-bank operands) instead of weights indexed per node
-  for (int row = cta_ * (TPB / 32) + (threadIdx.x >> 5); row < nrows; row += ncta_ * (TPB / 32)) {
-    const int iy = row % P.ny, iz = row / P.ny;
-    const long long m0 = (long long)nx * row;
-    const RowExact q = row_exact(P, iy, iz);
-    double* const Rr = R + m0;
-    if (iy == 0 || iz == 0 || iy == P.ny - 1 || iz == P.nz - 1) {
-      for (int ix = lane; ix < nx; ix += 32) Rr[ix] = row_outer(P, q, ix, E);
-      continue;
-    }
-    // the row's two face nodes, then its interior in groups of G x 32
-    if (lane < 2) {
-      const int ix = lane ? nx - 1 : 0;
-      Rr[ix] = row_outer(P, q, ix, E);
-    }
-    const double* const uc_r = un + m0;
-    const double* const uym_r = uc_r - sy;
-    const double* const uyp_r = uc_r + sy;
-    const double* const uzm_r = uc_r - sz;
-    const double* const uzp_r = uc_r + sz;
-    const uint8_t* const tg_r = P.tag + m0;
-    for (int ix0 = 1; ix0 < nx - 1; ix0 += 32 * G) {
-      double uc[G], uym[G], uyp[G], uzm[G], uzp[G];
-      int tg[G];
-#pragma unroll
-      for (int g = 0; g < G; g++) {
-        const int ix = ix0 + 32 * g + lane;
-        if (ix < nx - 1) {
-          tg[g] = tg_r[ix];
-          uc[g] = uc_r[ix];
-          uym[g] = uym_r[ix];
-          uyp[g] = uyp_r[ix];
-          uzm[g] = uzm_r[ix];
-          uzp[g] = uzp_r[ix];
-        }
-      }
-#pragma unroll
-      for (int g = 0; g < G; g++) {
-        const int ix = ix0 + 32 * g + lane;
-        if (ix >= nx - 1) break;
-        if (tg[g] & (TAG_MIBX | TAG_MIBY | TAG_MIBZ)) continue;  // a MIB row: k_adi_rhs_mib writes it
-        auto node = [&](auto S) {
-          constexpr int sd = decltype(S)::value;
-          double sum = 0.0;
-          sum += uym[g] * P.vd[1][sd][0];
-          sum += uc[g] * P.vd[1][sd][1];
-          sum += uyp[g] * P.vd[1][sd][2];
-          const double ydt = dt * sum;
-          sum = 0.0;
-          sum += uzm[g] * P.vd[2][sd][0];
-          sum += uc[g] * P.vd[2][sd][1];
-          sum += uzp[g] * P.vd[2][sd][2];
-          const double zdt = dt * sum;
-          const double src = row_source(P, q, ix, E, sd);
-          double r = ydt + zdt;
-          r += uc[g];
-          r += dt * src;
-          return r;
-        };
-        Rr[ix] = (tg[g] & TAG_OUT) ? node(IntC<1>{}) : node(IntC<0>{});
-      }
-    }
-  }
+  mib_nodes(P, un, step_e(P, E, 2), 0, P.nmibnode, cta_ * (TPB / 32) + (threadIdx.x >> 5), ncta_ * (TPB / 32),
+            [&](long long m, int, int, int, double, double sy, double sz, double src) {
+              double r = sy * dt + sz * dt;
+              r += un[m];
+              r += dt * src;
+              R[m] = r;
+            });
 }
 
-template <int G>
-__global__ void __launch_bounds__(TPB, 8) k_adi_rhs(const __grid_constant__ Dev P, const double* __restrict__ un,
+__global__ void __launch_bounds__(TPB) k_adi_mib(const __grid_constant__ Dev P, const double* __restrict__ un,
                                                  double* __restrict__ R, double E) {
-  k_adi_rhs_body<G>(P, blockIdx.x, gridDim.x, un, R, E);
-}
-
-// The MIB rows of RHS1, one thread per listed node.
-__device__ __forceinline__ void k_adi_rhs_mib_body(const Dev& P, unsigned cta_, unsigned ncta_,
-                                                   const double* __restrict__ un, double* __restrict__ R, double E) {
-  const int k = cta_ * TPB + threadIdx.x;
-  if (k >= P.nmibnode) return;
-  E = step_e(P, E, 2);
-  const long long m = P.mibnode[k];
-  int ix, iy, iz;
-  node_xyz(P, m, ix, iy, iz);
-  R[m] = adi_rhs_mib(P, un, E, m, ix, iy, iz, P.tag[m]);
-}
-
-__global__ void __launch_bounds__(TPB) k_adi_rhs_mib(const __grid_constant__ Dev P, const double* __restrict__ un,
-                                                     double* __restrict__ R, double E) {
-  k_adi_rhs_mib_body(P, blockIdx.x, gridDim.x, un, R, E);
+  k_adi_mib_body(P, blockIdx.x, gridDim.x, un, R, E);
 }
 
 // TS explicit half step along D = x or y (TS::D_xx_r / D_yy_r, the LOD
 // Crank-Nicolson operators, trapezoidal.cc:319-895), then Set_bc at t_half.
 template <int D>
-__device__ __forceinline__ double ts_explicit_mib(const Dev& P, const double* __restrict__ in, long long m, int ix,
-                                               int iy, int iz, int tg) {
+__device__ __noinline__ double ts_explicit_mib(const Dev& P, const double* in, double E1, long long m, int ix, int iy,
+                                               int iz, int tg) {
   const long long s = D == 0 ? 1 : (long long)P.nx;
   const double* vd = P.vd[D][tg & TAG_OUT];
   int r = 0;
@@ -205,7 +65,8 @@ __device__ __forceinline__ double ts_explicit_mib(const Dev& P, const double* __
   double sum;
   if (b) {
     const long long base = D == 0 ? m - ix : m - (long long)iy * P.nx;
-    sum = mib_sum(*b, r, [&](int j) { return in[base + (long long)j * s]; }, vd, true, P.jv);
+    sum = mib_sum(*b, r, [&](int j) { return in[base + (long long)j * s]; }, vd, true, jump_at(P, b->c0, E1),
+                  jump_at(P, b->c1, E1));
   } else {
     sum = 0.0;
     sum += in[m - s] * vd[0];
@@ -215,38 +76,35 @@ __device__ __forceinline__ double ts_explicit_mib(const Dev& P, const double* __
   return P.kex * sum + in[m];
 }
 
-template <int D>
-__device__ __forceinline__ void k_ts_explicit_mib_body(const Dev& P, unsigned cta_, unsigned ncta_,
-                                                       const double* __restrict__ in, double* __restrict__ out) {
-  const int k = cta_ * TPB + threadIdx.x;
-  if (k >= P.nmibnode) return;
-  const long long m = P.mibnode[k];
-  const int tg = P.tag[m];
-  if (!(tg & (D == 0 ? TAG_MIBX : TAG_MIBY))) return;
-  int ix, iy, iz;
-  node_xyz(P, m, ix, iy, iz);
-  out[m] = ts_explicit_mib<D>(P, in, m, ix, iy, iz, tg);
-}
-
-template <int D>
-__global__ void __launch_bounds__(TPB) k_ts_explicit_mib(const __grid_constant__ Dev P,
-                                                         const double* __restrict__ in, double* __restrict__ out) {
-  k_ts_explicit_mib_body<D>(P, blockIdx.x, gridDim.x, in, out);
-}
+// CTAs of the pass that take the MIB rows, a thread per listed node, after
+// the ones that walk the grid's rows.
+__host__ __device__ __forceinline__ unsigned mib_ctas(const Dev& P) { return (unsigned)((P.nmibnode + TPB - 1) / TPB); }
 
 template <int D>
 __device__ __forceinline__ void k_ts_explicit_body(const Dev& P, unsigned cta_, unsigned ncta_,
                                                    const double* __restrict__ in, double* __restrict__ out,
-                                                   double eh) {
-  eh = step_e(P, eh, 1);
+                                                   double eh, double e1) {
   const long long s = D == 0 ? 1 : (long long)P.nx;
   const int flag = D == 0 ? TAG_MIBX : TAG_MIBY;
+  const unsigned nrow = ncta_ - mib_ctas(P);
+  if (cta_ >= nrow) {
+    const int k = (int)(cta_ - nrow) * TPB + threadIdx.x;
+    if (k >= P.nmibnode) return;
+    const long long m = P.mibnode[k];
+    const int tg = P.tag[m];
+    if (!(tg & flag)) return;
+    int ix, iy, iz;
+    node_xyz(P, m, ix, iy, iz);
+    out[m] = ts_explicit_mib<D>(P, in, step_e(P, e1, 2), m, ix, iy, iz, tg);
+    return;
+  }
+  eh = step_e(P, eh, 1);
   const int lane = threadIdx.x & 31;
   const int nrows = P.ny * P.nz;
   const double kex = P.kex;
   const double w0i = P.vd[D][0][0], w1i = P.vd[D][0][1], w2i = P.vd[D][0][2];
   const double w0o = P.vd[D][1][0], w1o = P.vd[D][1][1], w2o = P.vd[D][1][2];
-  for (int row = cta_ * (TPB / 32) + (threadIdx.x >> 5); row < nrows; row += ncta_ * (TPB / 32)) {
+  for (int row = cta_ * (TPB / 32) + (threadIdx.x >> 5); row < nrows; row += nrow * (TPB / 32)) {
     const int iy = row % P.ny, iz = row / P.ny;
     const long long m0 = (long long)P.nx * row;
     const RowExact q = row_exact(P, iy, iz);
@@ -284,7 +142,7 @@ __device__ __forceinline__ void k_ts_explicit_body(const Dev& P, unsigned cta_, 
           sum += up[g] * (side ? w2o : w2i);
           v = kex * sum + uc[g];
         } else {
-          continue;  // a MIB row of a D block: k_ts_explicit_mib writes it
+          continue;  // a MIB row of a D block: the CTAs past the rows write it
         }
         out[m] = v;
       }
@@ -294,576 +152,876 @@ __device__ __forceinline__ void k_ts_explicit_body(const Dev& P, unsigned cta_, 
 
 template <int D>
 __global__ void __launch_bounds__(TPB) k_ts_explicit(const __grid_constant__ Dev P, const double* __restrict__ in,
-                                                     double* __restrict__ out, double eh) {
-  k_ts_explicit_body<D>(P, blockIdx.x, gridDim.x, in, out, eh);
+                                                     double* __restrict__ out, double eh, double e1) {
+  k_ts_explicit_body<D>(P, blockIdx.x, gridDim.x, in, out, eh, e1);
 }
 
 // ---------------------------------------------------------------------------
-// The persistent line sweep.  Shape: CH rows per staged chunk, NS chunks in
-// the ring (both powers of two), NT threads per CTA (one CTA per SM).
+// The line solves of one direction.  A CTA takes a tile of NL lines, keeps it
+// in shared memory from the right-hand side to the solution, and leaves:
+//   load    all threads build the right-hand sides of the tile's regular rows
+//           (the line's stencil, or for the Douglas-ADI x solve the whole
+//           first right-hand side, douglas_adi.cc:89-359) with every load
+//           coalesced and several rows in flight per thread;
+//   blocks  a thread per MIB block builds its rows' right-hand sides (the
+//           explicit MIB stencil of douglas_adi.cc:112-210 / lod.cc:337-496,
+//           the jump terms of D_xx_l lod.cc:960-1097, the Convert2Tri row
+//           operations) from the line's own values;
+//   solve   one warp runs the Thomas recurrences, a lane per line, forward
+//           and back, in place in shared memory, the rows' factors copied in
+//           ahead of use;
+//   store   all threads write the tile back, coalesced.
+// Interior lines are taken in the order of Dev::lperm: the lines that cross
+// the interface, whose tiles take longest, then the others by side, each in
+// memory order.  Tiles are full whatever the grid's extents.  CTAs past the
+// tiles write the face lines.
 //
-// Shared memory per thread column: three staged fields of NS*CH rows
-// (forward: stencil field, added field, bet from the first MIB row on;
-// backward: d'_j, gam_{j+1}).  Whole chunks are staged without per-row bound
-// checks: every field the sweep reads (the solution fields, the per-node
-// factors, the d' scratch) carries kRowPad rows of slack past its last row,
-// so the rows of a line's last chunk beyond n are readable (and never used).
-// The forward pass handles a chunk of regular rows (no MIB row, no line end)
-// with a fully unrolled loop at compile-time shared-memory offsets whose
-// stencil window slides in registers; chunks that hold a MIB block or a line
-// end take the row-by-row path.  The backward pass does the same for chunks
-// without the line end (and without the LOD epilogue).
+// What bounds it: the recurrence is one dependent chain a row, so a tile
+// costs its line's length whatever its width (one warp, B200: 88 clocks a row
+// forward and back, 130 with the lines' own factors), and an SM solves as many
+// lines at once as its shared memory holds (32 lines of 257 rows take 68 KB:
+// 3 tiles); the other tiles' loads and stores overlap the chains.  Up to 4
+// tiles an SM (129^3) the step is one tile's latency; at 257^3 the loads are
+// the longer part, held to about 3.9 TB/s by the small L1 that the tiles
+// leave (a plain tile copy: 5.9 TB/s with 1 KB of shared memory per CTA, 3.9
+// with 36 KB or more).  Against one line per thread over a ring of staged
+// rows with the partial solutions in a global scratch (the form before), us
+// per step: 65^3 Douglas-ADI 158 -> 54, 129^3 LOD-CN 277 -> 84, 113 x 97 x
+// 141 TS 252 -> 99, 257^3 Douglas-ADI 688 -> 680.
 
-struct BlockHead {
-  int L, kind, sides;
-  double a0, a1, a2;  // sub-diagonal of the block's rows after Convert2Tri
-  double r0, r1, r2;  // their right-hand sides this sweep (block pre-pass)
-};
+// Lines per tile and threads per CTA of each shape (mts_set_sweep_shape).
+#define MTS_SHAPES(X)                                                                           \
+  X(0, 32, 256) X(1, 32, 128) X(2, 32, 192) X(3, 16, 256) X(4, 16, 128) X(5, 16, 96) X(6, 8, 128) \
+  X(7, 8, 96) X(8, 4, 128) X(9, 4, 96)
 
-__device__ __forceinline__ void load_head(const MibBlock* blk, const double* rblk, int k, int end,
-                                          BlockHead& h) {
-  if (k < end) {
-    const MibBlock& b = blk[k];
-    h.L = b.L;
-    h.kind = b.kind;
-    h.sides = b.sides;
-    h.a0 = b.ia[0];
-    h.a1 = b.ia[1];
-    h.a2 = b.ia[2];
-    h.r0 = rblk[3 * k];
-    h.r1 = rblk[3 * k + 1];
-    h.r2 = rblk[3 * k + 2];
-  } else {
-    h.L = 0x7fffffff;
-    h.kind = 0;
-    h.sides = 0;
+// Doubles per row of a tile: an x tile is written along its lines, so its
+// rows are padded to an odd stride.
+template <int D, int NL>
+__host__ __device__ constexpr int tile_row() { return D == 0 ? NL + 1 : NL; }
+// Rows of a chunk of the lines' own factors while a tile is solved: 8, or 4
+// for x lines, where the smaller buffers let an SM hold three 257-row tiles
+// (257^3: x 229 against 244 us; y and z, whose loads gain from the L1 that two
+// tiles leave, 195 and 213 against 196 and 233).
+template <int D>
+__host__ __device__ constexpr int own_rows() { return D == 0 ? 4 : 8; }
+// Bytes for the factors: those of a side ((bet, 1/bet), gam by row), or two
+// chunks of the lines' own ((bet, 1/bet), a).
+template <int D, int NL>
+__host__ __device__ constexpr int factor_bytes(int n) {
+  const int side = (24 * n + 15) / 16 * 16, own = 2 * 24 * NL * own_rows<D>();
+  return side > own ? side : own;
+}
+template <int D, int NL>
+constexpr size_t tile_smem(int n) {
+  return factor_bytes<D, NL>(n) + sizeof(double) * (size_t)n * tile_row<D, NL>();
+}
+
+// Interior lines of direction D.
+template <int D>
+__host__ __device__ __forceinline__ long long interior_lines(const Dev& P) {
+  return (long long)((D == 0 ? P.ny : P.nx) - 2) * ((D == 2 ? P.ny : P.nz) - 2);
+}
+
+template <int D>
+__device__ __forceinline__ long long line_base(const Dev& P, int i1, int i2) {
+  if (D == 0) return (long long)P.nx * (i1 + (long long)P.ny * i2);
+  if (D == 1) return i1 + (long long)P.nx * P.ny * i2;
+  return i1 + (long long)P.nx * i2;
+}
+
+// Face lines of direction D, all their nodes: Outer_u(t_next), with dt f
+// added after the last sweep of a LOD step.
+template <int D>
+__device__ __forceinline__ void face_lines(const Dev& P, unsigned cta, unsigned ncta, const SweepIO& io, double E1) {
+  if (!io.bmode) return;
+  const int n = D == 0 ? P.nx : D == 1 ? P.ny : P.nz;
+  const int n1 = D == 0 ? P.ny : P.nx, n2 = D == 2 ? P.ny : P.nz;
+  const long long s = D == 0 ? 1 : D == 1 ? (long long)P.nx : (long long)P.nx * P.ny;
+  const int nf = 2 * n1 + 2 * (n2 - 2);
+  const long long total = (long long)nf * n;
+  for (long long e = (long long)cta * blockDim.x + threadIdx.x; e < total; e += (long long)ncta * blockDim.x) {
+    int f, j;  // neighbouring threads: neighbouring nodes in memory
+    if (D == 0) {
+      f = (int)(e / n);
+      j = (int)(e % n);
+    } else {
+      j = (int)(e / nf);
+      f = (int)(e % nf);
+    }
+    int i1, i2;
+    if (f < 2 * n1) {
+      i1 = f % n1;
+      i2 = f < n1 ? 0 : n2 - 1;
+    } else {
+      i2 = 1 + (f - 2 * n1) % (n2 - 2);
+      i1 = f - 2 * n1 < n2 - 2 ? 0 : n1 - 1;
+    }
+    const long long m = line_base<D>(P, i1, i2) + j * s;
+    const int ix = D == 0 ? j : i1;
+    const int iy = D == 0 ? i1 : D == 1 ? j : i2;
+    const int iz = D == 2 ? j : i2;
+    double v = outer_u(P, E1, ix, iy, iz);
+    if (io.bmode == 2) v = v + P.dt * source(P, E1, P.tag[m] & TAG_OUT, ix, iy, iz);
+    io.out[m] = v;
   }
 }
 
-// Block pre-pass of a sweep: one thread per MIB block of direction D computes
-// the right-hand sides of the block's rows exactly as the sweep would (the
-// explicit MIB stencil of douglas_adi.cc:112-210 / lod.cc:337-496, the jump
-// terms of D_xx_l lod.cc:960-1097, the Convert2Tri row operations) and stores
-// them for the sweep, which then spends no time on MIB data.
-template <int D, int KIND>
-__device__ __forceinline__ void k_block_rhs_body(const Dev& P, unsigned cta_, unsigned ncta_, const SweepIO io,
-                                                 int nblk) {
-  const int k = cta_ * TPB + threadIdx.x;
-  if (k >= nblk) return;
+// Right-hand sides of block k's rows (K_COPY, K_STENCIL, K_TS_Z) from the
+// fields, jump terms and Convert2Tri row operations included.  row0: the
+// shared-memory row 0 of the line.
+template <int D, int KIND, int RS>
+__device__ __forceinline__ void block_rhs(const Dev& P, const SweepIO& io, double E0, double E1, int k, long long base,
+                                       int i1, int i2, double* row0) {
+  const long long s = D == 0 ? 1 : D == 1 ? (long long)P.nx : (long long)P.nx * P.ny;
   const MibBlock& b = P.blk[D][k];
-  const int n2 = D == 2 ? P.ny : P.nz;
-  Line L;
-  decode_line<D>(P, (long long)(b.line % n2) * (D == 0 ? P.ny : P.nx) + b.line / n2, L);
-  const double* stin = KIND == K_COPY ? io.add : io.stin;
-  const double e0 = step_e(P, io.e0, 0), e1 = step_e(P, io.e1, 2);
-  auto U = [&](int j) { return stin[L.base + (long long)j * L.s]; };
+  double2 Jl = make_double2(0.0, 0.0), Jr = Jl;
+  if (io.jumps) {
+    Jl = jump_at(P, b.c0, E1);
+    if (b.kind == 3) Jr = jump_at(P, b.c1, E1);
+  }
+  const double* const stin = KIND == K_COPY ? io.add : io.stin;
+  auto U = [&](int j) { return stin[base + (long long)j * s]; };
   double r[3] = {0.0, 0.0, 0.0};
   for (int q = 0; q < b.kind; q++) {
     const int jj = b.L + q;
     const int side = (b.sides >> q) & 1;
-    const double av = io.add[L.base + (long long)jj * L.s];
+    const double av = io.add[base + (long long)jj * s];
     if (KIND == K_COPY) {
       r[q] = av;
     } else {
-      double sum = mib_sum(b, q, U, P.vd[D][side], io.jumps, P.jv);
+      const double sum = mib_sum(b, q, U, P.vd[D][side], io.jumps, Jl, Jr);
       double v = io.k * sum + av;
       if (KIND == K_TS_Z) {
-        int ix, iy, iz;
-        node_of<D>(L, jj, ix, iy, iz);
-        v = v + P.hdt * source(P, e0, side, ix, iy, iz);
-        v = v + P.hdt * source(P, e1, side, ix, iy, iz);
+        v = v + P.hdt * source(P, E0, side, i1, i2, jj);
+        v = v + P.hdt * source(P, E1, side, i1, i2, jj);
       }
       r[q] = v;
     }
   }
   implicit_rows(P, b, r, P.vd[D][b.sides & 1], P.vd[D][(b.sides >> 1) & 1], P.vd[D][(b.sides >> 2) & 1], io.jumps,
-                P.jv);
-  for (int q = 0; q < 3; q++) P.rblk[D][3 * k + q] = r[q];
+                Jl, Jr);
+  for (int q = 0; q < b.kind; q++) row0[(b.L + q) * RS] = r[q];
 }
 
-template <int D, int KIND>
-__global__ void __launch_bounds__(TPB) k_block_rhs(const __grid_constant__ Dev P, const SweepIO io, int nblk) {
-  k_block_rhs_body<D, KIND>(P, blockIdx.x, gridDim.x, io, nblk);
+// The Convert2Tri row operations of x block k on the first right-hand side's
+// rows in shared memory (Douglas-ADI).
+template <int RS>
+__device__ __forceinline__ void block_ops(const Dev& P, int k, double* row0) {
+  const MibBlock& b = P.blk[0][k];
+  double* const r0 = row0 + b.L * RS;
+  double r[3] = {r0[0], r0[RS], b.kind == 3 ? r0[2 * RS] : 0.0};
+  implicit_rows(P, b, r, nullptr, nullptr, nullptr, false, make_double2(0.0, 0.0), make_double2(0.0, 0.0));
+  for (int q = 0; q < b.kind; q++) r0[q * RS] = r[q];
 }
 
-// Exact-solution parts along a line: the fixed axes are read once per line,
-// the sweep axis from shared memory.  S = (sin2x cos2y) sin2z and
-// R2 = (x*x + y*y) + z*z keep the operand order of the exact-solution code,
-// so S*E and R2*E are the inner and outer solutions bit for bit.
-struct LineExact {
-  double x, y, z, s2x, c2y, s2z;
-};
-
-template <int D>
-__device__ __forceinline__ void line_exact(const Dev& P, const Line& L, LineExact& f) {
-  int ix, iy, iz;
-  node_of<D>(L, 0, ix, iy, iz);
-  f.x = P.ax[0][ix];
-  f.y = P.ax[1][iy];
-  f.z = P.ax[2][iz];
-  f.s2x = P.s2[0][ix];
-  f.c2y = P.c2[1][iy];
-  f.s2z = P.s2[2][iz];
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
+  unsigned s = (unsigned)__cvta_generic_to_shared(smem_dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gsrc) : "memory");
 }
 
-// sX: [coordinate | sin 2x | cos 2x] of the sweep axis, nd rows each.
-template <int D>
-__device__ __forceinline__ void row_parts(const LineExact& f, const double* sX, int nd, int j, double& S,
-                                          double& R2) {
-  if (D == 0) {
-    const double x = sX[j];
-    S = (sX[nd + j] * f.c2y) * f.s2z;
-    R2 = (x * x + f.y * f.y) + f.z * f.z;
-  } else if (D == 1) {
-    const double y = sX[j];
-    S = (f.s2x * sX[2 * nd + j]) * f.s2z;
-    R2 = (f.x * f.x + y * y) + f.z * f.z;
-  } else {
-    const double z = sX[j];
-    S = (f.s2x * f.c2y) * sX[nd + j];
-    R2 = (f.x * f.x + f.y * f.y) + z * z;
+// Quotients from the reciprocal.  With y = 1/b rounded to nearest, the
+// quotient of n by b is formed as
+//   t = n (y (1 - b y)),  q0 = n y + t,  q = q0 + (n - b q0) y
+// with fused multiply-adds.  1 - b y is exact, so q0 is n (1/b) to a relative
+// 2^-104 before its own rounding, one of the two doubles around n/b, and then
+// q is the correctly rounded quotient (Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", 1990: from y correctly
+// rounded and q0 within one unit, one correction by the exact remainder).
+// That holds while nothing over- or underflows on the way: |b| in [2^-100,
+// 2^100] (checked where the factors are made, Dev::plain_div) and |q| in
+// [2^-800, 2^800].  A tile with a quotient outside that (zeros, infinities
+// and NaN among them) is built and solved again with the divide.
+// One warp alone (B200): 52 clocks a row of the recurrence against 125 with
+// the divide, whose own reciprocal and tests are on the chain.
+constexpr unsigned kQLo = (1023u - 800u) << 21, kQRange = 1600u << 21;
+__device__ __forceinline__ bool quotient_out(double q) {
+  return ((unsigned)__double2hiint(q) << 1) - kQLo >= kQRange;
+}
+
+// G rows of the forward recurrence d_j = (r_j - a_j d_{j-1}) / bet_j (TDMA,
+// douglas_adi.cc:1794-1800): r in, d out, d_{j-1} of the first row in d.
+// f: (bet, 1/bet) by row.
+template <int G, bool PLAIN>
+__device__ __forceinline__ void forward_rows(double (&r)[G], const double (&a)[G], const double2 (&f)[G], double& d) {
+#pragma unroll
+  for (int k = 0; k < G; k++) {
+    const double nn = r[k] - a[k] * d;
+    const double b = f[k].x, y = f[k].y;
+    if (PLAIN) {
+      d = nn / b;
+    } else {
+      const double yl = y * __fma_rn(-b, y, 1.0);
+      const double q0 = __fma_rn(nn, y, nn * yl);
+      d = __fma_rn(__fma_rn(-b, q0, nn), y, q0);
+    }
+    r[k] = d;
   }
 }
-__device__ __forceinline__ double outer_from(const Dev& P, double R2, double E) {
-  return P.eq == 0 ? 100.0 : R2 * E;
-}
-__device__ __forceinline__ double source_from(const Dev& P, double S, double R2, double E, int out) {
-  if (P.eq == 0) return 0.0;
-  if (out) return -(R2 * E) - P.c6bo * E;
-  return P.kin * (S * E);
+
+// The recurrences of a line whose rows are its side's, with the row factors
+// of that side in shared memory ((bet, 1/bet) and gam_{j+1} by row); row0:
+// row 0 of the line, right-hand sides in, solution out.  Returns whether a
+// quotient is out of range.
+template <int RS, bool PLAIN>
+__device__ __forceinline__ bool solve_side(const double2* bet, const double* gam, double ac, double* row0, int n) {
+  constexpr int G = 4;
+  const int last = n - 1;
+  double d = 0.0;
+  auto single = [&](int j, double aj) {
+    const double a[1] = {aj};
+    const double2 f[1] = {bet[j]};
+    double r[1] = {row0[j * RS]};
+    forward_rows<1, PLAIN>(r, a, f, d);
+    row0[j * RS] = d;
+  };
+  single(0, 0.0);  // (the end rows are identities)
+  double a[G], r[G], rn[G];
+  double2 f[G], fn[G];
+#pragma unroll
+  for (int k = 0; k < G; k++) a[k] = ac;
+  int j = 1;
+  auto ahead = [&](int at) {
+#pragma unroll
+    for (int k = 0; k < G; k++) {
+      rn[k] = row0[(at + k) * RS];
+      fn[k] = bet[at + k];
+    }
+  };
+  if (j + G <= last) ahead(j);
+  for (; j + G <= last; j += G) {
+#pragma unroll
+    for (int k = 0; k < G; k++) {
+      r[k] = rn[k];
+      f[k] = fn[k];
+    }
+    // the next rows, off the chain (for the last group any will do)
+    ahead(j + 2 * G <= last ? j + G : j);
+    forward_rows<G, PLAIN>(r, a, f, d);
+#pragma unroll
+    for (int k = 0; k < G; k++) row0[(j + k) * RS] = r[k];
+  }
+  for (; j < n; j++) single(j, j == last ? 0.0 : ac);
+
+  // back: u_j = d_j - gam_{j+1} u_{j+1} (douglas_adi.cc:1805-1806)
+  double u = d, g[G], gn[G];
+  bool out = quotient_out(d);
+  j = n - 2;
+  auto behind = [&](int at) {
+#pragma unroll
+    for (int k = 0; k < G; k++) {
+      rn[k] = row0[(at - k) * RS];
+      gn[k] = gam[at - k];
+    }
+  };
+  if (j - G + 1 >= 0) behind(j);
+  for (; j - G + 1 >= 0; j -= G) {
+#pragma unroll
+    for (int k = 0; k < G; k++) {
+      r[k] = rn[k];
+      g[k] = gn[k];
+    }
+    behind(j - 2 * G + 1 >= 0 ? j - G : j);
+#pragma unroll
+    for (int k = 0; k < G; k++) {
+      out |= quotient_out(r[k]);
+      r[k] -= g[k] * u;
+      u = r[k];
+      row0[(j - k) * RS] = u;
+    }
+  }
+  for (; j >= 0; j--) {
+    double v = row0[j * RS];
+    out |= quotient_out(v);
+    v -= gam[j] * u;
+    u = v;
+    row0[j * RS] = u;
+  }
+  return out;
 }
 
-// Shared memory of a shape: the staging ring, the two prefix factor tables
-// of the sweep direction (2 sides x 2 values x n rows) and its exact-solution
-// tables (3 x n).
-template <int CH, int NS, int NT, int D = 0>
-constexpr size_t shape_smem(int n) {
-  // D = 0 pads each ring row by 4 doubles (the x sweeps' cooperative staging);
-  // the default D = 0 is the largest, used for the fit check
-  return sizeof(double) * ((size_t)3 * NS * CH * (D == 0 ? NT + 4 : NT) + (size_t)7 * n);
-}
+// Named barriers of two warps: one arrives and goes on, the other waits.
+__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;\n" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void pair_arrive(int id) { asm volatile("bar.arrive %0, 64;\n" ::"r"(id) : "memory"); }
 
-
-template <int D, int KIND, int CH, int NS, int NT>
-__device__ __forceinline__ void k_sweep_body(const Dev& P, unsigned cta_, unsigned ncta_, const SweepIO io) {
-  static_assert((CH & (CH - 1)) == 0 && (NS & (NS - 1)) == 0 && NS >= 4 && CH >= 4, "shape");
-  static_assert(CH <= kRowPad, "chunk rows past a line end must stay within the fields' slack");
-  constexpr int RING = NS * CH;    // rows in a field's ring
-  // x lines (kCoop, below) are staged by the warp together, with 4 doubles of
-  // padding per ring row so that a copy instruction's lanes, which write
-  // CH rows of 32/CH columns, fall on distinct banks in pairs
-  constexpr int RS = D == 0 ? NT + 4 : NT;  // doubles per ring row
-  constexpr int SLOT = CH * RS;    // doubles per chunk slot
-  extern __shared__ double sm[];
-  const int tid = threadIdx.x;
-  double* const sA = sm + tid;             // [NS][CH][NT]
-  double* const sB = sA + NS * SLOT;       // [NS][CH][NT]
-  double* const sC = sB + NS * SLOT;       // [NS][CH][NT]
-#define SA(j) sA[((j) & (RING - 1)) * RS]
-#define SB(j) sB[((j) & (RING - 1)) * RS]
-#define SC(j) sC[((j) & (RING - 1)) * RS]
-  const long long T = (long long)ncta_ * NT;
-  const long long gt = (long long)cta_ * NT + tid;
-  double* const dp = P.dp + gt;
-  const long long nl = nlines<D>(P);
-  const MibBlock* __restrict__ blk = P.blk[D];
-  const double* __restrict__ fbet = P.fbet[D];
-  const double* __restrict__ fgam = P.fgam[D];
-  const double* __restrict__ rblk = P.rblk[D];
-  const double E1 = step_e(P, io.e1, 2);
-  const double E0 = step_e(P, io.e0, 0);
-  const double kx = io.k;
-  // per-direction constants by side (0 inside, 1 outside), in registers
-  const double v0i = P.vd[D][0][0], v0o = P.vd[D][1][0];
-  const double v1i = P.vd[D][0][1], v1o = P.vd[D][1][1];
-  const double v2i = P.vd[D][0][2], v2o = P.vd[D][1][2];
-  const double cai = P.ia[D][0], cao = P.ia[D][1];
-  // prefix factor tables [side][row][bet, gam] and exact-solution tables of
-  // the sweep axis [coordinate | sin 2x | cos 2x] into shared memory (they sit
-  // on the recurrence chain; the staging stream would evict them from L1)
-  const int nd = D == 0 ? P.nx : D == 1 ? P.ny : P.nz;
-  double* const sP = sm + 3 * NS * SLOT;
-  double* const sX = sP + 4 * nd;
-  for (int i = tid; i < 4 * nd; i += NT) sP[i] = i < 2 * nd ? P.ptab[D][0][i] : P.ptab[D][1][i - 2 * nd];
-  for (int i = tid; i < nd; i += NT) {
-    sX[i] = P.ax[D][i];
-    sX[nd + i] = P.s2[D][i];
-    sX[2 * nd + i] = P.c2[D][i];
+// The same for a tile with lines of their own factors, called by the whole
+// CTA: of row j of this lane's line a_j at fa[j st], (bet_j, 1/bet_j) at
+// fb[j st], gam_{j+1} at g[j st].  Up to seven other warps bring the factors
+// in, OWN_C rows a chunk in turn: each holds its next chunk in registers and
+// puts it down in one of two buffers (buf) once warp ws, which solves, is
+// done with the chunk two before.  Barrier 1 + p: a chunk of producer p is
+// down; 8 + p: its buffer is free.  (Two producers at least: a producer's
+// next chunk waits for a chunk that the solving warp takes no earlier than
+// its last one, so neither barrier is arrived at twice in a round.)
+template <int NL, int RS, int NW, int C, bool PLAIN>
+__device__ __forceinline__ bool solve_own(const double* __restrict__ fa, const double2* __restrict__ fb,
+                                          const double* __restrict__ g, long long st, double* buf, double* row0, int n,
+                                          int ws) {
+  constexpr int NP = NW - 1 < 7 ? NW - 1 : 7;  // producers
+  static_assert(NP >= 2, "two producers");
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const bool on = lane < NL;
+  const int last = n - 1;
+  double2* const bb = reinterpret_cast<double2*>(buf) + lane;  // [2][C][NL]
+  double* const ba = buf + 4 * C * NL + lane;                  // [2][C][NL]
+  const int chunks = (n + C - 1) / C;
+  if (w != ws) {
+    const int p = (w - ws - 1 + NW) % NW;
+    double a[C];
+    double2 f[C];
+    if (p < NP) {
+      auto fetch = [&](int k) {
+        if (on && k < chunks) {
+#pragma unroll
+          for (int e = 0; e < C; e++) {
+            const long long o = (long long)min(k * C + e, last) * st;
+            a[e] = fa[o];
+            f[e] = fb[o];
+          }
+        }
+      };
+      fetch(p);
+      for (int k = p; k < chunks; k += NP) {
+        if (k >= 2) pair_sync(8 + p);
+        if (on) {
+#pragma unroll
+          for (int e = 0; e < C; e++) {
+            ba[((k & 1) * C + e) * NL] = a[e];
+            bb[((k & 1) * C + e) * NL] = f[e];
+          }
+        }
+        __syncwarp();
+        pair_arrive(1 + p);
+        fetch(k + NP);
+      }
+    }
+    __syncthreads();
+    if (p < NP) {
+      const double* const gl = g + (long long)last * st;
+      auto fetch = [&](int k) {
+        if (on && k < chunks) {
+#pragma unroll
+          for (int e = 0; e < C; e++) a[e] = gl[-(long long)min(k * C + e, last) * st];
+        }
+      };
+      fetch(p);
+      for (int k = p; k < chunks; k += NP) {
+        if (k >= 2) pair_sync(8 + p);
+        if (on) {
+#pragma unroll
+          for (int e = 0; e < C; e++) ba[((k & 1) * C + e) * NL] = a[e];
+        }
+        __syncwarp();
+        pair_arrive(1 + p);
+        fetch(k + NP);
+      }
+    }
+    return false;
+  }
+  // the solving warp: forward
+  bool out = false;
+  double d = 0.0;
+  for (int k = 0, q = 0, q2 = 2 % NP; k < chunks; k++) {
+    pair_sync(1 + q);
+    if (on) {
+      double a[C], r[C];
+      double2 f[C];
+#pragma unroll
+      for (int e = 0; e < C; e++) {
+        a[e] = ba[((k & 1) * C + e) * NL];
+        f[e] = bb[((k & 1) * C + e) * NL];
+        r[e] = row0[min(k * C + e, last) * RS];
+      }
+      // (rows past the end repeat the last one's inputs; not stored)
+      forward_rows<C, PLAIN>(r, a, f, d);
+#pragma unroll
+      for (int e = 0; e < C; e++)
+        if (k * C + e < n) row0[(k * C + e) * RS] = r[e];
+    }
+    __syncwarp();
+    if (k + 2 < chunks) pair_arrive(8 + q2);
+    q = q + 1 < NP ? q + 1 : 0;
+    q2 = q2 + 1 < NP ? q2 + 1 : 0;
   }
   __syncthreads();
-
-  // x lines are contiguous in memory and 2 KB apart, so a thread staging its
-  // own line would touch 32 segments per warp instruction.  There the warp
-  // stages and stores its 32 lines together (kCoop): lane e of copy q moves
-  // row e % CH of line e / CH, so runs of CH lanes read one line's
-  // consecutive rows, into that line's column of the ring.  The warp then
-  // walks its lines' chunks in step, including lanes whose line is a face
-  // line or past the end, which only help with the copies.
-  constexpr bool kCoop = D == 0;
-  const int lane = tid & 31;
-  double* const sAw = sm + (tid - lane);  // the warp's first column of ring A
-  const long long nxl = P.nx;
-
-  for (long long t0 = gt - (kCoop ? lane : 0); t0 < nl; t0 += T) {
-    const long long t = kCoop ? t0 + lane : t0;
-    const bool act = t < nl;
-    Line L;
-    decode_line<D>(P, act ? t : nl - 1, L);
-    const int n = L.n;
-    const long long s = L.s;
-    LineExact fx;
-    line_exact<D>(P, L, fx);
-    if (L.boundary && act) {
-      if (io.bmode) {
-        for (int j = 0; j < n; j++) {
-          long long m = L.base + (long long)j * s;
-          double S, R2;
-          row_parts<D>(fx, sX, nd, j, S, R2);
-          double v = outer_from(P, R2, E1);
-          if (io.bmode == 2) v = v + P.dt * source_from(P, S, R2, E1, P.tag[m] & TAG_OUT);
-          io.out[m] = v;
+  // back, rows counted from the last (gam_n = 0)
+  double* const rl = row0 + last * RS;
+  double u = 0.0;
+  for (int k = 0, q = 0, q2 = 2 % NP; k < chunks; k++) {
+    pair_sync(1 + q);
+    if (on) {
+      double a[C], r[C];
+#pragma unroll
+      for (int e = 0; e < C; e++) {
+        a[e] = ba[((k & 1) * C + e) * NL];
+        r[e] = rl[-min(k * C + e, last) * RS];
+      }
+#pragma unroll
+      for (int e = 0; e < C; e++) {
+        if (k * C + e < n) {
+          out |= quotient_out(r[e]);
+          r[e] -= a[e] * u;
+          u = r[e];
+          rl[-(k * C + e) * RS] = u;
         }
       }
     }
-    const bool solve = act && !L.boundary;
-    if (!kCoop && !solve) continue;
-    unsigned solvers = 0;
-    if (kCoop) {
-      __syncwarp();
-      solvers = __ballot_sync(0xffffffffu, solve);
-      if (!solvers) continue;
-    }
-    const int nch = (n + CH - 1) / CH;
-    const int ls = P.lside[D][L.lid];
-    const int bfirst = P.bstart[D][L.lid];
-    const int bend = P.bstart[D][L.lid + 1];
-    const int L1 = bfirst < bend ? blk[bfirst].L : n;  // first MIB row
-    const double* pt = sP + ((ls >> 1) & 1) * 2 * nd;
-    const bool two = KIND != K_COPY && io.add != io.stin;
-    // row j of a field: g[j*s]; rows up to nch*CH-1 are readable (the fields
-    // carry one chunk of slack past their end)
-    const double* gA = (KIND == K_COPY ? io.add : io.stin) + L.base;
-    const double* gB = io.add + L.base;
-    const double* gC = fbet + L.base;
-    // kCoop: the first MIB row of the line each of this lane's copies serves
-    int L1q[CH];
-    long long gq[CH];  // start of the line each copy serves, or -1 past the end
-    if (kCoop) {
-#pragma unroll
-      for (int q = 0; q < CH; q++) {
-        const int l = (q * 32 + lane) / CH;
-        L1q[q] = __shfl_sync(0xffffffffu, L1, l);
-        gq[q] = t0 + l < nl ? (t0 + l) * nxl + (q * 32 + lane) % CH : -1;
-      }
-    }
-    auto stage = [&](int c) {
-      if (kCoop) {
-        if (c < nch) {
-          const double* fA = KIND == K_COPY ? io.add : io.stin;
-          double* aw = sAw + (c & (NS - 1)) * SLOT;
-          double* bw = aw + NS * SLOT;
-          double* cw = bw + NS * SLOT;
-#pragma unroll
-          for (int q = 0; q < CH; q++) {
-            const int e = q * 32 + lane, l = e / CH, r = e % CH;
-            if (gq[q] >= 0) {
-              const long long g = gq[q] + (long long)c * CH;
-              cp_async8(aw + r * RS + l, fA + g);
-              if (two) cp_async8(bw + r * RS + l, io.add + g);
-              if ((c + 1) * CH > L1q[q] && L1q[q] < n) cp_async8(cw + r * RS + l, fbet + g);
-            }
-          }
-        }
-        cp_async_commit();
-        return;
-      }
-      if (c < nch) {
-        const long long off = (long long)c * CH * s;
-        double* a = sA + (c & (NS - 1)) * SLOT;
-#pragma unroll
-        for (int r = 0; r < CH; r++) cp_async8(a + r * RS, gA + off + r * s);
-        if (two) {
-          double* b = sB + (c & (NS - 1)) * SLOT;
-#pragma unroll
-          for (int r = 0; r < CH; r++) cp_async8(b + r * RS, gB + off + r * s);
-        }
-        if ((c + 1) * CH > L1 && L1 < n) {  // per-node factors exist only for lines with blocks
-          double* cc = sC + (c & (NS - 1)) * SLOT;
-#pragma unroll
-          for (int r = 0; r < CH; r++) cp_async8(cc + r * RS, gC + off + r * s);
-        }
-      }
-      cp_async_commit();
-    };
-    auto outer_at = [&](int j) -> double {
-      double S, R2;
-      row_parts<D>(fx, sX, nd, j, S, R2);
-      return outer_from(P, R2, E1);
-    };
-    // right-hand side of a regular row from its stencil values
-    auto rhs = [&](int j, double xm, double x0, double xp, double addv, double w0, double w1, double w2,
-                   int side) -> double {
-      if (KIND == K_COPY) return x0;
-      double sum = 0.0;
-      sum += xm * w0;
-      sum += x0 * w1;
-      sum += xp * w2;
-      double r = kx * sum + addv;
-      if (KIND == K_TS_Z) {
-        double S, R2;
-        row_parts<D>(fx, sX, nd, j, S, R2);
-        r = r + P.hdt * source_from(P, S, R2, E0, side);
-        r = r + P.hdt * source_from(P, S, R2, E1, side);
-      }
-      return r;
-    };
-
-    // ---- forward substitution with the precomputed factors (TDMA,
-    // douglas_adi.cc:1794-1800): d'_j = (r_j - a_j d'_{j-1}) / bet_j
-    for (int c = 0; c < NS - 2; c++) stage(c);
-    int mb = bfirst;
-    BlockHead hb, hb2;  // the next block and the one after (prefetched)
-    load_head(blk, rblk, mb, bend, hb);
-    load_head(blk, rblk, mb + 1, bend, hb2);
-    int mside = (ls >> 1) & 1;
-    double dprev = 0.0;
-    int j = 1;
-    for (int c = 0; c < nch; c++) {
-      if (kCoop) __syncwarp();  // every lane is done with the slot restaged next
-      stage(c + NS - 2);
-      cp_async_wait<NS - 3>();  // chunks c-1, c, c+1 resident
-      if (kCoop) {
-        __syncwarp();  // and the other lanes' copies into this lane's column visible
-        if (!solve) continue;
-      }
-      if (c == 0) {
-        dprev = outer_at(0) / pt[0];
-        dp[0] = dprev;
-      }
-      const int c0 = c * CH;
-      const int cend = min(c0 + CH, n - 1);
-      if (j >= cend) continue;
-      if (j == c0 && cend == c0 + CH && hb.L >= cend && (cend <= L1 || c0 >= L1)) {
-        // a chunk of regular rows, same side, factors from one source
-        const double w0 = mside ? v0o : v0i, w1 = mside ? v1o : v1i, w2 = mside ? v2o : v2i;
-        const double ac = mside ? cao : cai;
-        const double* a = sA + (c & (NS - 1)) * SLOT;
-        const double* ap = sA + ((c - 1) & (NS - 1)) * SLOT;
-        const double* an = sA + ((c + 1) & (NS - 1)) * SLOT;
-        const double* b = sB + (c & (NS - 1)) * SLOT;
-        double* q = dp + (long long)c0 * T;
-        auto run = [&](auto tag) {
-          // tag: bet from the staged per-node factors, else from the prefix table
-          constexpr bool kField = decltype(tag)::value;
-          const double* bt = kField ? sC + (c & (NS - 1)) * SLOT : pt + 2 * c0;
-          double xm = ap[(CH - 1) * RS];
-          double x0 = a[0];
-#pragma unroll
-          for (int rr = 0; rr < CH; rr++) {
-            const double xp = rr == CH - 1 ? an[0] : a[(rr + 1) * RS];
-            const double r = rhs(c0 + rr, xm, x0, xp, two ? b[rr * RS] : x0, w0, w1, w2, mside);
-            const double bet = kField ? bt[rr * RS] : bt[2 * rr];
-            const double d = (r - ac * dprev) / bet;
-            q[rr * T] = d;
-            dprev = d;
-            xm = x0;
-            x0 = xp;
-          }
-        };
-        if (c0 >= L1)
-          run(BoolC<true>{});
-        else
-          run(BoolC<false>{});
-        j = cend;
-      } else {
-        while (j < cend) {
-          const double bet = j >= L1 ? SC(j) : pt[2 * j];
-          if (j == hb.L) {
-            // a MIB block: its rows' right-hand sides come mixed from the
-            // block pre-pass (k_block_rhs); substitute them
-            double d = (hb.r0 - hb.a0 * dprev) / bet;
-            dp[(long long)j * T] = d;
-            dprev = d;
-            d = (hb.r1 - hb.a1 * dprev) / SC(j + 1);
-            dp[(long long)(j + 1) * T] = d;
-            dprev = d;
-            if (hb.kind == 3) {
-              d = (hb.r2 - hb.a2 * dprev) / SC(j + 2);
-              dp[(long long)(j + 2) * T] = d;
-              dprev = d;
-            }
-            mside = (hb.sides >> (hb.kind - 1)) & 1;
-            j += hb.kind;
-            mb++;
-            hb = hb2;
-            load_head(blk, rblk, mb + 1, bend, hb2);
-          } else {
-            const double r = rhs(j, SA(j - 1), SA(j), SA(j + 1), two ? SB(j) : SA(j), mside ? v0o : v0i,
-                                 mside ? v1o : v1i, mside ? v2o : v2i, mside);
-            const double d = (r - (mside ? cao : cai) * dprev) / bet;
-            dp[(long long)j * T] = d;
-            dprev = d;
-            j++;
-          }
-        }
-      }
-    }
-    if (solve) {
-      // last row: the Dirichlet identity row (a = 0)
-      const double r = outer_at(n - 1);
-      const double a = 0.0;
-      const double bet = n - 1 >= L1 ? SC(n - 1) : pt[2 * (n - 1)];
-      dp[(long long)(n - 1) * T] = (r - a * dprev) / bet;
-    }
-    cp_async_wait<0>();
-
-    // ---- back substitution u_j = d'_j - gam_{j+1} u_{j+1} (douglas_adi.cc:
-    // 1805-1806), staged back through the ring: field A = d'_j, field B =
-    // gam_{j+1} where it comes from the per-node factors.  The fence orders
-    // this thread's d' stores before the asynchronous copies that read them.
-    __threadfence_block();
-    const double* gG = fgam + L.base;
-    auto bstage = [&](int c) {
-      if (c >= 0) {
-        double* a = sA + (c & (NS - 1)) * SLOT;
-        const double* g = dp + (long long)c * CH * T;
-#pragma unroll
-        for (int r = 0; r < CH; r++) cp_async8(a + r * RS, g + r * T);
-        if ((c + 1) * CH >= L1 && L1 < n) {
-          double* b = sB + (c & (NS - 1)) * SLOT;
-          const long long off = ((long long)c * CH + 1) * s;
-#pragma unroll
-          for (int r = 0; r < CH; r++) cp_async8(b + r * RS, gG + off + r * s);
-        }
-      }
-      cp_async_commit();
-    };
-    // side tracking downwards (only the LOD epilogue needs it): below a block
-    // the side is that of the block's first row, above the last block that of
-    // its last row.
-    int db = bend - 1;
-    int dbL = db >= bfirst ? blk[db].L : -1, dbK = db >= bfirst ? blk[db].kind : 0;
-    int dbS = db >= bfirst ? blk[db].sides : 0;
-    int dside = db >= bfirst ? (dbS >> (dbK - 1)) & 1 : (ls >> 1) & 1;
-    double unext = 0.0;
-    for (int c = nch - 1; c > nch - NS; c--) bstage(c);
-    for (int c = nch - 1; c >= 0; c--) {
-      if (kCoop) __syncwarp();  // the previous chunk's stores have read its slot
-      bstage(c - NS + 1);
-      cp_async_wait<NS - 1>();
-      const int c0 = c * CH;
-      // kCoop: results go to this lane's column of the slot, then the warp
-      // stores its lines' rows together
-      double* const aslot = sA + (c & (NS - 1)) * SLOT;
-      if (!solve) {
-      } else if (!io.last && c0 + CH <= n - 1 && (c0 + CH < L1 || c0 + 1 >= L1)) {
-        // every row has a successor; gam_{j+1} from one source
-        double* a = aslot;
-        double* o = io.out + L.base + (long long)c0 * s;
-        auto run = [&](auto tag) {
-          // tag: gam_{j+1} from the staged per-node factors, else from the
-          // prefix table (pt + 2*c0 + 3 is gam of row c0 + 1)
-          constexpr bool kField = decltype(tag)::value;
-          const double* gb = kField ? sB + (c & (NS - 1)) * SLOT : pt + 2 * c0 + 3;
-#pragma unroll
-          for (int rr = CH - 1; rr >= 0; rr--) {
-            const double gm = kField ? gb[rr * RS] : gb[2 * rr];
-            double u = a[rr * RS];
-            u -= gm * unext;
-            unext = u;
-            if (kCoop)
-              a[rr * RS] = u;
-            else
-              o[rr * s] = u;
-          }
-        };
-        if (c0 + 1 >= L1)
-          run(BoolC<true>{});
-        else
-          run(BoolC<false>{});
-      } else {
-        for (int rr = CH - 1; rr >= 0; rr--) {
-          const int jj = c0 + rr;
-          if (jj >= n) continue;
-          double u = SA(jj);
-          if (jj != n - 1) u -= (jj + 1 >= L1 ? SB(jj) : pt[2 * (jj + 1) + 1]) * unext;
-          unext = u;
-          double v = u;
-          if (io.last) {
-            int side;
-            if (jj == 0) {
-              side = ls & 1;
-            } else if (jj == n - 1) {
-              side = (ls >> 2) & 1;
-            } else if (jj >= dbL && jj < dbL + dbK) {
-              side = (dbS >> (jj - dbL)) & 1;
-              if (jj == dbL) {
-                dside = dbS & 1;
-                db--;
-                if (db >= bfirst) {
-                  dbL = blk[db].L;
-                  dbK = blk[db].kind;
-                  dbS = blk[db].sides;
-                } else {
-                  dbL = -1;
-                  dbK = 0;
-                }
-              }
-            } else {
-              side = dside;
-            }
-            double S, R2;
-            row_parts<D>(fx, sX, nd, jj, S, R2);
-            v = u + P.dt * source_from(P, S, R2, E1, side);
-          }
-          if (kCoop)
-            SA(jj) = v;
-          else
-            io.out[L.base + (long long)jj * s] = v;
-        }
-      }
-      if (kCoop) {
-        __syncwarp();
-        const double* aw = sAw + (c & (NS - 1)) * SLOT;
-#pragma unroll
-        for (int q = 0; q < CH; q++) {
-          const int e = q * 32 + lane, l = e / CH, r = e % CH;
-          if (((solvers >> l) & 1u) && c0 + r < n) io.out[gq[q] + c0] = aw[r * RS + l];
-        }
-      }
-    }
-    cp_async_wait<0>();
+    __syncwarp();
+    if (k + 2 < chunks) pair_arrive(8 + q2);
+    q = q + 1 < NP ? q + 1 : 0;
+    q2 = q2 + 1 < NP ? q2 + 1 : 0;
   }
-#undef SA
-#undef SB
-#undef SC
+  return out;
 }
 
-template <int D, int KIND, int CH, int NS, int NT>
-__global__ void __launch_bounds__(NT, 1) k_sweep(const __grid_constant__ Dev P, const SweepIO io) {
-  k_sweep_body<D, KIND, CH, NS, NT>(P, blockIdx.x, gridDim.x, io);
+// What the phases of a tile share.
+template <int NL>
+struct TileState {
+  int i1[NL], i2[NL];  // the tile's lines
+  int next_task;       // of the load phase
+  int side;            // the side whose factors all its lines have, -1: not so
+  int again;           // a quotient was out of range
+};
+
+// The MIB rows' right-hand sides (the warps from BW on).
+template <int D, int KIND, int NL, int NT>
+__device__ __forceinline__ void tile_blocks(const Dev& P, const SweepIO& io, const TileState<NL>& T, double* sm, int t0,
+                                         int nlive) {
+  constexpr int RS = tile_row<D, NL>(), NW = NT / 32, BW = NW / 2;
+  const int tid = threadIdx.x, w = tid >> 5;
+  const double E1 = step_e(P, io.e1, 2);
+  if (KIND != K_ADI && P.nblk[D] > 0) {
+    const int e = tid - 32 * BW, c = e % NL;
+    if (c < nlive) {
+      const int i1 = T.i1[c], i2 = T.i2[c];
+      const int lid = i1 * (D == 2 ? P.ny : P.nz) + i2;
+      const int bend = P.bstart[D][lid + 1];
+      const long long base = line_base<D>(P, i1, i2);
+      const double E0 = KIND == K_TS_Z ? step_e(P, io.e0, 0) : 0.0;
+      for (int k = P.bstart[D][lid] + e / NL; k < bend; k += (NT - 32 * BW) / NL)
+        block_rhs<D, KIND, RS>(P, io, E0, E1, k, base, i1, i2, sm + c);
+    }
+  }
+}
+
+// The regular rows' right-hand sides: warps take tasks (a few rows of the
+// tile each) until none is left; all loads of a task are issued before any is
+// used.
+constexpr int TASK_ROWS = 6;
+template <int D, int KIND, int NL, int NT>
+__device__ __forceinline__ void tile_rows(const Dev& P, const SweepIO& io, TileState<NL>& T, double* sm, int nlive) {
+  constexpr int RS = tile_row<D, NL>();
+  const int lane = threadIdx.x & 31;
+  constexpr int SUB = 32 / NL;
+  const int n = D == 0 ? P.nx : D == 1 ? P.ny : P.nz;
+  const double E1 = step_e(P, io.e1, 2);
+  const double kx = io.k;
+  auto task = [&]() {
+    int t = 0;
+    if (lane == 0) t = atomicAdd(&T.next_task, 1);
+    return __shfl_sync(0xffffffffu, t, 0);
+  };
+  if (D != 0) {
+    // lanes: lines (32 / NL runs of rows at a time), U rows a lane; the last
+    // run is moved back to end with the line (the rows it shares with the one
+    // before get the same values twice)
+    const long long s = D == 1 ? (long long)P.nx : (long long)P.nx * P.ny;
+    const int c = lane % NL, sub = lane / NL;
+    const int i1 = T.i1[c], i2 = T.i2[c];
+    const long long base = line_base<D>(P, i1, i2);
+    const bool two = KIND != K_COPY && io.add != io.stin;
+    const double E0 = KIND == K_TS_Z ? step_e(P, io.e0, 0) : 0.0;
+    constexpr int flag = D == 1 ? TAG_MIBY : TAG_MIBZ;
+    auto run = [&](auto UU) {
+      constexpr int U = decltype(UU)::value;
+      for (int t = task(); t * (U * SUB) < n; t = task()) {
+        const int j0 = min((t * SUB + sub) * U, n - U);
+        const long long g0 = base + (long long)j0 * s;
+        double u[U + 2], av[U];
+        int tt[U];
+        {
+          const uint8_t* tg = P.tag + g0;
+          const double* gb = io.add + g0;
+#pragma unroll
+          for (int k = 0; k < U; k++, tg += s) tt[k] = *tg;
+          if (KIND == K_COPY || two) {
+#pragma unroll
+            for (int k = 0; k < U; k++, gb += s) av[k] = __ldcg(gb);
+          }
+        }
+        if (KIND != K_COPY) {
+          // (the neighbours past the line's ends are not used)
+          const double* ga = io.stin + g0;
+          u[0] = j0 > 0 ? __ldcg(ga - s) : 0.0;
+#pragma unroll
+          for (int k = 1; k <= U; k++, ga += s) u[k] = __ldcg(ga);
+          u[U + 1] = j0 + U < n ? __ldcg(ga) : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+          const int j = j0 + k;
+          double r;
+          if (KIND == K_COPY) {
+            r = av[k];
+          } else {
+            auto val = [&](auto S) {
+              constexpr int sd = decltype(S)::value;
+              double sum = 0.0;
+              sum += u[k] * P.vd[D][sd][0];
+              sum += u[k + 1] * P.vd[D][sd][1];
+              sum += u[k + 2] * P.vd[D][sd][2];
+              double v = kx * sum + (two ? av[k] : u[k + 1]);
+              if (KIND == K_TS_Z) {
+                v = v + P.hdt * source(P, E0, sd, i1, i2, j);
+                v = v + P.hdt * source(P, E1, sd, i1, i2, j);
+              }
+              return v;
+            };
+            r = (tt[k] & TAG_OUT) ? val(IntC<1>{}) : val(IntC<0>{});
+          }
+          if (j == 0 || j == n - 1) r = outer_u(P, E1, i1, D == 1 ? j : i2, D == 1 ? i2 : j);
+          if (!(tt[k] & flag) && c < nlive) sm[j * RS + c] = r;
+        }
+      }
+    };
+    if (n >= TASK_ROWS)
+      run(IntC<TASK_ROWS>{});
+    else
+      run(IntC<1>{});
+    return;
+  }
+  // lanes: 32 columns of U lines; the interior columns, then the two ends
+  constexpr int U = 4, GROUPS = (NL + U - 1) / U;
+  const int chunks = (n - 2 + 31) / 32;
+  for (int t = task(); t <= chunks * GROUPS; t = task()) {
+    if (t == chunks * GROUPS) {
+      for (int e = lane; e < 2 * nlive; e += 32) {
+        const int ix = (e & 1) ? n - 1 : 0;
+        sm[ix * RS + (e >> 1)] = outer_u(P, E1, ix, T.i1[e >> 1], T.i2[e >> 1]);
+      }
+      continue;
+    }
+    const int c0 = t / chunks * U;
+    if (c0 >= nlive) continue;
+    const int ixl = 1 + t % chunks * 32 + lane;
+    const int ix = min(ixl, n - 2);
+    const bool in = ixl < n - 1;
+    if (KIND != K_ADI) {
+      double um[U], uc[U], up[U], av[U];
+      int tt[U];
+#pragma unroll
+      for (int k = 0; k < U; k++) {
+        const int c = min(c0 + k, nlive - 1);
+        const long long m = line_base<0>(P, T.i1[c], T.i2[c]) + ix;
+        tt[k] = P.tag[m];
+        if (KIND == K_COPY) {
+          av[k] = io.add[m];
+        } else {
+          uc[k] = io.stin[m];
+          um[k] = io.stin[m - 1];
+          up[k] = io.stin[m + 1];
+          av[k] = io.add[m];
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < U; k++) {
+        double r;
+        if (KIND == K_COPY) {
+          r = av[k];
+        } else {
+          const bool out = tt[k] & TAG_OUT;
+          double sum = 0.0;
+          sum += um[k] * (out ? P.vd[0][1][0] : P.vd[0][0][0]);
+          sum += uc[k] * (out ? P.vd[0][1][1] : P.vd[0][0][1]);
+          sum += up[k] * (out ? P.vd[0][1][2] : P.vd[0][0][2]);
+          r = kx * sum + av[k];
+        }
+        if (in && c0 + k < nlive && !(tt[k] & TAG_MIBX)) sm[ix * RS + c0 + k] = r;
+      }
+    } else {
+      // Douglas-ADI: the first right-hand side ((dt D_yy u + dt D_zz u) + u)
+      // + dt src (douglas_adi.cc:89-359); the lines' y neighbours are one
+      // another where they lie in one plane
+      const double* const un = io.stin;
+      const long long sy = P.nx, sz = (long long)P.nx * P.ny;
+      const double dt = P.dt;
+      double um[U], uc[U], up[U], zm[U], zp[U];
+      int tt[U], yy[U], zz[U];
+      const double xv = P.ax[0][ix], s2x = P.s2[0][ix];
+      const double x2 = xv * xv;
+#pragma unroll
+      for (int k = 0; k < U; k++) {
+        const int c = min(c0 + k, nlive - 1);
+        yy[k] = T.i1[c];
+        zz[k] = T.i2[c];
+      }
+      bool plane = c0 + U <= nlive;  // four neighbours
+#pragma unroll
+      for (int k = 1; k < U; k++) plane = plane && yy[k] == yy[0] + k && zz[k] == zz[0];
+      if (plane) {
+        const long long m0 = line_base<0>(P, yy[0], zz[0]) + ix;
+        double u[U + 2];
+#pragma unroll
+        for (int k = 0; k < U + 2; k++) u[k] = un[m0 + (k - 1) * sy];
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+          zm[k] = __ldcg(un + m0 + k * sy - sz);
+          zp[k] = __ldcg(un + m0 + k * sy + sz);
+          tt[k] = P.tag[m0 + k * sy];
+        }
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+          um[k] = u[k];
+          uc[k] = u[k + 1];
+          up[k] = u[k + 2];
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+          const long long m = line_base<0>(P, yy[k], zz[k]) + ix;
+          um[k] = un[m - sy];
+          uc[k] = un[m];
+          up[k] = un[m + sy];
+          zm[k] = un[m - sz];
+          zp[k] = un[m + sz];
+          tt[k] = P.tag[m];
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < U; k++) {
+        if (!in || c0 + k >= nlive) continue;
+        if (tt[k] & (TAG_MIBX | TAG_MIBY | TAG_MIBZ)) {
+          sm[ix * RS + c0 + k] = io.out[line_base<0>(P, yy[k], zz[k]) + ix];  // a MIB row: from k_adi_mib
+          continue;
+        }
+        const RowExact q = row_exact(P, yy[k], zz[k]);
+        auto val = [&](auto S) {
+          constexpr int sd = decltype(S)::value;
+          double sum = 0.0;
+          sum += um[k] * P.vd[1][sd][0];
+          sum += uc[k] * P.vd[1][sd][1];
+          sum += up[k] * P.vd[1][sd][2];
+          const double ydt = dt * sum;
+          sum = 0.0;
+          sum += zm[k] * P.vd[2][sd][0];
+          sum += uc[k] * P.vd[2][sd][1];
+          sum += zp[k] * P.vd[2][sd][2];
+          const double zdt = dt * sum;
+          double src = 0.0;
+          if (P.eq != 0) {
+            if (sd)
+              src = -(((x2 + q.y2) + q.z2) * E1) - P.c6bo * E1;
+            else
+              src = P.kin * (((s2x * q.c2y) * q.s2z) * E1);
+          }
+          double v = ydt + zdt;
+          v += uc[k];
+          v += dt * src;
+          return v;
+        };
+        sm[ix * RS + c0 + k] = (tt[k] & TAG_OUT) ? val(IntC<1>{}) : val(IntC<0>{});
+      }
+    }
+  }
+}
+
+// A tile from its fields to its solution in shared memory.
+template <int D, int KIND, int NL, int NT, bool PLAIN>
+__device__ __forceinline__ void tile_solution(const Dev& P, const SweepIO& io, TileState<NL>& T, double* sm_, int t0,
+                                              int nlive) {
+  constexpr int RS = tile_row<D, NL>();
+  constexpr int NW = NT / 32;
+  constexpr int BW = NW / 2;  // the warps from this one on take the blocks first
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int n = D == 0 ? P.nx : D == 1 ? P.ny : P.nz;
+  const int n1 = D == 0 ? P.ny : P.nx, n2 = D == 2 ? P.ny : P.nz;
+  double* const sm = sm_ + factor_bytes<D, NL>(n) / 8;  // [n][RS]
+  const int ws = (blockIdx.x / P.sweep_blocks) % NW;  // the solving warp: another sub-core CTA by CTA
+  // ---- which factors the solve needs (the first warp): one side's, copied
+  // into shared memory here, or the lines' own
+  if (w == 0) {
+    const int i1 = T.i1[lane % NL], i2 = T.i2[lane % NL];
+    const int c = P.cline[D] ? P.cline[D][i1 + n1 * i2] : -1;
+    const int side = (P.lside[D][i1 * n2 + i2] >> 1) & 1;
+    const int side0 = __shfl_sync(0xffffffffu, side, 0);
+    const bool same = __all_sync(0xffffffffu, c < 0 && side == side0);
+    if (lane == 0) T.side = same ? side : -1;
+    if (same) {
+      for (int j = lane; j < n; j += 32) {
+        cp_async16(sm_ + 2 * j, P.tab[D][side] + j);
+        cp_async8(sm_ + 2 * n + j, P.tabg[D][side] + j);
+      }
+    }
+  }
+  // ---- load
+  if (w >= BW) tile_blocks<D, KIND, NL, NT>(P, io, T, sm, t0, nlive);
+  tile_rows<D, KIND, NL, NT>(P, io, T, sm, nlive);
+  if (w == 0) {
+    cp_async_commit();
+    cp_async_wait<0>();
+  }
+  __syncthreads();
+  const int side = T.side;
+  if (KIND == K_ADI && side < 0) {
+    // the x blocks' row operations on their right-hand sides
+    const int c = tid % NL;
+    if (c < nlive) {
+      const int lid = T.i1[c] * n2 + T.i2[c];
+      const int bend = P.bstart[0][lid + 1];
+      for (int k = P.bstart[0][lid] + tid / NL; k < bend; k += NT / NL) block_ops<RS>(P, k, sm + c);
+    }
+    __syncthreads();
+  }
+  // ---- solve: one warp
+  if (side >= 0) {
+    if (w == ws && lane < nlive) {
+      if (solve_side<RS, PLAIN>(reinterpret_cast<const double2*>(sm_), sm_ + 2 * n, side ? P.ia[D][1] : P.ia[D][0],
+                                sm + lane, n))
+        T.again = 1;
+    }
+  } else {
+    // (lanes past the tile's lines run the last line's factors on columns
+    // that are not stored)
+    const int cl = min(lane, nlive - 1);
+    const int i1 = T.i1[cl], i2 = T.i2[cl];
+    const int c = P.cline[D] ? P.cline[D][i1 + n1 * i2] : -1;
+    const int ls = (P.lside[D][i1 * n2 + i2] >> 1) & 1;
+    if (solve_own<NL, RS, NW, own_rows<D>(), PLAIN>(c >= 0 ? P.ca[D] + c : P.taba[D][ls], c >= 0 ? P.cb[D] + c : P.tab[D][ls],
+                                     c >= 0 ? P.cg[D] + c : P.tabg[D][ls], c >= 0 ? P.nfcross[D] : 1, sm_,
+                                     sm + min(lane, NL - 1), n, ws) &&
+        lane < nlive)
+      T.again = 1;
+  }
+  __syncthreads();
+}
+
+// The same with the divide, out of line (rare).
+template <int D, int KIND, int NL, int NT>
+__device__ __noinline__ void tile_solution_plain(const Dev& P, const SweepIO& io, TileState<NL>& T, double* sm_, int t0,
+                                                 int nlive) {
+  tile_solution<D, KIND, NL, NT, true>(P, io, T, sm_, t0, nlive);
+}
+
+template <int D, int KIND, int NL, int NT>
+__device__ __forceinline__ void k_line_body(const Dev& P, unsigned cta_, unsigned ncta_, const SweepIO& io) {
+  static_assert(NT % 32 == 0 && NT >= 96 && NL <= 32 && 32 % NL == 0, "shape");
+  static_assert(D == 0 || KIND != K_ADI, "the first right-hand side belongs to the x solve");
+  constexpr int RS = tile_row<D, NL>();
+  constexpr int NW = NT / 32;
+  const int tid = threadIdx.x;
+  const int n = D == 0 ? P.nx : D == 1 ? P.ny : P.nz;
+  const int nint = (int)interior_lines<D>(P);
+  const int ntile = (nint + NL - 1) / NL;
+  if ((int)cta_ >= ntile) {
+    face_lines<D>(P, cta_ - ntile, ncta_ - ntile, io, step_e(P, io.e1, 2));
+    return;
+  }
+  extern __shared__ __align__(16) double sm_[];
+  __shared__ TileState<NL> T;
+  const int t0 = (int)cta_ * NL;
+  const int nlive = min(NL, nint - t0);
+  if (tid < NL) {
+    const int n1 = D == 0 ? P.ny : P.nx;
+    const int v = P.lperm[D][min(t0 + tid, nint - 1)];
+    const int q = v / n1;
+    T.i1[tid] = v - q * n1;
+    T.i2[tid] = q;
+  }
+  if (tid == 0) {
+    T.next_task = 0;
+    T.again = P.plain_div;
+  }
+  __syncthreads();
+  if (!P.plain_div) tile_solution<D, KIND, NL, NT, false>(P, io, T, sm_, t0, nlive);
+  if (T.again) {
+    __syncthreads();
+    if (tid == 0) T.next_task = 0;
+    __syncthreads();
+    tile_solution_plain<D, KIND, NL, NT>(P, io, T, sm_, t0, nlive);
+  }
+
+  // ---- store
+  const double* const sm = sm_ + factor_bytes<D, NL>(n) / 8;
+  if (D != 0) {
+    constexpr int SUB = NT / NL;
+    const long long s = D == 1 ? (long long)P.nx : (long long)P.nx * P.ny;
+    const int c = tid % NL;
+    if (c < nlive) {
+      const int i1 = T.i1[c], i2 = T.i2[c];
+      const long long base = line_base<D>(P, i1, i2);
+      double* const o = io.out + base;
+      if (io.last) {
+        const uint8_t* const tg = P.tag + base;
+        const double E1 = step_e(P, io.e1, 2);
+#pragma unroll 4
+        for (int j = tid / NL; j < n; j += SUB)
+          o[j * s] = sm[j * RS + c] +
+                     P.dt * source(P, E1, tg[j * s] & TAG_OUT, i1, D == 1 ? j : i2, D == 1 ? i2 : j);
+      } else {
+#pragma unroll 8
+        for (int j = tid / NL; j < n; j += SUB) o[j * s] = sm[j * RS + c];
+      }
+    }
+  } else {
+    for (int c = tid >> 5; c < nlive; c += NW) {
+      double* const o = io.out + line_base<0>(P, T.i1[c], T.i2[c]);
+#pragma unroll 8
+      for (int ix = tid & 31; ix < n; ix += 32) o[ix] = sm[ix * RS + c];
+    }
+  }
+}
+
+// CTAs of a direction's line solves: its tiles, and for the face lines one
+// per 4096 nodes.
+template <int D>
+unsigned line_grid(const Dev& P, int nl, bool faces) {
+  const long long tiles = (interior_lines<D>(P) + nl - 1) / nl;
+  const long long n1 = D == 0 ? P.ny : P.nx, n2 = D == 2 ? P.ny : P.nz, n = D == 0 ? P.nx : D == 1 ? P.ny : P.nz;
+  const long long fn = (2 * n1 + 2 * (n2 - 2)) * n;
+  return (unsigned)(tiles + (faces ? (fn + 4095) / 4096 : 0));
+}
+
+// CTAs per SM that the registers should allow: four of 256 threads (a 129^3
+// grid's 504 tiles are then all on the chip at once: LOD-CN step 82 against 96
+// us), three for the first right-hand side, which holds more (x sweep of 257^3
+// 229 against 301 us).
+template <int KIND, int NT>
+constexpr int line_min_ctas() { return NT == 256 ? (KIND == K_ADI ? 3 : 4) : NT == 192 ? 4 : NT == 128 ? 5 : 6; }
+
+template <int D, int KIND, int NL, int NT>
+__global__ void __launch_bounds__(NT, line_min_ctas<KIND, NT>()) k_line(const __grid_constant__ Dev P,
+                                                                       const __grid_constant__ SweepIO io) {
+  k_line_body<D, KIND, NL, NT>(P, blockIdx.x, gridDim.x, io);
 }
 
 // Thomas factors of the lines that cross the interface (the factor half of
 // TDMA, douglas_adi.cc:1790-1798: gam_j = c_{j-1}/bet, bet = b_j - a_j*gam_j,
-// the same IEEE operations as the host's prefix tables), once at setup, one
-// thread per line.  A line's rows are the identity on its faces, the regular
-// three-point rows of the node's side elsewhere, and the Convert2Tri rows of
-// its blocks; from the first MIB row on, bet and gam are stored per node in
-// FP64 (fbet, fgam) and as 1/bet and gam in FP32 (fib32, fgam32).  A zero
-// pivot sets *zero_pivot.
+// the same IEEE operations as the host's side tables), once at setup, one
+// thread per listed line.  A line's rows are the identity on its faces, the
+// regular three-point rows of the node's side elsewhere, and the Convert2Tri
+// rows of its blocks; a_j, (bet_j, 1/bet_j) and gam_{j+1} are stored by row,
+// the lines of a row side by side, and for the FP32 ring sweeps (where fib32 is there)
+// 1/bet and gam per node from the first MIB row on.  A zero pivot sets bit 0
+// of *flags, a factor out of the range of the quotients from reciprocals bit
+// 1.
 template <int D>
-__global__ void __launch_bounds__(TPB) k_factor_lines(const __grid_constant__ Dev P, int* zero_pivot) {
-  const long long t = (long long)blockIdx.x * TPB + threadIdx.x;
-  if (t >= nlines<D>(P)) return;
+__global__ void __launch_bounds__(TPB) k_factor_lines(const __grid_constant__ Dev P, int* flags) {
+  const int l = blockIdx.x * TPB + threadIdx.x;
+  const int nc = P.nfcross[D];
+  if (l >= nc) return;
+  const int lid = P.fcross[D][l];
+  const int n2 = D == 2 ? P.ny : P.nz;
   Line L;
-  decode_line<D>(P, t, L);
-  if (L.boundary) return;
-  const int bfirst = P.bstart[D][L.lid], bend = P.bstart[D][L.lid + 1];
-  if (bfirst == bend) return;
+  decode_line<D>(P, (long long)(lid % n2) * (D == 0 ? P.ny : P.nx) + lid / n2, L);
+  const int bfirst = P.bstart[D][lid], bend = P.bstart[D][lid + 1];
   const MibBlock* const blk = P.blk[D];
   const int n = L.n;
   const int L1 = blk[bfirst].L;
+  // (the factors are read-only to the step kernels; setup fills them here)
+  double* const fa = const_cast<double*>(P.ca[D]) + l;
+  double2* const fb = const_cast<double2*>(P.cb[D]) + l;
+  double* const g = const_cast<double*>(P.cg[D]) + l;
+  fa[0] = 0.0;
+  fb[0] = make_double2(1.0, 1.0);
   int b = bfirst;
   double bet = 1.0;   // row 0: b = 1
   double cprev = 0.0; // c of the previous row
@@ -888,35 +1046,47 @@ __global__ void __launch_bounds__(TPB) k_factor_lines(const __grid_constant__ De
     const double gm = cprev / bet;
     bet = bj - aj * gm;
     if (bet == 0.0) {
-      atomicOr(zero_pivot, 1);
+      atomicOr(flags, 1);
       return;
     }
-    if (j >= L1) {
-      // (the factor fields are read-only to the step kernels; setup fills them here)
+    fa[(long long)j * nc] = aj;
+    fb[(long long)j * nc] = make_double2(bet, 1.0 / bet);
+    if (!(fabs(bet) >= 0x1p-100 && fabs(bet) <= 0x1p100)) atomicOr(flags, 2);
+    g[(long long)(j - 1) * nc] = gm;
+    if (j >= L1 && P.fib32[D]) {
       const long long m = L.base + (long long)j * L.s;
-      const_cast<double*>(P.fbet[D])[m] = bet;
-      const_cast<double*>(P.fgam[D])[m] = gm;
       const_cast<float*>(P.fib32[D])[m] = (float)(1.0 / bet);
       const_cast<float*>(P.fgam32[D])[m] = (float)gm;
     }
     cprev = cj;
   }
+  g[(long long)(n - 1) * nc] = 0.0;
 }
 
-// Refresh_Jump (intersection.cc:2294-2490): [u] and u_dir per crossing.
-__device__ __forceinline__ void k_jumps_body(const Dev& P, unsigned cta_, unsigned ncta_, double E) {
-  int c = cta_ * TPB + threadIdx.x;
-  if (c >= P.ncross) return;
-  E = step_e(P, E, 2);
-  const CrossConst q = P.cc[c];
-  double ju, jb[3];
-  exact_jumps(P, q, E, ju, jb);
-  double bxi = q.p[0] * jb[0] + q.p[1] * jb[1] + q.p[2] * jb[2];
-  P.jv[c] = make_double2(ju, q.pinv * bxi);
-}
-
-__global__ void __launch_bounds__(TPB) k_jumps(const __grid_constant__ Dev P, double E) {
-  k_jumps_body(P, blockIdx.x, gridDim.x, E);
+// Per MIB node its block in x, y, z, once at setup: 16 block + 4 kind + row,
+// -1: none.
+__global__ void __launch_bounds__(TPB) k_mibref(const __grid_constant__ Dev P) {
+  const int k = blockIdx.x * TPB + threadIdx.x;
+  if (k >= P.nmibnode) return;
+  const long long m = P.mibnode[k];
+  const int tg = P.tag[m];
+  int ix, iy, iz;
+  node_xyz(P, m, ix, iy, iz);
+  int4 r = make_int4(-1, -1, -1, 0);
+  int row = 0;
+  if (tg & TAG_MIBX) {
+    const MibBlock* b = find_block<0>(P, iy * P.nz + iz, ix, row);
+    if (b) r.x = (int)(b - P.blk[0]) * 16 + b->kind * 4 + row;
+  }
+  if (tg & TAG_MIBY) {
+    const MibBlock* b = find_block<1>(P, ix * P.nz + iz, iy, row);
+    if (b) r.y = (int)(b - P.blk[1]) * 16 + b->kind * 4 + row;
+  }
+  if (tg & TAG_MIBZ) {
+    const MibBlock* b = find_block<2>(P, ix * P.ny + iy, iz, row);
+    if (b) r.z = (int)(b - P.blk[2]) * 16 + b->kind * 4 + row;
+  }
+  const_cast<int4*>(P.mibref)[k] = r;
 }
 
 __global__ void __launch_bounds__(TPB) k_init(const Dev P, double E, double* u) {
@@ -1000,39 +1170,34 @@ unsigned pointwise_blocks(const Dev& P) {
   return (unsigned)(b < cap ? b : cap);
 }
 
-// Sweep shapes (rows per chunk, ring chunks, threads per CTA), selected per
-// sweep of a step by Dev::shape (mts_set_sweep_shape / mts_autotune).
-#define MTS_SHAPES(X)                                                                        \
-  X(0, 8, 8, 128) X(1, 4, 16, 128) X(2, 4, 8, 256) X(3, 8, 4, 256) X(4, 4, 8, 192) X(5, 4, 8, 288) \
-  X(6, 4, 4, 384) X(7, 4, 4, 512) X(8, 4, 4, 448) X(9, 4, 4, 128)
+// Whether the sweep of direction d of a step writes the face lines: the
+// Douglas-ADI y solve and the TS y and x solves keep them.
+bool sweep_faces(int method, int d) { return method == 0 ? d != 1 : method == 3 ? d == 2 : true; }
 
-template <int D, int KIND, int CH, int NS, int NT>
+template <int D, int KIND, int NL, int NT>
 void sweep_shape(const Dev& P, const SweepIO& io, cudaStream_t st) {
-  // persistent CTAs, one per SM at most, no more than the lines need
   const int nd = D == 0 ? P.nx : D == 1 ? P.ny : P.nz;
-  k_sweep<D, KIND, CH, NS, NT><<<sweep_grid(P, nlines<D>(P), NT), NT, shape_smem<CH, NS, NT, D>(nd), st>>>(P, io);
+  k_line<D, KIND, NL, NT>
+      <<<line_grid<D>(P, NL, sweep_faces(P.method, D)), NT, tile_smem<D, NL>(nd), st>>>(P, io);
 }
 
+// One sweep in the shape selected for it (Dev::shape).
 template <int D, int KIND>
 void sweep(const Dev& P, const SweepIO& io, int shape, cudaStream_t st) {
-  if (P.nblk[D] > 0) k_block_rhs<D, KIND><<<(P.nblk[D] + TPB - 1) / TPB, TPB, 0, st>>>(P, io, P.nblk[D]);
   switch (shape) {
-#define MTS_CASE(id, ch, ns, nt) \
-  case id:                       \
-    sweep_shape<D, KIND, ch, ns, nt>(P, io, st); \
+#define MTS_CASE(id, nl, nt)                    \
+  case id:                                      \
+    sweep_shape<D, KIND, nl, nt>(P, io, st);    \
     break;
     MTS_SHAPES(MTS_CASE)
 #undef MTS_CASE
-    default:
-      sweep_shape<D, KIND, 16, 4, 128>(P, io, st);
   }
 }
 
 template <int D, int KIND>
 void set_smem_attr() {
-#define MTS_ATTR(id, ch, ns, nt)                                                             \
-  cudaFuncSetAttribute(k_sweep<D, KIND, ch, ns, nt>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                       kMaxSweepSmem);
+#define MTS_ATTR(id, nl, nt) \
+  cudaFuncSetAttribute(k_line<D, KIND, nl, nt>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem);
   MTS_SHAPES(MTS_ATTR)
 #undef MTS_ATTR
 }
@@ -1043,22 +1208,30 @@ int sweep_shape_count() { return 10; }
 
 bool sweep_shape_fits(int shape, int nmax) {
   switch (shape) {
-#define MTS_FITS(id, ch, ns, nt) \
-  case id:                       \
-    return shape_smem<ch, ns, nt>(nmax) <= (size_t)kMaxSweepSmem;
+#define MTS_FITS(id, nl, nt) \
+  case id:                   \
+    return nmax <= kMaxLineRows && tile_smem<0, nl>(nmax) <= (size_t)kMaxTileSmem;
     MTS_SHAPES(MTS_FITS)
 #undef MTS_FITS
     default:
       return false;
   }
 }
-int sweep_shape_max_threads() { return 512; }
+
+// 32 lines per tile while shared memory holds them, else the most it holds.
+int sweep_shape_default(int nmax) {
+  const int order[4] = {0, 3, 6, 8};
+  for (int s : order)
+    if (sweep_shape_fits(s, nmax)) return s;
+  return -1;
+}
 
 void configure_kernels() {
   set_smem_attr<0, K_COPY>();
   set_smem_attr<1, K_COPY>();
   set_smem_attr<2, K_COPY>();
   set_smem_attr<0, K_STENCIL>();
+  set_smem_attr<0, K_ADI>();
   set_smem_attr<1, K_STENCIL>();
   set_smem_attr<2, K_STENCIL>();
   set_smem_attr<2, K_TS_Z>();
@@ -1068,24 +1241,24 @@ __global__ void k_tick(int* step) { ++*step; }
 
 void launch_tick(const Dev& P, cudaStream_t st) { k_tick<<<1, 1, 0, st>>>(P.tstep); }
 
-void launch_jumps(const Dev& P, double E, cudaStream_t st) {
-  k_jumps<<<(P.ncross + TPB - 1) / TPB, TPB, 0, st>>>(P, E);
-}
-
 unsigned pointwise_rows_grid(const Dev& P) { return pointwise_blocks(P); }
 
-int launch_factor_lines(const Dev& P, int* zero_pivot, cudaStream_t st) {
+int launch_factor_lines(const Dev& P, int* flags, cudaStream_t st) {
   int launches = 0;
-  if (P.nblk[0] > 0) {
-    k_factor_lines<0><<<(unsigned)((nlines<0>(P) + TPB - 1) / TPB), TPB, 0, st>>>(P, zero_pivot);
+  if (P.mibref && P.nmibnode > 0) {
+    k_mibref<<<(P.nmibnode + TPB - 1) / TPB, TPB, 0, st>>>(P);
     launches++;
   }
-  if (P.nblk[1] > 0) {
-    k_factor_lines<1><<<(unsigned)((nlines<1>(P) + TPB - 1) / TPB), TPB, 0, st>>>(P, zero_pivot);
+  if (P.nfcross[0] > 0) {
+    k_factor_lines<0><<<(P.nfcross[0] + TPB - 1) / TPB, TPB, 0, st>>>(P, flags);
     launches++;
   }
-  if (P.nblk[2] > 0) {
-    k_factor_lines<2><<<(unsigned)((nlines<2>(P) + TPB - 1) / TPB), TPB, 0, st>>>(P, zero_pivot);
+  if (P.nfcross[1] > 0) {
+    k_factor_lines<1><<<(P.nfcross[1] + TPB - 1) / TPB, TPB, 0, st>>>(P, flags);
+    launches++;
+  }
+  if (P.nfcross[2] > 0) {
+    k_factor_lines<2><<<(P.nfcross[2] + TPB - 1) / TPB, TPB, 0, st>>>(P, flags);
     launches++;
   }
   return launches;
@@ -1109,61 +1282,43 @@ int launch_norms(const Dev& P, double E, const double* u, double* partial, int n
   return 2;
 }
 
-// One time step.  u0 holds u^n on entry and u^{n+1} on return (the two
-// pointers are swapped when the result lands in the other buffer).
-int launch_step(const Dev& P, const StepTimes& T, double*& u0, double*& u1, cudaStream_t st, cudaEvent_t* ev,
-                const SideStream* side) {
+// One time step.  u0 holds u^n on entry and u^{n+1} on return; u1 is scratch.
+int launch_step(const Dev& P, const StepTimes& T, double* u0, double* u1, cudaStream_t st, cudaEvent_t* ev) {
   int launches = 0;
   int slot = 0;
   auto mark = [&](int k) {
     if (ev) cudaEventRecord(ev[2 * slot + k], st);
     if (k == 1) slot++;
   };
-  // Douglas-ADI: the jumps and the MIB rows of the first right-hand side
-  // (which read the jumps) run on the side stream beside its pointwise pass;
-  // the two passes write disjoint nodes and read only u^n.
-  const bool fork = side && side->stream && P.method == 0 && (P.ncross > 0 || P.nmibnode > 0);
-  cudaStream_t sst = fork ? side->stream : st;
-  if (fork) {
-    cudaEventRecord(side->fork, st);
-    cudaStreamWaitEvent(sst, side->fork, 0);
-  }
-  if (ev) cudaEventRecord(ev[0], sst);
-  if (P.ncross > 0) {
-    k_jumps<<<(P.ncross + TPB - 1) / TPB, TPB, 0, sst>>>(P, T.e_next);
-    launches++;
-  }
-  if (ev) cudaEventRecord(ev[1], sst);
-  slot = 1;
+  // (slot 0, once the jump pass: the kernels evaluate the jumps they use)
+  mark(0);
+  mark(1);
   SweepIO io{};
   io.e1 = T.e_next;
   io.e0 = T.e_prev;
   if (P.method == 0) {
-    // Douglas-ADI.  u1 <- uhs (pointwise); x sweep in place gives u*; y sweep
-    // builds uhss = -dt D_yy u^n + u* and solves in place (u**); z sweep builds
-    // uh1 = -dt D_zz u^n + u** and writes u^{n+1} over u^n in u0 (a z line
-    // reads only its own nodes of u^n; its faces get Outer_u(t_next), the
-    // value u** holds there).  The state stays in u0, u1 is scratch.
+    // Douglas-ADI.  The x sweep forms uhs of its lines from u0 and solves it
+    // into u1 (u*); the y sweep builds uhss = -dt D_yy u^n + u* and solves in
+    // place (u**); the z sweep builds uh1 = -dt D_zz u^n + u** and writes
+    // u^{n+1} over u^n in u0 (a z line reads only its own nodes of u^n).  The
+    // faces get Outer_u(t_next) in u1 and in u0.  The state stays in u0, u1
+    // is scratch.
     mark(0);
     if (P.nmibnode > 0) {
-      k_adi_rhs_mib<<<(P.nmibnode + TPB - 1) / TPB, TPB, 0, sst>>>(P, u0, u1, T.e_next);
+      k_adi_mib<<<mib_nodes_grid(P), TPB, 0, st>>>(P, u0, u1, T.e_next);
       launches++;
     }
-    k_adi_rhs<2><<<pointwise_blocks(P), TPB, 0, st>>>(P, u0, u1, T.e_next);
-    if (fork) {
-      cudaEventRecord(side->join, sst);
-      cudaStreamWaitEvent(st, side->join, 0);
-    }
-    mark(1);
-    io.stin = u1;
-    io.add = u1;
-    io.out = u1;
-    io.jumps = 0;
-    io.bmode = 0;
-    mark(0);
-    sweep<0, K_COPY>(P, io, P.shape[0], st);
     mark(1);
     io.stin = u0;
+    io.add = u0;
+    io.out = u1;
+    io.jumps = 0;
+    io.bmode = 1;
+    mark(0);
+    sweep<0, K_ADI>(P, io, P.shape[0], st);
+    mark(1);
+    io.add = u1;
+    io.bmode = 0;
     io.k = -P.dt;
     mark(0);
     sweep<1, K_STENCIL>(P, io, P.shape[1], st);
@@ -1173,7 +1328,7 @@ int launch_step(const Dev& P, const StepTimes& T, double*& u0, double*& u1, cuda
     mark(0);
     sweep<2, K_STENCIL>(P, io, P.shape[2], st);
     mark(1);
-    launches += 4;
+    launches += 3;
   } else if (P.method == 1 || P.method == 2) {
     // LOD, in place on u0.
     io.jumps = 1;
@@ -1206,19 +1361,12 @@ int launch_step(const Dev& P, const StepTimes& T, double*& u0, double*& u1, cuda
   } else {
     // TS: explicit x (u0 -> u1) and y (u1 -> u0) half steps, fused explicit
     // z + sources + implicit z in place on u0, then implicit y and x in place.
+    const unsigned rows = pointwise_blocks(P) + mib_ctas(P);
     mark(0);
-    k_ts_explicit<0><<<pointwise_blocks(P), TPB, 0, st>>>(P, u0, u1, T.e_half);
-    if (P.nmibnode > 0) {
-      k_ts_explicit_mib<0><<<(P.nmibnode + TPB - 1) / TPB, TPB, 0, st>>>(P, u0, u1);
-      launches++;
-    }
+    k_ts_explicit<0><<<rows, TPB, 0, st>>>(P, u0, u1, T.e_half, T.e_next);
     mark(1);
     mark(0);
-    k_ts_explicit<1><<<pointwise_blocks(P), TPB, 0, st>>>(P, u1, u0, T.e_half);
-    if (P.nmibnode > 0) {
-      k_ts_explicit_mib<1><<<(P.nmibnode + TPB - 1) / TPB, TPB, 0, st>>>(P, u1, u0);
-      launches++;
-    }
+    k_ts_explicit<1><<<rows, TPB, 0, st>>>(P, u1, u0, T.e_half, T.e_next);
     mark(1);
     io.jumps = 1;
     io.k = P.kex;
@@ -1238,9 +1386,6 @@ int launch_step(const Dev& P, const StepTimes& T, double*& u0, double*& u1, cuda
     mark(1);
     launches += 5;
   }
-  // every method sweeps each direction once; each sweep with MIB blocks is
-  // preceded by its block pre-pass
-  for (int d = 0; d < 3; d++) launches += P.nblk[d] > 0;
   return launches;
 }
 
@@ -1365,51 +1510,30 @@ __device__ __forceinline__ SweepIO make_io(const Dev& P, const Roles& r) {
   return io;
 }
 
-__global__ void __launch_bounds__(TPB) kb_jumps(const Dev* __restrict__ Ps, const BatchItem* __restrict__ items) {
+__global__ void __launch_bounds__(TPB) kb_adi_mib(const Dev* __restrict__ Ps, const BatchItem* __restrict__ items) {
   BATCH_PROLOGUE
-  k_jumps_body(P, w.cta, w.ncta, 0.0);
-}
-
-__global__ void __launch_bounds__(TPB) kb_adi_rhs(const Dev* __restrict__ Ps, const BatchItem* __restrict__ items) {
-  BATCH_PROLOGUE
-  k_adi_rhs_body<2>(P, w.cta, w.ncta, P.u0, P.u1, 0.0);
-}
-
-__global__ void __launch_bounds__(TPB) kb_adi_rhs_mib(const Dev* __restrict__ Ps,
-                                                      const BatchItem* __restrict__ items) {
-  BATCH_PROLOGUE
-  k_adi_rhs_mib_body(P, w.cta, w.ncta, P.u0, P.u1, 0.0);
+  k_adi_mib_body(P, w.cta, w.ncta, P.u0, P.u1, 0.0);
 }
 
 template <int D>
 __global__ void __launch_bounds__(TPB) kb_ts_explicit(const Dev* __restrict__ Ps,
                                                       const BatchItem* __restrict__ items, int in) {
   BATCH_PROLOGUE
-  k_ts_explicit_body<D>(P, w.cta, w.ncta, in ? P.u1 : P.u0, in ? P.u0 : P.u1, 0.0);
+  k_ts_explicit_body<D>(P, w.cta, w.ncta, in ? P.u1 : P.u0, in ? P.u0 : P.u1, 0.0, 0.0);
 }
 
-template <int D>
-__global__ void __launch_bounds__(TPB) kb_ts_explicit_mib(const Dev* __restrict__ Ps,
-                                                          const BatchItem* __restrict__ items, int in) {
-  BATCH_PROLOGUE
-  k_ts_explicit_mib_body<D>(P, w.cta, w.ncta, in ? P.u1 : P.u0, in ? P.u0 : P.u1);
-}
+// tiles of batches of small problems: many CTAs per SM
+constexpr int BNL = 32, BNT = 128;
 
 template <int D, int KIND>
-__global__ void __launch_bounds__(TPB) kb_block_rhs(const Dev* __restrict__ Ps, const BatchItem* __restrict__ items,
-                                                    Roles r) {
+__global__ void __launch_bounds__(BNT, line_min_ctas<KIND, BNT>()) kb_line(const Dev* __restrict__ Ps,
+                                                                           const BatchItem* __restrict__ items,
+                                                                           Roles r) {
   BATCH_PROLOGUE
-  k_block_rhs_body<D, KIND>(P, w.cta, w.ncta, make_io(P, r), P.nblk[D]);
-}
-
-// the small-CTA shape (several CTAs per SM) for batches of small problems
-constexpr int BCH = 4, BNS = 4, BNT = 128;
-
-template <int D, int KIND>
-__global__ void __launch_bounds__(BNT) kb_sweep(const Dev* __restrict__ Ps, const BatchItem* __restrict__ items,
-                                                Roles r) {
-  BATCH_PROLOGUE
-  k_sweep_body<D, KIND, BCH, BNS, BNT>(P, w.cta, w.ncta, make_io(P, r));
+  __shared__ SweepIO io;
+  if (threadIdx.x == 0) io = make_io(P, r);
+  __syncthreads();
+  k_line_body<D, KIND, BNL, BNT>(P, w.cta, w.ncta, io);
 }
 
 __global__ void kb_tick(const Dev* __restrict__ Ps, int n) {
@@ -1419,30 +1543,21 @@ __global__ void kb_tick(const Dev* __restrict__ Ps, int n) {
 
 template <int D, int KIND>
 void bsweep(const BatchPlan& b, const Roles& r, cudaStream_t st, int& launches) {
-  if (b.nblk[D] > 0) {
-    kb_block_rhs<D, KIND><<<b.nblk[D], TPB, 0, st>>>(b.Ps, b.blk[D], r);
-    launches++;
-  }
   if (b.nsw[D] > 0) {
-    kb_sweep<D, KIND><<<b.nsw[D], BNT, shape_smem<BCH, BNS, BNT, D>(b.nmax), st>>>(b.Ps, b.sw[D], r);
+    kb_line<D, KIND><<<b.nsw[D], BNT, tile_smem<D, BNL>(b.nmax), st>>>(b.Ps, b.sw[D], r);
     launches++;
   }
 }
 
 template <int D, int KIND>
 void bsweep_attr() {
-  cudaFuncSetAttribute(kb_sweep<D, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       kMaxSweepSmem - (int)sizeof(Dev) - 64);
+  cudaFuncSetAttribute(kb_line<D, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBatchTileSmem);
 }
 
 }  // namespace
 
-int batch_sweep_threads() { return BNT; }
-
-int launch_batch_jumps(const Dev* Ps, const BatchItem* items, int nitems, cudaStream_t st) {
-  if (nitems <= 0) return 0;
-  kb_jumps<<<nitems, TPB, 0, st>>>(Ps, items);
-  return 1;
+bool batch_lines_fit(int nmax) {
+  return tile_smem<0, BNL>(nmax) <= (size_t)kBatchTileSmem && tile_smem<1, BNL>(nmax) <= (size_t)kBatchTileSmem;
 }
 
 int launch_batch_tick(const Dev* Ps, int n, cudaStream_t st) {
@@ -1450,11 +1565,12 @@ int launch_batch_tick(const Dev* Ps, int n, cudaStream_t st) {
   return 1;
 }
 
-unsigned jumps_grid(const Dev& P) { return (unsigned)((P.ncross + TPB - 1) / TPB); }
-unsigned mib_grid(const Dev& P) { return (unsigned)((P.nmibnode + TPB - 1) / TPB); }
+unsigned mib_grid(const Dev& P) { return mib_nodes_grid(P); }
 unsigned block_grid(const Dev& P, int d) { return (unsigned)((P.nblk[d] + TPB - 1) / TPB); }
+unsigned ts_explicit_grid(const Dev& P) { return pointwise_blocks(P) + mib_ctas(P); }
 unsigned batch_sweep_grid(const Dev& P, int d) {
-  return sweep_grid(P, d == 0 ? nlines<0>(P) : d == 1 ? nlines<1>(P) : nlines<2>(P), BNT);
+  const bool faces = sweep_faces(P.method, d);
+  return d == 0 ? line_grid<0>(P, BNL, faces) : d == 1 ? line_grid<1>(P, BNL, faces) : line_grid<2>(P, BNL, faces);
 }
 
 void configure_batch_kernels() {
@@ -1462,6 +1578,7 @@ void configure_batch_kernels() {
   bsweep_attr<1, K_COPY>();
   bsweep_attr<2, K_COPY>();
   bsweep_attr<0, K_STENCIL>();
+  bsweep_attr<0, K_ADI>();
   bsweep_attr<1, K_STENCIL>();
   bsweep_attr<2, K_STENCIL>();
   bsweep_attr<2, K_TS_Z>();
@@ -1470,18 +1587,12 @@ void configure_batch_kernels() {
 // One step of every problem of the plan, the launch sequence of launch_step.
 int launch_step_batch(const BatchPlan& b, cudaStream_t st) {
   int launches = 0;
-  if (b.njumps > 0) {
-    kb_jumps<<<b.njumps, TPB, 0, st>>>(b.Ps, b.jumps);
-    launches++;
-  }
   if (b.method == 0) {
-    kb_adi_rhs<<<b.nrows, TPB, 0, st>>>(b.Ps, b.rows);
-    launches++;
     if (b.nmib > 0) {
-      kb_adi_rhs_mib<<<b.nmib, TPB, 0, st>>>(b.Ps, b.mib);
+      kb_adi_mib<<<b.nmib, TPB, 0, st>>>(b.Ps, b.mib);
       launches++;
     }
-    bsweep<0, K_COPY>(b, Roles{1, 1, 1, 0, 0, 0, 0}, st, launches);
+    bsweep<0, K_ADI>(b, Roles{0, 0, 1, 0, 0, 1, 0}, st, launches);
     bsweep<1, K_STENCIL>(b, Roles{0, 1, 1, 1, 0, 0, 0}, st, launches);
     bsweep<2, K_STENCIL>(b, Roles{0, 1, 0, 1, 0, 1, 0}, st, launches);
   } else if (b.method == 1 || b.method == 2) {
@@ -1496,17 +1607,8 @@ int launch_step_batch(const BatchPlan& b, cudaStream_t st) {
     }
   } else {
     kb_ts_explicit<0><<<b.nrows, TPB, 0, st>>>(b.Ps, b.rows, 0);
-    launches++;
-    if (b.nmib > 0) {
-      kb_ts_explicit_mib<0><<<b.nmib, TPB, 0, st>>>(b.Ps, b.mib, 0);
-      launches++;
-    }
     kb_ts_explicit<1><<<b.nrows, TPB, 0, st>>>(b.Ps, b.rows, 1);
-    launches++;
-    if (b.nmib > 0) {
-      kb_ts_explicit_mib<1><<<b.nmib, TPB, 0, st>>>(b.Ps, b.mib, 1);
-      launches++;
-    }
+    launches += 2;
     bsweep<2, K_TS_Z>(b, Roles{0, 0, 0, 2, 1, 1, 0}, st, launches);
     bsweep<1, K_COPY>(b, Roles{0, 0, 0, 2, 1, 0, 0}, st, launches);
     bsweep<0, K_COPY>(b, Roles{0, 0, 0, 2, 1, 0, 0}, st, launches);

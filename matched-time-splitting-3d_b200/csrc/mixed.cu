@@ -104,56 +104,20 @@ __global__ void __launch_bounds__(TPB, 8) k_adi_resid(const __grid_constant__ De
   adi_resid_body<G>(P, blockIdx.x, gridDim.x, un, rho, E);
 }
 
-// The MIB rows of rho, one thread per listed node: the explicit MIB sums of
+// The MIB rows of rho, three lanes per listed node: the explicit MIB sums of
 // every direction the node is a MIB row of (douglas_adi.cc:112-210, without
 // jumps) and the jump terms of Src_2nd (douglas_adi.cc:1156-1427).
-__device__ __forceinline__ void adi_resid_mib_body(const Dev& P, unsigned cta_, const double* __restrict__ un,
-                                                   float* __restrict__ rho, double E) {
-  const int k = cta_ * TPB + threadIdx.x;
-  if (k >= P.nmibnode) return;
-  E = step_e(P, E, 2);
-  const long long m = P.mibnode[k];
-  int ix, iy, iz;
-  node_xyz(P, m, ix, iy, iz);
-  const int tg = P.tag[m];
-  const int side = tg & TAG_OUT;
-  const long long sy = P.nx, sz = (long long)P.nx * P.ny;
-  const double* vdx = P.vd[0][side];
-  const double* vdy = P.vd[1][side];
-  const double* vdz = P.vd[2][side];
-  int xr = 0, yr = 0, zr = 0;
-  const MibBlock* xb = (tg & TAG_MIBX) ? find_block<0>(P, iy * P.nz + iz, ix, xr) : nullptr;
-  const MibBlock* yb = (tg & TAG_MIBY) ? find_block<1>(P, ix * P.nz + iz, iy, yr) : nullptr;
-  const MibBlock* zb = (tg & TAG_MIBZ) ? find_block<2>(P, ix * P.ny + iy, iz, zr) : nullptr;
-  double sx, sy_, sz_;
-  if (xb) {
-    const long long base = m - ix;
-    sx = mib_sum(*xb, xr, [&](int j) { return un[base + j]; }, vdx, false, P.jv);
-  } else {
-    sx = (un[m - 1] * vdx[0] + un[m] * vdx[1]) + un[m + 1] * vdx[2];
-  }
-  if (yb) {
-    const long long base = ix + sz * iz;
-    sy_ = mib_sum(*yb, yr, [&](int j) { return un[base + (long long)j * sy]; }, vdy, false, P.jv);
-  } else {
-    sy_ = (un[m - sy] * vdy[0] + un[m] * vdy[1]) + un[m + sy] * vdy[2];
-  }
-  if (zb) {
-    const long long base = ix + (long long)P.nx * iy;
-    sz_ = mib_sum(*zb, zr, [&](int j) { return un[base + (long long)j * sz]; }, vdz, false, P.jv);
-  } else {
-    sz_ = (un[m - sz] * vdz[0] + un[m] * vdz[1]) + un[m + sz] * vdz[2];
-  }
-  double src = source(P, E, side, ix, iy, iz);
-  if (xb) src = adi_src_add(src, *xb, xr, vdx, P.jv);
-  if (yb) src = adi_src_add(src, *yb, yr, vdy, P.jv);
-  if (zb) src = adi_src_add(src, *zb, zr, vdz, P.jv);
-  rho[m] = (float)(P.dt * (((sx + sy_) + sz_) + src));
+__device__ __forceinline__ void adi_resid_mib_body(const Dev& P, unsigned cta_, unsigned ncta_,
+                                                   const double* __restrict__ un, float* __restrict__ rho, double E) {
+  mib_nodes(P, un, step_e(P, E, 2), 0, P.nmibnode, cta_ * (TPB / 32) + (threadIdx.x >> 5), ncta_ * (TPB / 32),
+            [&](long long m, int, int, int, double sx, double sy, double sz, double src) {
+              rho[m] = (float)(P.dt * (((sx + sy) + sz) + src));
+            });
 }
 
 __global__ void __launch_bounds__(TPB) k_adi_resid_mib(const __grid_constant__ Dev P, const double* __restrict__ un,
                                                        float* __restrict__ rho, double E) {
-  adi_resid_mib_body(P, blockIdx.x, un, rho, E);
+  adi_resid_mib_body(P, blockIdx.x, gridDim.x, un, rho, E);
 }
 
 // ---------------------------------------------------------------------------
@@ -505,47 +469,23 @@ __global__ void __launch_bounds__(NT, 1) k_sweep32(const __grid_constant__ Dev P
 // increment.  The block pre-pass writes the block rows' right-hand sides into
 // the field in place first, so every row reads its right-hand side there.
 
-// Coefficients of one direction, one thread per line that crosses the
-// interface, walking the line as the sequential sweep does (side of the
-// regular rows from the line's start and after each block, factors from the
-// prefix tables up to the first MIB row and per node from there on).
+// Coefficients of one direction from the crossing lines' factors, one thread
+// per listed line.
 template <int D>
 __global__ void __launch_bounds__(TPB) k_coef32(const __grid_constant__ Dev P) {
-  const long long t = (long long)blockIdx.x * TPB + threadIdx.x;
-  if (t >= nlines<D>(P)) return;
+  const int c = blockIdx.x * TPB + threadIdx.x;
+  const int nc = P.nfcross[D];
+  if (c >= nc) return;
+  const int lid = P.fcross[D][c];
+  const int n2 = D == 2 ? P.ny : P.nz;
   Line L;
-  decode_line<D>(P, t, L);
-  if (L.boundary) return;
-  const int bfirst = P.bstart[D][L.lid], bend = P.bstart[D][L.lid + 1];
-  if (bfirst == bend) return;  // no crossing: the line reads the row tables
-  const int n = L.n;
-  const long long s = L.s;
-  const int ls = P.lside[D][L.lid];
-  const MibBlock* const blk = P.blk[D];
-  const int L1 = blk[bfirst].L;
-  const double* const pt = P.ptab[D][(ls >> 1) & 1];
-  int b = bfirst;
-  int side = (ls >> 1) & 1;
-  for (int j = 0; j < n; j++) {
-    const long long g = L.base + (long long)j * s;
-    const double bet = j >= L1 ? P.fbet[D][g] : pt[2 * j];
-    double a;
-    if (j == 0 || j == n - 1) {
-      a = 0.0;
-    } else if (b < bend && j >= blk[b].L) {
-      const int q = j - blk[b].L;
-      a = blk[b].ia[q];
-      if (q == blk[b].kind - 1) {
-        side = (blk[b].sides >> q) & 1;
-        b++;
-      }
-    } else {
-      a = P.ia[D][side];
-    }
-    const double gn = j == n - 1 ? 0.0 : j + 1 >= L1 ? P.fgam[D][g + s] : pt[2 * (j + 1) + 1];
-    P.cib[D][g] = (float)(1.0 / bet);
-    P.cp[D][g] = (float)(-(a / bet));
-    P.cq[D][g] = (float)(-gn);
+  decode_line<D>(P, (long long)(lid % n2) * (D == 0 ? P.ny : P.nx) + lid / n2, L);
+  for (int j = 0; j < L.n; j++) {
+    const long long g = L.base + (long long)j * L.s;
+    const double2 b = P.cb[D][(long long)j * nc + c];
+    P.cib[D][g] = (float)b.y;
+    P.cp[D][g] = (float)(-(P.ca[D][(long long)j * nc + c] / b.x));
+    P.cq[D][g] = (float)(-P.cg[D][(long long)j * nc + c]);
   }
 }
 
@@ -557,14 +497,11 @@ __global__ void __launch_bounds__(TPB) k_ctab32(const __grid_constant__ Dev P) {
   const int i = blockIdx.x * TPB + threadIdx.x;
   if (i >= 2 * n) return;
   const int side = i / n, j = i % n;
-  const double* const pt = P.ptab[D][side];
-  const double bet = pt[2 * j];
-  const double a = j == 0 || j == n - 1 ? 0.0 : P.ia[D][side];
-  const double gn = j == n - 1 ? 0.0 : pt[2 * (j + 1) + 1];
+  const double2 b = P.tab[D][side][j];
   float* const T = P.ctab[D] + (size_t)side * 3 * n;
-  T[j] = (float)(1.0 / bet);
-  T[n + j] = (float)(-(a / bet));
-  T[2 * n + j] = (float)(-gn);
+  T[j] = (float)b.y;
+  T[n + j] = (float)(-(P.taba[D][side][j] / b.x));
+  T[2 * n + j] = (float)(-P.tabg[D][side][j]);
 }
 
 constexpr int WL_WARPS = 8;
@@ -922,7 +859,7 @@ __global__ void __launch_bounds__(TPB, 8) kbm_adi_resid(const Dev* __restrict__ 
 __global__ void __launch_bounds__(TPB) kbm_adi_resid_mib(const Dev* __restrict__ Ps,
                                                          const BatchItem* __restrict__ items) {
   BATCH_PROLOGUE
-  adi_resid_mib_body(P, w.cta, P.u0, P.r32, 0.0);
+  adi_resid_mib_body(P, w.cta, w.ncta, P.u0, P.r32, 0.0);
 }
 
 template <int D>
@@ -1026,9 +963,9 @@ bool mixed_shape_fits(int nmax) { return shape32_smem<S32_CH, S32_NS, S32_NT>(nm
 bool mixed_segments_fit(int n) { return n <= kSegMaxRows; }
 
 int build_mixed_coefs(const Dev& P, cudaStream_t st) {
-  k_coef32<0><<<(unsigned)((nlines<0>(P) + TPB - 1) / TPB), TPB, 0, st>>>(P);
-  k_coef32<1><<<(unsigned)((nlines<1>(P) + TPB - 1) / TPB), TPB, 0, st>>>(P);
-  k_coef32<2><<<(unsigned)((nlines<2>(P) + TPB - 1) / TPB), TPB, 0, st>>>(P);
+  if (P.nfcross[0] > 0) k_coef32<0><<<(P.nfcross[0] + TPB - 1) / TPB, TPB, 0, st>>>(P);
+  if (P.nfcross[1] > 0) k_coef32<1><<<(P.nfcross[1] + TPB - 1) / TPB, TPB, 0, st>>>(P);
+  if (P.nfcross[2] > 0) k_coef32<2><<<(P.nfcross[2] + TPB - 1) / TPB, TPB, 0, st>>>(P);
   k_ctab32<0><<<(2 * P.nx + TPB - 1) / TPB, TPB, 0, st>>>(P);
   k_ctab32<1><<<(2 * P.ny + TPB - 1) / TPB, TPB, 0, st>>>(P);
   k_ctab32<2><<<(2 * P.nz + TPB - 1) / TPB, TPB, 0, st>>>(P);
@@ -1066,7 +1003,7 @@ void configure_mixed_batch_kernels() {
 }
 
 int launch_step_batch_mixed(const MixedBatchPlan& b, cudaStream_t st) {
-  int launches = launch_batch_jumps(b.Ps, b.jumps, b.njumps, st);
+  int launches = 0;
   if (b.nmib > 0) {
     kbm_adi_resid_mib<<<b.nmib, TPB, 0, st>>>(b.Ps, b.mib);
     launches++;
@@ -1082,24 +1019,20 @@ int launch_step_batch_mixed(const MixedBatchPlan& b, cudaStream_t st) {
 int launch_step_mixed(const Dev& P, const StepTimes& T, double* u, cudaStream_t st, cudaEvent_t* ev,
                       const SideStream* side) {
   int launches = 0;
-  // The jumps and the residual's MIB rows (which read the jumps) run on the
-  // side stream, beside the pointwise residual: the two passes write
-  // disjoint nodes and read only the state.
-  const bool fork = side && side->stream && (P.ncross > 0 || P.nmibnode > 0);
+  // The residual's MIB rows run on the side stream, beside the pointwise
+  // residual: the two passes write disjoint nodes and read only the state.
+  const bool fork = side && side->stream && P.nmibnode > 0;
   cudaStream_t sst = fork ? side->stream : st;
   if (fork) {
     cudaEventRecord(side->fork, st);
     cudaStreamWaitEvent(sst, side->fork, 0);
   }
-  if (ev) cudaEventRecord(ev[0], sst);
-  if (P.ncross > 0) {
-    launch_jumps(P, T.e_next, sst);
-    launches++;
-  }
-  if (ev) cudaEventRecord(ev[1], sst);
+  // (slot 0, once the jump pass: the MIB rows evaluate the jumps they use)
+  if (ev) cudaEventRecord(ev[0], st);
+  if (ev) cudaEventRecord(ev[1], st);
   if (ev) cudaEventRecord(ev[2], st);
   if (P.nmibnode > 0) {
-    k_adi_resid_mib<<<(P.nmibnode + TPB - 1) / TPB, TPB, 0, sst>>>(P, u, P.r32, T.e_next);
+    k_adi_resid_mib<<<mib_nodes_grid(P), TPB, 0, sst>>>(P, u, P.r32, T.e_next);
     launches++;
   }
   k_adi_resid<2><<<pointwise_rows_grid(P), TPB, 0, st>>>(P, u, P.r32, T.e_next);

@@ -94,28 +94,28 @@ def size_class(spec: Spec) -> str:
 def device_bytes_bound(spec: Spec, ncrossings: int, sms: int = 148, precision: str = "plain") -> int:
     """An upper bound on the device memory mts_create allocates for `spec`
     with `ncrossings` crossings (the layout of the library's allocations: two
-    FP64 fields, FP64 and FP32 per-node factors for every direction, the FP32
-    increment, both d' scratches, the tables and the MIB data), plus, for the
-    mixed form, the segmented solves' per-node coefficients (three FP32
-    values per node and direction, built when the form is switched on)."""
+    FP64 fields, the FP32 increment, the crossing lines' factors, the FP32
+    ring sweeps' scratch and, for lines over 544 nodes, their per-node
+    factors, the tables and the MIB data), plus, for the mixed form, the
+    segmented solves' per-node coefficients (three FP32 values per node and
+    direction, built when the form is switched on)."""
     nx, ny, nz = spec.n
     N = nx * ny * nz
     nmax = max(spec.n)
     lines = [ny * nz, nx * nz, nx * ny]
     maxlines = max(lines)
     pad = 16 * nx * ny
-    t64 = min(sms * 512, maxlines + 512)
     t32 = min(sms * 448, maxlines + 448)
     b = 0
     b += 2 * 8 * (N + pad)                       # u0, u1
-    b += 8 * (nmax + 16) * t64                   # d' scratch, FP64
-    b += 3 * 2 * 8 * (N + pad)                   # per-node bet, gam (FP64)
-    b += 3 * 2 * 4 * (N + pad)                   # per-node 1/bet, gam (FP32)
+    b += ncrossings * nmax * 32                  # crossing lines' a, (bet, 1/bet), gam by row
     b += 4 * (N + pad) + 4 * (nmax + 16) * t32   # FP32 increment and d' scratch
-    b += N + sum(lines) * 5 + 4 * 3              # tags, line sides, CSR offsets
-    b += 3 * 2 * 2 * 12 * nmax + 3 * 3 * 8 * nmax  # prefix tables, axis tables
-    b += ncrossings * (432 + 3 * 12 + 88 + 16 + 3 * 8)  # blocks, block RHS, constants, jumps, MIB nodes
-    b += 4096 * 3 * 8 + 64                        # norm partials
+    if nmax > 544:
+        b += 3 * 2 * 4 * (N + pad)               # per-node 1/bet, gam (FP32)
+    b += N + pad + sum(lines) * 13 + 4 * 3       # tags, line sides, CSR offsets, line lists
+    b += 3 * 2 * 40 * nmax + 3 * 3 * 8 * nmax    # side tables, axis tables
+    b += ncrossings * (432 + 3 * 4 + 88 + 3 * 24 + 4)  # blocks, block RHS, constants, MIB nodes, line list
+    b += 4096 * 3 * 8 + 64 + 60 * 256            # norm partials, alignment
     if precision == "mixed" and spec.method == "adi" and nmax <= 544:
         b += 3 * 3 * 4 * N                        # cib, cp, cq per direction
     return int(b * 1.02) + (1 << 20)

@@ -63,18 +63,18 @@ def peak_hbm() -> float:
 # Algorithmic HBM bytes per grid node per launch of each kernel slot
 # (field reads/writes at 8 B plus the 1-byte node tag; scratch excluded).
 ALG_BYTES = {
-    "adi": {1: 17, 2: 16, 3: 24, 4: 24},
+    "adi": {2: 17, 3: 25, 4: 25},
     "lod-ie": {1: 17, 2: 17, 3: 17},
     "lod-cn": {1: 17, 2: 17, 3: 17},
     "ts": {1: 17, 2: 17, 3: 17, 4: 17, 5: 17},
 }
 SLOT_NAMES = {
-    # ADI: the jumps (with the MIB rows of the first right-hand side) run on
-    # a side stream beside the pointwise pass; that slot's time overlaps the next
-    "adi": ["jumps_side_stream", "adi_rhs", "adi_x_sweep", "adi_y_sweep", "adi_z_sweep"],
-    "lod-ie": ["jumps", "lod_x_sweep", "lod_y_sweep", "lod_z_sweep"],
-    "lod-cn": ["jumps", "lod_x_sweep", "lod_y_sweep", "lod_z_sweep"],
-    "ts": ["jumps", "ts_explicit_x", "ts_explicit_y", "ts_z_sweep", "ts_y_sweep", "ts_x_sweep"],
+    # (slot 0 is empty: the kernels evaluate the jumps they read; the ADI x
+    # sweep forms the first right-hand side of its lines)
+    "adi": ["empty", "adi_mib_rows", "adi_x_sweep", "adi_y_sweep", "adi_z_sweep"],
+    "lod-ie": ["empty", "lod_x_sweep", "lod_y_sweep", "lod_z_sweep"],
+    "lod-cn": ["empty", "lod_x_sweep", "lod_y_sweep", "lod_z_sweep"],
+    "ts": ["empty", "ts_explicit_x", "ts_explicit_y", "ts_z_sweep", "ts_y_sweep", "ts_x_sweep"],
 }
 
 
@@ -710,11 +710,10 @@ def main():
     if u_head is not None and not a.no_mixed:
         ms_m, kms_m, kn_m, (lm, l2m, _), um, _ = timed_run("mixed")
         v_m = job_value(world, nodes, a.steps, ms_m)
-        # the jumps and the residual's MIB rows run on a side stream beside
-        # the pointwise residual: the first slot is that stream's jumps
-        # launch (its time overlaps the second), the second the residual
-        # up to the join
-        names_m = ["jumps_side_stream", "residual_fp64", "x_solve_fp32", "y_solve_fp32", "z_solve_fp32_and_accumulate"]
+        # the residual's MIB rows run on a side stream beside the pointwise
+        # residual: the second slot is the residual up to the join (the first
+        # is empty)
+        names_m = ["empty", "residual_fp64", "x_solve_fp32", "y_solve_fp32", "z_solve_fp32_and_accumulate"]
         mixed = {
             "value": v_m, "unit": "cell-steps/s", "ms_per_step": ms_m / a.steps,
             "speedup_vs_plain": v_m / value,

@@ -634,7 +634,7 @@ mts_status finish_create(mts_problem* h) {
       D.mibnode = dm;
       D.nmibnode = (int)mibn.size();
       int4* ref = nullptr;
-      if (p.method == MTS_ADI && !mibn.empty()) CUDA_TRY(h->put(&ref, (const int4*)nullptr, mibn.size()));
+      if ((p.method == MTS_ADI || p.method == MTS_TS) && !mibn.empty()) CUDA_TRY(h->put(&ref, (const int4*)nullptr, mibn.size()));
       D.mibref = ref;
     }
     for (int d = 0; d < 3; d++) {

@@ -144,7 +144,7 @@ struct Dev {
   double* u1;  // scratch field
   const long long* mibnode;  // nodes with a MIB flag (any direction), ascending
   int nmibnode;
-  const int4* mibref;        // Douglas-ADI: per listed node its block in x, y, z (16 block + 4 kind + row, -1: none)
+  const int4* mibref;        // Douglas-ADI and TS: per listed node its block in x, y, z (16 block + 4 kind + row, -1: none)
   int* status;       // reserved
 };
 

@@ -55,24 +55,18 @@ __global__ void __launch_bounds__(TPB) k_adi_mib(const __grid_constant__ Dev P, 
 
 // TS explicit half step along D = x or y (TS::D_xx_r / D_yy_r, the LOD
 // Crank-Nicolson operators, trapezoidal.cc:319-895), then Set_bc at t_half.
+// At a MIB row of a D block, with its jump terms.  The block comes from ref
+// (Dev::mibref) and not from a search of the line's list, whose loads a thread
+// waits on one by one (113 x 97 x 141, 48 steps: 5.28 -> 4.95 ms).
 template <int D>
-__device__ __noinline__ double ts_explicit_mib(const Dev& P, const double* in, double E1, long long m, int ix, int iy,
-                                               int iz, int tg) {
+__device__ __forceinline__ double ts_explicit_mib(const Dev& P, const double* in, double E1, long long m, int ref,
+                                                  int side) {
   const long long s = D == 0 ? 1 : (long long)P.nx;
-  const double* vd = P.vd[D][tg & TAG_OUT];
-  int r = 0;
-  const MibBlock* b = D == 0 ? find_block<0>(P, iy * P.nz + iz, ix, r) : find_block<1>(P, ix * P.nz + iz, iy, r);
-  double sum;
-  if (b) {
-    const long long base = D == 0 ? m - ix : m - (long long)iy * P.nx;
-    sum = mib_sum(*b, r, [&](int j) { return in[base + (long long)j * s]; }, vd, true, jump_at(P, b->c0, E1),
-                  jump_at(P, b->c1, E1));
-  } else {
-    sum = 0.0;
-    sum += in[m - s] * vd[0];
-    sum += in[m] * vd[1];
-    sum += in[m + s] * vd[2];
-  }
+  const MibBlock& b = P.blk[D][ref >> 4];
+  const int kind = (ref >> 2) & 3, row = ref & 3;
+  const double* const p = in + m - (row + b.L) * s;  // row 0 of the line
+  const double2 Jl = jump_at(P, b.c0, E1), Jr = kind == 3 ? jump_at(P, b.c1, E1) : Jl;
+  const double sum = mib_sum(b, row, [&](int j) { return p[j * s]; }, P.vd[D][side], true, Jl, Jr);
   return P.kex * sum + in[m];
 }
 
@@ -91,11 +85,8 @@ __device__ __forceinline__ void k_ts_explicit_body(const Dev& P, unsigned cta_, 
     const int k = (int)(cta_ - nrow) * TPB + threadIdx.x;
     if (k >= P.nmibnode) return;
     const long long m = P.mibnode[k];
-    const int tg = P.tag[m];
-    if (!(tg & flag)) return;
-    int ix, iy, iz;
-    node_xyz(P, m, ix, iy, iz);
-    out[m] = ts_explicit_mib<D>(P, in, step_e(P, e1, 2), m, ix, iy, iz, tg);
+    const int ref = reinterpret_cast<const int*>(P.mibref)[4 * (long long)k + D];
+    if (ref >= 0) out[m] = ts_explicit_mib<D>(P, in, step_e(P, e1, 2), m, ref, P.tag[m] & TAG_OUT);
     return;
   }
   eh = step_e(P, eh, 1);
@@ -187,7 +178,7 @@ __global__ void __launch_bounds__(TPB) k_ts_explicit(const __grid_constant__ Dev
 // with 36 KB or more).  Against one line per thread over a ring of staged
 // rows with the partial solutions in a global scratch (the form before), us
 // per step: 65^3 Douglas-ADI 158 -> 54, 129^3 LOD-CN 277 -> 84, 113 x 97 x
-// 141 TS 252 -> 99, 257^3 Douglas-ADI 688 -> 680.
+// 141 TS 252 -> 99 (92 with the half steps' rows), 257^3 Douglas-ADI 688 -> 680.
 
 // Lines per tile and threads per CTA of each shape (mts_set_sweep_shape).
 #define MTS_SHAPES(X)                                                                           \

@@ -266,8 +266,10 @@ mts_status mts_set_profiling(mts_handle h, int32_t on);
 mts_status mts_profile_read(mts_handle h, double ms[8], int64_t launches[8]);
 
 /* Launch shape of the line-sweep kernels (lines per tile, threads per CTA),
- * chosen separately for the first, second and third implicit sweep of a step.  Every shape computes the same
- * bits; they differ only in speed.  mts_autotune times each compiled shape on
+ * chosen separately for the first, second and third implicit sweep of a step
+ * (x, y, z; for TS z, y, x); a shape is refused where its tile does not hold
+ * the lines of that sweep's direction.  Every shape computes the same bits;
+ * they differ only in speed.  mts_autotune times each compiled shape on
  * the handle's own problem for `steps` steps (the solution and time are
  * restored afterwards) and keeps the fastest per sweep; shapes[3] receives
  * the choice.  mts_sweep_shape_count gives the number of shapes. */

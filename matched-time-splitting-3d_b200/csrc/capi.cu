@@ -544,7 +544,8 @@ mts_status finish_create(mts_problem* h) {
   const int nmax = std::max(g.nx, std::max(g.ny, g.nz));
   for (int k = 0; k < 3; k++) {
     // (mts_autotune picks per problem and sweep)
-    D.shape[k] = mts::sweep_shape_default(nmax);
+    const int d = mts::sweep_direction(p.method, k);
+    D.shape[k] = mts::sweep_shape_default(d, nd[d]);
     if (D.shape[k] < 0) return fail(MTS_ERR_ARG, "grid lines too long for the sweep kernels' shared memory");
   }
   CUDA_TRY(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
@@ -1462,7 +1463,8 @@ int32_t mts_sweep_shape_count(void) { return mts::sweep_shape_count(); }
 mts_status mts_set_sweep_shape(mts_handle h, int32_t sweep, int32_t shape) {
   if (!h || sweep < 0 || sweep > 2 || shape < 0 || shape >= mts::sweep_shape_count())
     return fail(MTS_ERR_ARG, "bad sweep or shape index");
-  if (!mts::sweep_shape_fits(shape, std::max(h->g.nx, std::max(h->g.ny, h->g.nz))))
+  const int d = mts::sweep_direction(h->prm.method, sweep);
+  if (!mts::sweep_shape_fits(shape, d, d == 0 ? h->g.nx : d == 1 ? h->g.ny : h->g.nz))
     return fail(MTS_ERR_ARG, "shape needs more shared memory than this grid allows");
   h->dev.shape[sweep] = shape;
   return MTS_OK;
@@ -1569,10 +1571,16 @@ mts_status mts_autotune(mts_handle h, int32_t steps, int32_t shapes[3]) {
   h->profiling = true;
   int choice0[3] = {h->dev.shape[0], h->dev.shape[1], h->dev.shape[2]};
   for (int k = 0; k < 3; k++) choice[k] = choice0[k];
-  const int nmax = std::max(h->g.nx, std::max(h->g.ny, h->g.nz));
+  const int nd[3] = {h->g.nx, h->g.ny, h->g.nz};
   for (int s = 0; s < mts::sweep_shape_count() && st == MTS_OK; s++) {
-    if (!mts::sweep_shape_fits(s, nmax)) continue;
-    for (int k = 0; k < 3; k++) h->dev.shape[k] = s;
+    // (a sweep whose lines are too long for the shape keeps its own)
+    bool fits[3];
+    for (int k = 0; k < 3; k++) {
+      const int d = mts::sweep_direction(h->prm.method, k);
+      fits[k] = mts::sweep_shape_fits(s, d, nd[d]);
+      h->dev.shape[k] = fits[k] ? s : choice0[k];
+    }
+    if (!fits[0] && !fits[1] && !fits[2]) continue;
     st = mts_profile_read(h, nullptr, nullptr);
     if (st) break;
     st = advance(h, steps);
@@ -1582,7 +1590,7 @@ mts_status mts_autotune(mts_handle h, int32_t steps, int32_t shapes[3]) {
     st = mts_profile_read(h, ms, cnt);
     if (st) break;
     for (int k = 0; k < 3; k++)
-      if (ms[first + k] < best[k]) {
+      if (fits[k] && ms[first + k] < best[k]) {
         best[k] = ms[first + k];
         choice[k] = s;
       }

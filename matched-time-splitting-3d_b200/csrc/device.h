@@ -151,8 +151,9 @@ struct Dev {
 // Line-sweep shapes (lines per tile, threads per CTA); all give bit-identical
 // results, they differ only in speed.
 int sweep_shape_count();
-bool sweep_shape_fits(int shape, int nmax);  // shared memory of the shape within the limit
-int sweep_shape_default(int nmax);           // -1: no shape takes lines of nmax nodes
+int sweep_direction(int method, int sweep);       // direction of a step's first, second, third sweep
+bool sweep_shape_fits(int shape, int d, int n);   // shared memory of the shape for direction-d lines of n nodes
+int sweep_shape_default(int d, int n);            // -1: no shape takes them
 void configure_kernels();
 
 // Per-step exact-solution time factors.

@@ -182,8 +182,8 @@ __global__ void __launch_bounds__(TPB) k_ts_explicit(const __grid_constant__ Dev
 
 // Lines per tile and threads per CTA of each shape (mts_set_sweep_shape).
 #define MTS_SHAPES(X)                                                                           \
-  X(0, 32, 256) X(1, 32, 128) X(2, 32, 192) X(3, 16, 256) X(4, 16, 128) X(5, 16, 96) X(6, 8, 128) \
-  X(7, 8, 96) X(8, 4, 128) X(9, 4, 96)
+  X(0, 32, 256) X(1, 32, 128) X(2, 32, 192) X(3, 16, 256) X(4, 8, 96) X(5, 16, 96) X(6, 8, 128) \
+  X(7, 16, 128) X(8, 4, 128) X(9, 4, 96)
 
 // Doubles per row of a tile: an x tile is written along its lines, so its
 // rows are padded to an odd stride.
@@ -1197,11 +1197,14 @@ void set_smem_attr() {
 
 int sweep_shape_count() { return 10; }
 
-bool sweep_shape_fits(int shape, int nmax) {
+// TS runs its implicit sweeps z, y, x, the others x, y, z.
+int sweep_direction(int method, int sweep) { return method == 3 ? 2 - sweep : sweep; }
+
+bool sweep_shape_fits(int shape, int d, int n) {
   switch (shape) {
 #define MTS_FITS(id, nl, nt) \
   case id:                   \
-    return nmax <= kMaxLineRows && tile_smem<0, nl>(nmax) <= (size_t)kMaxTileSmem;
+    return n <= kMaxLineRows && (d == 0 ? tile_smem<0, nl>(n) : tile_smem<1, nl>(n)) <= (size_t)kMaxTileSmem;
     MTS_SHAPES(MTS_FITS)
 #undef MTS_FITS
     default:
@@ -1210,10 +1213,10 @@ bool sweep_shape_fits(int shape, int nmax) {
 }
 
 // 32 lines per tile while shared memory holds them, else the most it holds.
-int sweep_shape_default(int nmax) {
+int sweep_shape_default(int d, int n) {
   const int order[4] = {0, 3, 6, 8};
   for (int s : order)
-    if (sweep_shape_fits(s, nmax)) return s;
+    if (sweep_shape_fits(s, d, n)) return s;
   return -1;
 }
 

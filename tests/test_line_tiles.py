@@ -96,3 +96,28 @@ def test_factors_out_of_range_take_the_divide():
     """A time step so long that the factors pass 2^100."""
     spec = M.Spec(n=(25, 25, 25), method="lod-ie", mib=1, dt=1e32, t0=0.0, **ELL)
     _check(spec, None, 1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("method", ["adi", "lod-cn", "ts"])
+@pytest.mark.parametrize("n", [(1455, 17, 18), (17, 1455, 18), (18, 17, 815)])
+def test_a_sweep_takes_its_shape_by_its_own_axis(method, n):
+    """Grids with one long axis: the sweeps along the short ones take every
+    shape, the one along the long axis those whose tiles hold its lines."""
+    spec = M.Spec(n=n, method=method, mib=2, beta_out=37.5, dt=0.02, **ELL)
+    _check(spec, None, 2)
+    lines = (32, 32, 32, 16, 8, 16, 8, 16, 4, 4)  # of each shape's tile
+
+    def fits(d, shape):  # the tile's rows (x tiles padded by one) and a side's factors
+        return n[d] * (8 * (lines[shape] + (d == 0)) + 24) <= 226 * 1024
+
+    with M.Solver(spec) as s:
+        dirs = (2, 1, 0) if method == "ts" else (0, 1, 2)
+        for sweep, d in enumerate(dirs):
+            for shape in range(len(lines)):
+                if fits(d, shape):
+                    s.set_sweep_shape(sweep, shape)
+                else:
+                    with pytest.raises(M.MtsError, match="shared memory"):
+                        s.set_sweep_shape(sweep, shape)
+        assert all(fits(d, shape) for d, shape in zip(dirs, s.autotune(1)))

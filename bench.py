@@ -69,8 +69,9 @@ ALG_BYTES = {
     "ts": {1: 17, 2: 17, 3: 17, 4: 17, 5: 17},
 }
 SLOT_NAMES = {
-    # (slot 0 is empty: the kernels evaluate the jumps they read; the ADI x
-    # sweep forms the first right-hand side of its lines)
+    # (slot 0 is empty: the kernels evaluate the jumps they read; an ADI x
+    # tile forms the first right-hand side of its lines, before an x ring it is
+    # formed in slot 1)
     "adi": ["empty", "adi_mib_rows", "adi_x_sweep", "adi_y_sweep", "adi_z_sweep"],
     "lod-ie": ["empty", "lod_x_sweep", "lod_y_sweep", "lod_z_sweep"],
     "lod-cn": ["empty", "lod_x_sweep", "lod_y_sweep", "lod_z_sweep"],

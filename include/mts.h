@@ -257,18 +257,22 @@ mts_status mts_get_stream(mts_handle h, void** stream);
 
 /* Per-kernel timing with CUDA events recorded on the handle's stream around
  * every launch of a step (negligible overhead; off by default).  Slots, in
- * launch order: Douglas-ADI {0 empty, 1 MIB rows (mixed: residual), 2 x sweep,
- * 3 y sweep, 4 z sweep}; LOD {0 empty, 1 x sweep, 2 y sweep, 3 z sweep}; TS
+ * launch order: Douglas-ADI {0 empty, 1 MIB rows (before an x ring sweep the
+ * whole first right-hand side; mixed: residual), 2 x sweep, 3 y sweep, 4 z
+ * sweep}; LOD {0 empty, 1 x sweep, 2 y sweep, 3 z sweep}; TS
  * {0 empty, 1 explicit x, 2 explicit y, 3 z sweep, 4 y sweep, 5 x sweep}.
  * mts_profile_read synchronizes, returns the summed milliseconds and launch
  * counts per slot since the last read, and resets them. */
 mts_status mts_set_profiling(mts_handle h, int32_t on);
 mts_status mts_profile_read(mts_handle h, double ms[8], int64_t launches[8]);
 
-/* Launch shape of the line-sweep kernels (lines per tile, threads per CTA),
- * chosen separately for the first, second and third implicit sweep of a step
+/* Launch shape of the line-sweep kernels (tiles: lines per tile, threads per
+ * CTA; then rings: rows per chunk, chunks, threads per CTA), chosen separately for the first, second and third implicit sweep of a step
  * (x, y, z; for TS z, y, x); a shape is refused where its tile does not hold
- * the lines of that sweep's direction.  Every shape computes the same bits;
+ * the lines of that sweep's direction.  The ring sweeps' data (16 bytes a node
+ * and direction and a scratch of up to 0.53 MB per row of the longest line) is
+ * allocated with the first plain step that takes one; where there is no memory
+ * for it the tiles take the sweep.  Every shape computes the same bits;
  * they differ only in speed.  mts_autotune times each compiled shape on
  * the handle's own problem for `steps` steps (the solution and time are
  * restored afterwards) and keeps the fastest per sweep; shapes[3] receives

@@ -83,6 +83,11 @@ struct mts_problem {
   // form; a build that fails part way is done again on the next switch
   bool fast_built = false;
   bool mixed_built = false;
+  // the ring sweeps' data (ensure_rings): a block per direction, the d'
+  // scratch and its size
+  void* ring_mem[4] = {nullptr, nullptr, nullptr, nullptr};
+  size_t ring_bytes[4] = {0, 0, 0, 0};
+  bool ring_refused = false;  // no memory for them: the tiles take those sweeps
   // the error reports' tables (mts_fp_errors, mts_jump_errors), built on
   // first use
   mts_crossing* fp_cr = nullptr;
@@ -112,6 +117,8 @@ struct mts_problem {
     for (auto& a : ev_free)
       for (cudaEvent_t e : a) cudaEventDestroy(e);
     for (const Slab& sl : slabs) cudaFreeAsync(sl.base, stream);
+    for (void* b : ring_mem)
+      if (b) cudaFreeAsync(b, stream);
     if (stream) {
       cudaStreamSynchronize(stream);
       cudaStreamDestroy(stream);
@@ -266,6 +273,81 @@ cudaError_t ensure_side_stream(mts_problem* h) {
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->side.fork, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->side.join, cudaEventDisableTiming);
   return e;
+}
+
+// Gives back block i of the ring sweeps' data (a direction's, or 3: the d'
+// scratch).
+void release_ring(mts_problem* h, int i) {
+  if (h->ring_mem[i]) cudaFreeAsync(h->ring_mem[i], h->stream);
+  h->device_bytes -= (int64_t)h->ring_bytes[i];
+  h->ring_mem[i] = nullptr;
+  h->ring_bytes[i] = 0;
+  if (i == 3) {
+    h->dev.dp = nullptr;
+  } else {
+    h->dev.fbet[i] = h->dev.fgam[i] = nullptr;
+    h->dev.rblk[i] = nullptr;
+  }
+}
+
+// The data of the ring sweeps that the handle's shapes name, built on the
+// handle's stream before its first step that takes one: per direction the
+// crossing lines' factors by node and the block rows' right-hand sides, and
+// the d' scratch that the sweeps of a step share.  Where there is no memory
+// for them (or the stream is being captured, where memory would be the
+// graph's) the tiles take the sweep (kernels.cu).
+cudaError_t ensure_rings(mts_problem* h) {
+  mts::Dev& D = h->dev;
+  const int nd[3] = {D.nx, D.ny, D.nz};
+  size_t dp = 0;
+  bool need[3] = {false, false, false};
+  for (int k = 0; k < 3; k++) {
+    if (D.shape[k] < mts::kTileShapes) continue;
+    const int d = mts::sweep_direction(D.method, k);
+    need[d] = true;
+    dp = std::max(dp, sizeof(double) * (size_t)(nd[d] + mts::kRowPad) *
+                          (size_t)mts::ring_threads(D, D.shape[k] - mts::kTileShapes, d));
+  }
+  bool missing = dp > h->ring_bytes[3];
+  for (int d = 0; d < 3; d++) missing = missing || (need[d] && !D.rblk[d]);
+  if (!missing || h->ring_refused) return cudaSuccess;
+  cudaStreamCaptureStatus cap;
+  cudaError_t e = cudaStreamIsCapturing(h->stream, &cap);
+  if (e != cudaSuccess || cap != cudaStreamCaptureStatusNone) return e;
+  auto block = [&](int i, size_t bytes) {
+    e = cudaMallocAsync(&h->ring_mem[i], bytes, h->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(h->ring_mem[i], 0, bytes, h->stream);
+    if (e != cudaSuccess) return false;
+    h->ring_bytes[i] = bytes;
+    h->device_bytes += (int64_t)bytes;
+    return true;
+  };
+  bool ok = true;
+  if (dp > h->ring_bytes[3]) {
+    release_ring(h, 3);
+    ok = block(3, dp);
+    if (ok) D.dp = (double*)h->ring_mem[3];
+  }
+  const size_t field = (size_t)(D.nn + (long long)mts::kRowPad * D.nx * D.ny);
+  for (int d = 0; d < 3 && ok; d++) {
+    if (!need[d] || D.rblk[d]) continue;
+    const size_t f = D.nblk[d] > 0 ? field : 0;
+    ok = block(d, sizeof(double) * (2 * f + 3 * (size_t)D.nblk[d] + 1));
+    if (!ok) break;
+    double* const p = (double*)h->ring_mem[d];
+    if (f) mts::build_ring_factors(D, d, p, p + f, h->stream);
+    D.fbet[d] = p;
+    D.fgam[d] = p + f;
+    D.rblk[d] = p + 2 * f;
+  }
+  if (!ok) {
+    for (int i = 0; i < 4; i++) release_ring(h, i);
+    cudaGetLastError();
+    if (e != cudaErrorMemoryAllocation) return e;
+    h->ring_refused = true;
+    return cudaSuccess;
+  }
+  return cudaGetLastError();
 }
 
 // Builds every device-side table of a problem from its grid, tags and
@@ -530,6 +612,7 @@ mts_status finish_create(mts_problem* h) {
   static bool configured = false;
   if (!configured) {
     mts::configure_kernels();
+    mts::configure_ring_kernels();
     mts::configure_mixed_kernels();
     mts::configure_batch_kernels();
     mts::configure_fast_kernels();
@@ -545,7 +628,7 @@ mts_status finish_create(mts_problem* h) {
   for (int k = 0; k < 3; k++) {
     // (mts_autotune picks per problem and sweep)
     const int d = mts::sweep_direction(p.method, k);
-    D.shape[k] = mts::sweep_shape_default(d, nd[d]);
+    D.shape[k] = mts::sweep_shape_default(p.method, d, nd[d], line_count(g, d), D.sweep_blocks);
     if (D.shape[k] < 0) return fail(MTS_ERR_ARG, "grid lines too long for the sweep kernels' shared memory");
   }
   CUDA_TRY(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
@@ -757,8 +840,10 @@ mts_status enqueue_step(mts_problem* h, double t_prev, double t_half, double t_n
     h->launches += mts::launch_step_fast(h->dev, T, h->u0, h->u1, h->stream, ev, &h->side);
   else if (h->dev.precision == 1)
     h->launches += mts::launch_step_mixed(h->dev, T, h->u0, h->stream, ev, &h->side);
-  else
-    h->launches += mts::launch_step(h->dev, T, h->u0, h->u1, h->stream, ev);
+  else {
+    CUDA_TRY(ensure_rings(h));
+    h->launches += mts::launch_step(h->dev, T, h->u0, h->u1, h->stream, ev, &h->side);
+  }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(MTS_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(e));
   h->t = t_next;
@@ -1148,6 +1233,7 @@ mts_status mts_batch_advance_steps(const mts_handle* hs, const int32_t* counts, 
     mts_problem* h = hs[i];
     if (!solo(i)) continue;
     BATCH_TRY(ensure_side_stream(h));
+    if (h->dev.precision == 0) BATCH_TRY(ensure_rings(h));
     for (int k = 0; k < counts[i]; k++) {
       mts::StepTimes T{0, 0, 0};  // unused: the kernels read the table
       if (h->dev.precision == 2)
@@ -1155,7 +1241,7 @@ mts_status mts_batch_advance_steps(const mts_handle* hs, const int32_t* counts, 
       else if (h->dev.precision == 1)
         h->launches += mts::launch_step_mixed(h->dev, T, h->u0, h->stream, nullptr, &h->side);
       else
-        h->launches += mts::launch_step(h->dev, T, h->u0, h->u1, h->stream, nullptr);
+        h->launches += mts::launch_step(h->dev, T, h->u0, h->u1, h->stream, nullptr, &h->side);
       mts::launch_tick(h->dev, h->stream);
       h->launches++;
     }
@@ -1467,6 +1553,7 @@ mts_status mts_set_sweep_shape(mts_handle h, int32_t sweep, int32_t shape) {
   if (!mts::sweep_shape_fits(shape, d, d == 0 ? h->g.nx : d == 1 ? h->g.ny : h->g.nz))
     return fail(MTS_ERR_ARG, "shape needs more shared memory than this grid allows");
   h->dev.shape[sweep] = shape;
+  h->ring_refused = false;
   return MTS_OK;
 }
 
@@ -1581,6 +1668,7 @@ mts_status mts_autotune(mts_handle h, int32_t steps, int32_t shapes[3]) {
       h->dev.shape[k] = fits[k] ? s : choice0[k];
     }
     if (!fits[0] && !fits[1] && !fits[2]) continue;
+    h->ring_refused = false;
     st = mts_profile_read(h, nullptr, nullptr);
     if (st) break;
     st = advance(h, steps);
@@ -1589,11 +1677,16 @@ mts_status mts_autotune(mts_handle h, int32_t steps, int32_t shapes[3]) {
     int64_t cnt[8];
     st = mts_profile_read(h, ms, cnt);
     if (st) break;
-    for (int k = 0; k < 3; k++)
-      if (fits[k] && ms[first + k] < best[k]) {
-        best[k] = ms[first + k];
+    for (int k = 0; k < 3; k++) {
+      // (a Douglas-ADI x tile forms the first right-hand side itself, before
+      // an x ring sweep it has the slot before)
+      const double t = ms[first + k] + (k == 0 && h->prm.method == MTS_ADI ? ms[first - 1] : 0.0);
+      const int d = mts::sweep_direction(h->prm.method, k);
+      if (fits[k] && (s < mts::kTileShapes || h->dev.rblk[d]) && t < best[k]) {
+        best[k] = t;
         choice[k] = s;
       }
+    }
     CUDA_TRY(cudaMemcpyAsync(h->u0, backup, bytes, cudaMemcpyDeviceToDevice, h->stream));
     h->t = t0;
   }
@@ -1601,10 +1694,14 @@ mts_status mts_autotune(mts_handle h, int32_t steps, int32_t shapes[3]) {
   CUDA_TRY(cudaMemcpyAsync(h->u0, backup, bytes, cudaMemcpyDeviceToDevice, h->stream));
   CUDA_TRY(cudaStreamSynchronize(h->stream));
   h->t = t0;
+  bool ring[4] = {false, false, false, false};
   for (int k = 0; k < 3; k++) {
     h->dev.shape[k] = choice[k];
     if (shapes) shapes[k] = choice[k];
+    if (choice[k] >= mts::kTileShapes) ring[3] = ring[mts::sweep_direction(h->prm.method, k)] = true;
   }
+  for (int i = 0; i < 4; i++)
+    if (!ring[i]) release_ring(h, i);
   return st;
 }
 

@@ -96,6 +96,15 @@ struct Dev {
   const double* ca[3];
   const double2* cb[3];
   const double* cg[3];
+  // The ring sweeps' data (ring.cu), built before a handle's first step that
+  // takes one, for the directions that do (null before): by node bet_j and
+  // gam_j of the crossing lines from their first MIB row on; the block rows'
+  // right-hand sides of the sweep in flight, [3*block + q]; the partial
+  // solutions d'_j, [row][thread].
+  const double* fbet[3];
+  const double* fgam[3];
+  double* rblk[3];
+  double* dp;
   int plain_div;     // a factor is out of the range of the quotients from reciprocals (kernels.cu)
   int nblk[3];
   int sweep_blocks;  // SMs
@@ -148,13 +157,42 @@ struct Dev {
   int* status;       // reserved
 };
 
-// Line-sweep shapes (lines per tile, threads per CTA); all give bit-identical
-// results, they differ only in speed.
+// What a bit-exact line sweep does: its right-hand side (of the copied field,
+// of the line's explicit stencil, of TS's z step, or the whole first
+// right-hand side of Douglas-ADI) and its fields.
+enum Kind { K_COPY = 0, K_STENCIL = 1, K_TS_Z = 2, K_ADI = 3 };
+
+struct SweepIO {
+  const double* stin;  // field the explicit stencil reads
+  const double* add;   // field added to the explicit part (or copied)
+  double* out;         // result field (may alias stin/add: a line is read
+                       // completely before any of it is written)
+  double e1;           // exp(-t_next): boundary data, source, jumps
+  double e0;           // exp(-t_prev): TS source of the first half step
+  double k;            // explicit factor: -dt (ADI), 0.5*dt (LOD-CN, TS)
+  int jumps;           // MIB rows carry jump terms (LOD, TS)
+  int bmode;           // boundary lines: 0 keep, 1 Outer_u(t_next), 2 + dt*f
+  int last;            // LOD: epilogue adds dt*f(t_next)
+};
+
+// Line-sweep shapes: tiles (lines per tile, threads per CTA; kernels.cu), then
+// rings (rows per chunk, chunks, threads per CTA; ring.cu).  All give
+// bit-identical results, they differ only in speed.
+constexpr int kTileShapes = 10, kRingShapes = 3;
 int sweep_shape_count();
 int sweep_direction(int method, int sweep);       // direction of a step's first, second, third sweep
 bool sweep_shape_fits(int shape, int d, int n);   // shared memory of the shape for direction-d lines of n nodes
-int sweep_shape_default(int d, int n);            // -1: no shape takes them
+int sweep_shape_default(int method, int d, int n, long long lines, int sms);  // -1: no shape takes them
+int tile_shape_default(int d, int n, bool adi_x);  // among the tiles; adi_x: the x sweep of Douglas-ADI
 void configure_kernels();
+// The ring sweeps (ring.cu; ring: shape - kTileShapes).
+bool ring_fits(int ring, int n);
+int ring_default(int method, int d, int n, double per_sm);  // lines per SM; -1: none fits
+long long ring_threads(const Dev& P, int ring, int d);  // threads of the launch: columns of Dev::dp
+void configure_ring_kernels();
+void build_ring_factors(const Dev& P, int d, double* fbet, double* fgam, cudaStream_t stream);
+void launch_adi_rhs(const Dev& P, const double* u, double* r, double e_next, cudaStream_t stream);
+void launch_ring_sweep(const Dev& P, int d, int kind, const SweepIO& io, int ring, cudaStream_t stream);
 
 // Per-step exact-solution time factors.
 struct StepTimes {
@@ -175,7 +213,8 @@ struct SideStream {
   cudaStream_t stream;
   cudaEvent_t fork, join;
 };
-int launch_step(const Dev& P, const StepTimes& T, double* u0, double* u1, cudaStream_t stream, cudaEvent_t* ev);
+int launch_step(const Dev& P, const StepTimes& T, double* u0, double* u1, cudaStream_t stream, cudaEvent_t* ev,
+                const SideStream* side);
 // The mixed-precision Douglas-ADI step (mixed.cu), in place on u.
 int launch_step_mixed(const Dev& P, const StepTimes& T, double* u, cudaStream_t stream, cudaEvent_t* ev,
                       const SideStream* side);

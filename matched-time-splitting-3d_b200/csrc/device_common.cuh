@@ -17,21 +17,6 @@ constexpr int kMaxLineRows = 3245;     // the longest line the bit-exact form ta
 // The batched line tiles: three of them (and their problems' records) to an SM.
 constexpr int kBatchTileSmem = 70 * 1024;
 
-enum Kind { K_COPY = 0, K_STENCIL = 1, K_TS_Z = 2, K_ADI = 3 };
-
-struct SweepIO {
-  const double* stin;  // field the explicit stencil reads
-  const double* add;   // field added to the explicit part (or copied)
-  double* out;         // result field (may alias stin/add: a line is read
-                       // completely before any of it is written)
-  double e1;           // exp(-t_next): boundary data, source, jumps
-  double e0;           // exp(-t_prev): TS source of the first half step
-  double k;            // explicit factor: -dt (ADI), 0.5*dt (LOD-CN, TS)
-  int jumps;           // MIB rows carry jump terms (LOD, TS)
-  int bmode;           // boundary lines: 0 keep, 1 Outer_u(t_next), 2 + dt*f
-  int last;            // LOD: epilogue adds dt*f(t_next)
-};
-
 // ---------------------------------------------------------------------------
 // Exact solutions (eq 0: src/equation/eq_0.cc; eq 8: see oracle/ref_harness.cc
 // Eq8 for the operand order).
@@ -259,6 +244,43 @@ __device__ __forceinline__ const MibBlock* find_block(const Dev& P, int lid, int
   }
   row = 0;
   return nullptr;
+}
+
+// Right-hand sides of block k's rows (K_COPY, K_STENCIL, K_TS_Z) from the
+// fields, jump terms and Convert2Tri row operations included (the explicit MIB
+// stencil of douglas_adi.cc:112-210 / lod.cc:337-496, the jump terms of D_xx_l
+// lod.cc:960-1097).
+template <int D, int KIND>
+__device__ __forceinline__ void block_rhs(const Dev& P, const SweepIO& io, double E0, double E1, int k, long long base,
+                                          int i1, int i2, double (&r)[3]) {
+  const long long s = D == 0 ? 1 : D == 1 ? (long long)P.nx : (long long)P.nx * P.ny;
+  const MibBlock& b = P.blk[D][k];
+  double2 Jl = make_double2(0.0, 0.0), Jr = Jl;
+  if (io.jumps) {
+    Jl = jump_at(P, b.c0, E1);
+    if (b.kind == 3) Jr = jump_at(P, b.c1, E1);
+  }
+  const double* const stin = KIND == K_COPY ? io.add : io.stin;
+  auto U = [&](int j) { return stin[base + (long long)j * s]; };
+  r[0] = r[1] = r[2] = 0.0;
+  for (int q = 0; q < b.kind; q++) {
+    const int jj = b.L + q;
+    const int side = (b.sides >> q) & 1;
+    const double av = io.add[base + (long long)jj * s];
+    if (KIND == K_COPY) {
+      r[q] = av;
+    } else {
+      const double sum = mib_sum(b, q, U, P.vd[D][side], io.jumps, Jl, Jr);
+      double v = io.k * sum + av;
+      if (KIND == K_TS_Z) {
+        v = v + P.hdt * source(P, E0, side, i1, i2, jj);
+        v = v + P.hdt * source(P, E1, side, i1, i2, jj);
+      }
+      r[q] = v;
+    }
+  }
+  implicit_rows(P, b, r, P.vd[D][b.sides & 1], P.vd[D][(b.sides >> 1) & 1], P.vd[D][(b.sides >> 2) & 1], io.jumps,
+                Jl, Jr);
 }
 
 // The Douglas-ADI data of a MIB node in one direction: the explicit sum of

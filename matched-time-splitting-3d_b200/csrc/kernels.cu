@@ -13,6 +13,8 @@
 // makes the plain FP64 path bit-identical to the reference CPU build.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "device.h"
 
 #include "device_common.cuh"
@@ -255,43 +257,6 @@ __device__ __forceinline__ void face_lines(const Dev& P, unsigned cta, unsigned 
     if (io.bmode == 2) v = v + P.dt * source(P, E1, P.tag[m] & TAG_OUT, ix, iy, iz);
     io.out[m] = v;
   }
-}
-
-// Right-hand sides of block k's rows (K_COPY, K_STENCIL, K_TS_Z) from the
-// fields, jump terms and Convert2Tri row operations included.  row0: the
-// shared-memory row 0 of the line.
-template <int D, int KIND, int RS>
-__device__ __forceinline__ void block_rhs(const Dev& P, const SweepIO& io, double E0, double E1, int k, long long base,
-                                       int i1, int i2, double* row0) {
-  const long long s = D == 0 ? 1 : D == 1 ? (long long)P.nx : (long long)P.nx * P.ny;
-  const MibBlock& b = P.blk[D][k];
-  double2 Jl = make_double2(0.0, 0.0), Jr = Jl;
-  if (io.jumps) {
-    Jl = jump_at(P, b.c0, E1);
-    if (b.kind == 3) Jr = jump_at(P, b.c1, E1);
-  }
-  const double* const stin = KIND == K_COPY ? io.add : io.stin;
-  auto U = [&](int j) { return stin[base + (long long)j * s]; };
-  double r[3] = {0.0, 0.0, 0.0};
-  for (int q = 0; q < b.kind; q++) {
-    const int jj = b.L + q;
-    const int side = (b.sides >> q) & 1;
-    const double av = io.add[base + (long long)jj * s];
-    if (KIND == K_COPY) {
-      r[q] = av;
-    } else {
-      const double sum = mib_sum(b, q, U, P.vd[D][side], io.jumps, Jl, Jr);
-      double v = io.k * sum + av;
-      if (KIND == K_TS_Z) {
-        v = v + P.hdt * source(P, E0, side, i1, i2, jj);
-        v = v + P.hdt * source(P, E1, side, i1, i2, jj);
-      }
-      r[q] = v;
-    }
-  }
-  implicit_rows(P, b, r, P.vd[D][b.sides & 1], P.vd[D][(b.sides >> 1) & 1], P.vd[D][(b.sides >> 2) & 1], io.jumps,
-                Jl, Jr);
-  for (int q = 0; q < b.kind; q++) row0[(b.L + q) * RS] = r[q];
 }
 
 // The Convert2Tri row operations of x block k on the first right-hand side's
@@ -588,8 +553,12 @@ __device__ __forceinline__ void tile_blocks(const Dev& P, const SweepIO& io, con
       const int bend = P.bstart[D][lid + 1];
       const long long base = line_base<D>(P, i1, i2);
       const double E0 = KIND == K_TS_Z ? step_e(P, io.e0, 0) : 0.0;
-      for (int k = P.bstart[D][lid] + e / NL; k < bend; k += (NT - 32 * BW) / NL)
-        block_rhs<D, KIND, RS>(P, io, E0, E1, k, base, i1, i2, sm + c);
+      for (int k = P.bstart[D][lid] + e / NL; k < bend; k += (NT - 32 * BW) / NL) {
+        double r[3];
+        block_rhs<D, KIND>(P, io, E0, E1, k, base, i1, i2, r);
+        const MibBlock& b = P.blk[D][k];
+        for (int q = 0; q < b.kind; q++) sm[(b.L + q) * RS + c] = r[q];
+      }
     }
   }
 }
@@ -1182,6 +1151,12 @@ void sweep(const Dev& P, const SweepIO& io, int shape, cudaStream_t st) {
     break;
     MTS_SHAPES(MTS_CASE)
 #undef MTS_CASE
+    default:
+      // a ring, where its data could be built
+      if (KIND != K_ADI && P.rblk[D])
+        launch_ring_sweep(P, D, KIND, io, shape - kTileShapes, st);
+      else
+        sweep<D, KIND>(P, io, tile_shape_default(D, D == 0 ? P.nx : D == 1 ? P.ny : P.nz, KIND == K_ADI), st);
   }
 }
 
@@ -1195,7 +1170,7 @@ void set_smem_attr() {
 
 }  // namespace
 
-int sweep_shape_count() { return 10; }
+int sweep_shape_count() { return kTileShapes + kRingShapes; }
 
 // TS runs its implicit sweeps z, y, x, the others x, y, z.
 int sweep_direction(int method, int sweep) { return method == 3 ? 2 - sweep : sweep; }
@@ -1208,16 +1183,63 @@ bool sweep_shape_fits(int shape, int d, int n) {
     MTS_SHAPES(MTS_FITS)
 #undef MTS_FITS
     default:
-      return false;
+      return n <= kMaxLineRows && ring_fits(shape - kTileShapes, n);
   }
 }
 
-// 32 lines per tile while shared memory holds them, else the most it holds.
-int sweep_shape_default(int d, int n) {
-  const int order[4] = {0, 3, 6, 8};
-  for (int s : order)
-    if (sweep_shape_fits(s, d, n)) return s;
-  return -1;
+// Lines that an SM solves at once with tiles of a shape (0: too long for it).
+template <int NL, int NT>
+int lines_at_once(int d, int n, bool adi_x) {
+  const size_t bytes = d == 0 ? tile_smem<0, NL>(n) : tile_smem<1, NL>(n);
+  if (n > kMaxLineRows || bytes > (size_t)kMaxTileSmem) return 0;
+  const int regs = adi_x ? line_min_ctas<K_ADI, NT>() : line_min_ctas<K_COPY, NT>();
+  return NL * (int)std::min<size_t>(regs, (228 * 1024) / (bytes + 1024 + sizeof(TileState<NL>)));
+}
+
+// The tile with the most lines on an SM at once, the narrower of two with as
+// many (more tiles overlap their loads).  32 lines up to 258 (x) and 243 rows
+// (y, z), then 16 lines, then 32 again where two 32-line tiles beat three
+// 16-line ones, and so on.  B200, us per sweep with 32 / 16 lines: LOD-CN x,
+// 241 rows 148 / 160, 289 rows 300 / 264, 385 rows 698 / 730, 449 rows 1928 /
+// 1157; Douglas-ADI y, 193 rows 84 / 92, 257 rows 226 / 197, 513 rows 2842 /
+// 2185.
+int tile_shape_default(int d, int n, bool adi_x) {
+  const int id[4] = {0, 3, 6, 8};
+  const int lines[4] = {lines_at_once<32, 256>(d, n, adi_x), lines_at_once<16, 256>(d, n, adi_x),
+                        lines_at_once<8, 128>(d, n, adi_x), lines_at_once<4, 128>(d, n, adi_x)};
+  int k = 0;
+  for (int i = 1; i < 4; i++)
+    if (lines[i] >= lines[k]) k = i;
+  return lines[k] > 0 ? id[k] : -1;
+}
+
+// Tiles or a ring (ring.cu).  A ring has as many lines on the chain as its CTA
+// has threads, whatever their length, but waits for global memory on every
+// step of it and fills an SM with few lines poorly: it pays where an SM has
+// much to do (w: nodes per SM) in long lines, or very many short ones.  The
+// lines lie where the two measured equal (B200, 53 grids of 17 to 1600 rows an
+// axis); us per sweep, tiles / ring:
+//   x, LOD-IE                 353^3 465 / 508, 385^3 727 / 620, 449^3 1139 / 955
+//   x, Douglas-ADI, with its first right-hand side (a pass of its own before a
+//   ring)                     321^3 500 / 553, 385^3 922 / 913, 449^3 1468 / 1414
+//   y, z                      ADI y 225^3 142 / 136, 257^3 197 / 190, 385^3 738 / 515;
+//                             LOD-IE y (copied) 249^3 142 / 155, 273^3 201 / 190
+//   z of LOD (adds the source on the way out, row by row in a ring)
+//                             LOD-CN 321^3 429 / 529, 353^3 652 / 593, 385^3 878 / 815
+//   33 x 700 x 700 x, TS      209 / 169; 500 x 33 x 500 y, ADI 115 / 98
+int sweep_shape_default(int method, int d, int n, long long lines, int sms) {
+  const double per_sm = (double)lines / sms, w = per_sm * n;
+  bool ring;
+  if (d == 0)
+    ring = (n >= 360 && w >= 110e3) || (method != MTS_ADI && n <= 50 && per_sm >= 1500);
+  else if (d == 2 && (method == MTS_LOD_IE || method == MTS_LOD_CN))
+    ring = (n >= 340 && w >= 180e3) || (n <= 50 && per_sm >= 1500);
+  else if (method == MTS_LOD_IE || (method == MTS_TS && d == 1))
+    ring = (n >= 150 && w >= 110e3) || (n <= 82 && per_sm >= 1000);
+  else
+    ring = (n >= 150 && w >= 100e3) || per_sm >= 1000;
+  const int k = ring ? ring_default(method, d, n, per_sm) : -1;
+  return k >= 0 && n <= kMaxLineRows ? kTileShapes + k : tile_shape_default(d, n, method == MTS_ADI && d == 0);
 }
 
 void configure_kernels() {
@@ -1277,7 +1299,8 @@ int launch_norms(const Dev& P, double E, const double* u, double* partial, int n
 }
 
 // One time step.  u0 holds u^n on entry and u^{n+1} on return; u1 is scratch.
-int launch_step(const Dev& P, const StepTimes& T, double* u0, double* u1, cudaStream_t st, cudaEvent_t* ev) {
+int launch_step(const Dev& P, const StepTimes& T, double* u0, double* u1, cudaStream_t st, cudaEvent_t* ev,
+                const SideStream* side) {
   int launches = 0;
   int slot = 0;
   auto mark = [&](int k) {
@@ -1296,11 +1319,28 @@ int launch_step(const Dev& P, const StepTimes& T, double* u0, double* u1, cudaSt
     // place (u**); the z sweep builds uh1 = -dt D_zz u^n + u** and writes
     // u^{n+1} over u^n in u0 (a z line reads only its own nodes of u^n).  The
     // faces get Outer_u(t_next) in u1 and in u0.  The state stays in u0, u1
-    // is scratch.
+    // is scratch.  Before an x ring sweep uhs is formed in u1 by passes of its
+    // own, the MIB rows on the side stream beside the others (they write
+    // disjoint nodes and read only u0).
+    const bool ring_x = P.shape[0] >= kTileShapes && P.rblk[0];
+    const bool fork = ring_x && side && side->stream && P.nmibnode > 0;
+    cudaStream_t sst = fork ? side->stream : st;
     mark(0);
+    if (fork) {
+      cudaEventRecord(side->fork, st);
+      cudaStreamWaitEvent(sst, side->fork, 0);
+    }
     if (P.nmibnode > 0) {
-      k_adi_mib<<<mib_nodes_grid(P), TPB, 0, st>>>(P, u0, u1, T.e_next);
+      k_adi_mib<<<mib_nodes_grid(P), TPB, 0, sst>>>(P, u0, u1, T.e_next);
       launches++;
+    }
+    if (ring_x) {
+      launch_adi_rhs(P, u0, u1, T.e_next, st);
+      launches++;
+    }
+    if (fork) {
+      cudaEventRecord(side->join, sst);
+      cudaStreamWaitEvent(st, side->join, 0);
     }
     mark(1);
     io.stin = u0;
@@ -1309,7 +1349,15 @@ int launch_step(const Dev& P, const StepTimes& T, double* u0, double* u1, cudaSt
     io.jumps = 0;
     io.bmode = 1;
     mark(0);
-    sweep<0, K_ADI>(P, io, P.shape[0], st);
+    if (ring_x) {
+      io.stin = u1;
+      io.add = u1;
+      io.bmode = 0;
+      sweep<0, K_COPY>(P, io, P.shape[0], st);
+      io.stin = u0;
+    } else {
+      sweep<0, K_ADI>(P, io, P.shape[0], st);
+    }
     mark(1);
     io.add = u1;
     io.bmode = 0;

@@ -96,8 +96,9 @@ def device_bytes_bound(spec: Spec, ncrossings: int, sms: int = 148, precision: s
     with `ncrossings` crossings (the layout of the library's allocations: two
     FP64 fields, the FP32 increment, the crossing lines' factors, the FP32
     ring sweeps' scratch and, for lines over 544 nodes, their per-node
-    factors, the tables and the MIB data), plus, for the mixed form, the
-    segmented solves' per-node coefficients (three FP32 values per node and
+    factors, the tables and the MIB data), plus, for plain problems whose
+    sweeps may take the rings (nodes or lines enough for every SM), those
+    sweeps' data, and for the mixed form, the segmented solves' per-node coefficients (three FP32 values per node and
     direction, built when the form is switched on)."""
     nx, ny, nz = spec.n
     N = nx * ny * nz
@@ -116,6 +117,9 @@ def device_bytes_bound(spec: Spec, ncrossings: int, sms: int = 148, precision: s
     b += 3 * 2 * 40 * nmax + 3 * 3 * 8 * nmax    # side tables, axis tables
     b += ncrossings * (432 + 3 * 4 + 88 + 3 * 24 + 4)  # blocks, block RHS, constants, MIB nodes, line list
     b += 4096 * 3 * 8 + 64 + 60 * 256            # norm partials, alignment
+    if (precision == "plain" or spec.method != "adi") and (N >= 100e3 * sms or maxlines >= 1000 * sms):
+        # the ring sweeps' per-node factors, block right-hand sides and d' scratch
+        b += 3 * 2 * 8 * (N + pad) + ncrossings * 24 + 64 + 8 * (nmax + 16) * sms * 448
     if precision == "mixed" and spec.method == "adi" and nmax <= 544:
         b += 3 * 3 * 4 * N                        # cib, cp, cq per direction
     return int(b * 1.02) + (1 << 20)

@@ -121,3 +121,53 @@ def test_a_sweep_takes_its_shape_by_its_own_axis(method, n):
                     with pytest.raises(M.MtsError, match="shared memory"):
                         s.set_sweep_shape(sweep, shape)
         assert all(fits(d, shape) for d, shape in zip(dirs, s.autotune(1)))
+
+
+def _ring_default(s):
+    """Whether the default shapes name a ring: its data comes with the first
+    plain step."""
+    before = s.device_bytes()
+    s.advance(1)
+    return s.device_bytes() > before
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("method", ["adi", "lod-ie", "lod-cn", "ts"])
+def test_rings_beside_tiles_give_the_oracle_bits(method):
+    """Each sweep on a ring of staged rows, the others on tiles: the first,
+    the second, the third; then all three."""
+    n = (45, 38, 51)
+    spec = M.Spec(n=n, method=method, mib=2, beta_out=37.5, dt=0.03, **ELL)
+    tags, cr, _ = M.setup_host(spec)
+    p = O.Problem(n=n, surface=spec.surface, surface_params=spec.surface_params, beta_in=spec.beta_in,
+                  beta_out=spec.beta_out, method=method, mib=2, dt=spec.dt)
+    u = O.port_init(p, tags)
+    want = O.port_run(p, tags, cr, u, steps=2)
+    for rings in ((0,), (1,), (2,), (0, 1, 2)):
+        for ring in (10, 11, 12):
+            with M.Solver(spec) as s:
+                for k in rings:
+                    s.set_sweep_shape(k, ring)
+                s.set_solution(u)
+                s.advance(2)
+                assert np.array_equal(s.solution(), want), (rings, ring)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("method", ["adi", "lod-ie", "lod-cn", "ts"])
+def test_grids_of_very_many_lines_take_rings_and_give_the_oracle_bits(method):
+    """389 x 18 x 397: 1043 y lines an SM on a B200, on rings by default."""
+    spec = M.Spec(n=(389, 18, 397), method=method, mib=1, beta_out=37.5, dt=0.01, setup="device", **ELL)
+    with M.Solver(spec) as s:
+        s.initialize()
+        assert _ring_default(s)
+        many = s.device_bytes()
+        s.autotune(1)
+        assert s.device_bytes() <= many + 16 * 3 * spec.nodes * 2  # what the kept shapes do not use is given back
+    with M.Solver(M.Spec(n=(33, 33, 33), method=method)) as s:
+        s.initialize()
+        assert not _ring_default(s)
+        held = s.device_bytes()
+        shapes = s.autotune(1)
+        assert max(shapes) >= 10 or s.device_bytes() == held
+    _check(spec, None, 2)

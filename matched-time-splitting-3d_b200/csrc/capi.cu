@@ -1123,18 +1123,17 @@ mts_status mts_batch_advance_steps(const mts_handle* hs, const int32_t* counts, 
       if (mts::mixed_batch_class(h->dev, d) < 0) return false;
     return true;
   };
-  // plain ones whose lines' tiles let an SM hold a few
-  auto plain_batchable = [&](const mts_problem* h) {
-    return mts::batch_lines_fit(std::max(h->g.nx, std::max(h->g.ny, h->g.nz)));
-  };
   auto solo = [&](int i) {
-    return fills_gpu(hs[i]) || (hs[i]->dev.precision != 0 ? !mixed_batchable(hs[i]) : !plain_batchable(hs[i]));
+    return fills_gpu(hs[i]) || (hs[i]->dev.precision != 0 ? !mixed_batchable(hs[i]) : mts::batch_class(hs[i]->dev) < 0);
   };
-  // plain handles by method: one batched launch sequence per group
-  for (int method = 0; method < 4; method++) {
+  // plain handles by method and class of line length: one batched launch
+  // sequence per group
+  for (int group = 0; group < 4 * mts::kBatchClasses; group++) {
+    const int method = group / mts::kBatchClasses, cls = group % mts::kBatchClasses;
     std::vector<int> mem;
     for (int i = 0; i < n; i++)
-      if (!solo(i) && hs[i]->dev.precision == 0 && hs[i]->prm.method == method) mem.push_back(i);
+      if (!solo(i) && hs[i]->dev.precision == 0 && hs[i]->prm.method == method && mts::batch_class(hs[i]->dev) == cls)
+        mem.push_back(i);
     if (mem.empty()) continue;
     cudaStream_t q = nullptr;
     BATCH_TRY(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
@@ -1150,10 +1149,15 @@ mts_status mts_batch_advance_steps(const mts_handle* hs, const int32_t* counts, 
     for (int k = 0; k < (int)mem.size(); k++) {
       const mts::Dev& d = hs[mem[(size_t)k]]->dev;
       recs.push_back(d);
-      plan.nmax = std::max(plan.nmax, std::max(d.nx, std::max(d.ny, d.nz)));
+      const int nd[3] = {d.nx, d.ny, d.nz};
+      for (int dd = 0; dd < 3; dd++) plan.nmax[dd] = std::max(plan.nmax[dd], nd[dd]);
       if (method == MTS_TS) add(rows, k, mts::ts_explicit_grid(d));
       if (method == MTS_ADI && d.nmibnode > 0) add(mib, k, mts::mib_grid(d));
-      for (int dd = 0; dd < 3; dd++) add(sw[dd], k, mts::batch_sweep_grid(d, dd));
+    }
+    for (int dd = 0; dd < 3; dd++) {
+      plan.tile[dd] = mts::batch_tile(dd, plan.nmax[dd]);
+      for (int k = 0; k < (int)mem.size(); k++)
+        add(sw[dd], k, mts::batch_sweep_grid(hs[mem[(size_t)k]]->dev, plan.tile[dd], dd));
     }
     void* tmp = nullptr;
     BATCH_TRY(dev_upload(recs.data(), recs.size() * sizeof(mts::Dev), q, &tmp));

@@ -245,7 +245,8 @@ struct BatchItem {
 struct BatchPlan {
   int method;         // MTS_ADI .. MTS_TS, shared by all problems
   int n;              // problems
-  int nmax;           // longest line over the problems
+  int tile[3];        // batch_tile of each direction
+  int nmax[3];        // longest line of each direction over the problems
   const Dev* Ps;      // [n] device records (tsched/tstep set)
   const BatchItem* rows;  // TS explicit half steps
   int nrows;
@@ -274,13 +275,15 @@ unsigned mixed_line_ctas(const Dev& P, int d);      // CTAs of the line solves o
 int launch_step_batch_mixed(const MixedBatchPlan& plan, cudaStream_t stream);  // one step + tick
 void configure_mixed_batch_kernels();
 int launch_batch_tick(const Dev* Ps, int n, cudaStream_t stream);
-bool batch_lines_fit(int nmax);            // the batched sweeps take lines of nmax nodes
+constexpr int kBatchClasses = 2;
+int batch_tile(int d, int n);              // tiles of the batched sweeps for direction-d lines of up to n nodes; -1: none
+int batch_class(const Dev& P);             // a class is launched together; -1: the problem steps by itself
 unsigned ts_explicit_grid(const Dev& P);
 void configure_batch_kernels();
 int launch_step_batch(const BatchPlan& plan, cudaStream_t stream);  // one step + tick
 unsigned mib_grid(const Dev& P);
 unsigned block_grid(const Dev& P, int d);
-unsigned batch_sweep_grid(const Dev& P, int d);
+unsigned batch_sweep_grid(const Dev& P, int tile, int d);
 
 // Shared by both step forms (kernels.cu).
 void launch_tick(const Dev& P, cudaStream_t stream);  // ++(*P.tstep)

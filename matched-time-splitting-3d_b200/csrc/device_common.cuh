@@ -14,8 +14,10 @@ constexpr int TPB = 128;                // pointwise kernels and small kernels
 constexpr int kMaxSweepSmem = 232448;  // 227 KB: the sm_100 per-CTA limit
 constexpr int kMaxTileSmem = kMaxSweepSmem - 1024;  // the line tiles keep a few words of static shared memory too
 constexpr int kMaxLineRows = 3245;     // the longest line the bit-exact form takes
-// The batched line tiles: three of them (and their problems' records) to an SM.
+// The batched line tiles, with their problem's record beside them in static
+// shared memory: three to an SM, and at all.
 constexpr int kBatchTileSmem = 70 * 1024;
+constexpr int kMaxBatchTileSmem = kMaxSweepSmem - 3 * 1024;
 
 // ---------------------------------------------------------------------------
 // Exact solutions (eq 0: src/equation/eq_0.cc; eq 8: see oracle/ref_harness.cc

@@ -1564,10 +1564,7 @@ __global__ void __launch_bounds__(TPB) kb_ts_explicit(const Dev* __restrict__ Ps
   k_ts_explicit_body<D>(P, w.cta, w.ncta, in ? P.u1 : P.u0, in ? P.u0 : P.u1, 0.0, 0.0);
 }
 
-// tiles of batches of small problems: many CTAs per SM
-constexpr int BNL = 32, BNT = 128;
-
-template <int D, int KIND>
+template <int D, int KIND, int BNL, int BNT>
 __global__ void __launch_bounds__(BNT, line_min_ctas<KIND, BNT>()) kb_line(const Dev* __restrict__ Ps,
                                                                            const BatchItem* __restrict__ items,
                                                                            Roles r) {
@@ -1583,23 +1580,55 @@ __global__ void kb_tick(const Dev* __restrict__ Ps, int n) {
   if (i < n && *Ps[i].tstep < Ps[i].tstop) ++*Ps[i].tstep;
 }
 
+// Lines per tile and threads per CTA of the batched sweeps (batch_tile).
+#define MTS_BATCH_TILES(X) X(0, 32, 128) X(1, 16, 256)
+
 template <int D, int KIND>
 void bsweep(const BatchPlan& b, const Roles& r, cudaStream_t st, int& launches) {
-  if (b.nsw[D] > 0) {
-    kb_line<D, KIND><<<b.nsw[D], BNT, tile_smem<D, BNL>(b.nmax), st>>>(b.Ps, b.sw[D], r);
-    launches++;
+  if (b.nsw[D] == 0) return;
+  switch (b.tile[D]) {
+#define MTS_CASE(id, nl, nt)                                                                            \
+  case id:                                                                                              \
+    kb_line<D, KIND, nl, nt><<<b.nsw[D], nt, tile_smem<D, nl>(b.nmax[D]), st>>>(b.Ps, b.sw[D], r);      \
+    break;
+    MTS_BATCH_TILES(MTS_CASE)
+#undef MTS_CASE
   }
+  launches++;
 }
 
 template <int D, int KIND>
 void bsweep_attr() {
-  cudaFuncSetAttribute(kb_line<D, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBatchTileSmem);
+#define MTS_ATTR(id, nl, nt) \
+  cudaFuncSetAttribute(kb_line<D, KIND, nl, nt>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBatchTileSmem);
+  MTS_BATCH_TILES(MTS_ATTR)
+#undef MTS_ATTR
 }
 
 }  // namespace
 
-bool batch_lines_fit(int nmax) {
-  return tile_smem<0, BNL>(nmax) <= (size_t)kBatchTileSmem && tile_smem<1, BNL>(nmax) <= (size_t)kBatchTileSmem;
+int batch_tile(int d, int n) {
+  auto fits = [&](size_t x, size_t yz, int limit) { return (d == 0 ? x : yz) <= (size_t)limit; };
+  if (fits(tile_smem<0, 32>(n), tile_smem<1, 32>(n), kBatchTileSmem)) return 0;
+  return fits(tile_smem<0, 16>(n), tile_smem<1, 16>(n), kMaxBatchTileSmem) ? 1 : -1;
+}
+
+// Problems whose lines all fit three 32-line tiles to an SM (232 rows) always
+// batch.  Of the others a solo step costs 14 to 19 us of launches, and the
+// batched tiles take about as long for 200 thousand nodes (100 thousand for
+// TS with long y or z lines, whose z sweep spills; 260 thousand for ADI and TS
+// with long x lines alone): the smaller ones batch, in launches of their own.
+// B200, us per step of 64 problems, solo / batched: 17 x 17 x 300 ADI 1018 /
+// 598, 300 x 17 x 17 TS 1227 / 609, 9 x 1500 x 9 LOD-CN 1646 / 1220, 780 x 17 x
+// 17 ADI 1753 / 1502; 33 x 33 x 240 TS 1306 / 1771, 25 x 25 x 500 ADI 1353 /
+// 1511, 780 x 17 x 17 LOD-CN 1291 / 1423.
+int batch_class(const Dev& P) {
+  const int t[3] = {batch_tile(0, P.nx), batch_tile(1, P.ny), batch_tile(2, P.nz)};
+  if (std::min(t[0], std::min(t[1], t[2])) < 0) return -1;
+  if (std::max(t[0], std::max(t[1], t[2])) == 0) return 0;
+  const bool yz = t[1] > 0 || t[2] > 0, lod = P.method == MTS_LOD_IE || P.method == MTS_LOD_CN;
+  const long long most = yz && P.method == MTS_TS ? 100000 : yz || lod ? 200000 : 260000;
+  return P.nn <= most ? 1 : -1;
 }
 
 int launch_batch_tick(const Dev* Ps, int n, cudaStream_t st) {
@@ -1610,9 +1639,10 @@ int launch_batch_tick(const Dev* Ps, int n, cudaStream_t st) {
 unsigned mib_grid(const Dev& P) { return mib_nodes_grid(P); }
 unsigned block_grid(const Dev& P, int d) { return (unsigned)((P.nblk[d] + TPB - 1) / TPB); }
 unsigned ts_explicit_grid(const Dev& P) { return pointwise_blocks(P) + mib_ctas(P); }
-unsigned batch_sweep_grid(const Dev& P, int d) {
+unsigned batch_sweep_grid(const Dev& P, int tile, int d) {
+  const int nl = tile == 0 ? 32 : 16;
   const bool faces = sweep_faces(P.method, d);
-  return d == 0 ? line_grid<0>(P, BNL, faces) : d == 1 ? line_grid<1>(P, BNL, faces) : line_grid<2>(P, BNL, faces);
+  return d == 0 ? line_grid<0>(P, nl, faces) : d == 1 ? line_grid<1>(P, nl, faces) : line_grid<2>(P, nl, faces);
 }
 
 void configure_batch_kernels() {

@@ -151,3 +151,32 @@ def test_mixed_problems_batch_in_their_own_group():
     finally:
         for s in solvers:
             s.close()
+
+
+@pytest.mark.parametrize("method", METHODS)
+def test_problems_with_long_lines_batch_together(method):
+    """Thin plain problems with a line of over 232 rows batch in launches of
+    their own (every member is charged the launches of the longest count), a
+    large one and one with a line too long for the batched tiles step by
+    themselves; all bit-identical to stepping each alone."""
+    grids = [(17, 18, 300), (300, 17, 17), (17, 260, 19), (9, 1300, 8), (33, 25, 17), (9, 8, 1600), (65, 65, 257)]
+    counts = [1, 5, 2, 3, 4, 2, 2]
+    ell = (0.6123, 0.4517, 0.3739, 1.0, 0.0713, -0.1127, 0.0391)
+    specs = [M.Spec(n=n, surface="ellipsoid", surface_params=ell, beta_out=37.5, method=method, mib=2, dt=0.02,
+                    setup="device") for n in grids]
+    solvers = [M.Solver(sp) for sp in specs]
+    try:
+        for s in solvers:
+            s.initialize()
+        before = [s.launch_count() for s in solvers]
+        M.batch_advance_steps(solvers, counts)
+        made = [s.launch_count() - b for s, b in zip(solvers, before)]
+        assert made[0] == made[1] == made[2] == made[3], made
+        assert made[5] < made[1] and made[6] < made[1], made
+        for sp, s, c in zip(specs, solvers, counts):
+            u, t = solve_alone(sp, "plain", c)
+            assert s.time == t
+            assert np.array_equal(s.solution(), u), (sp, c)
+    finally:
+        for s in solvers:
+            s.close()

@@ -22,7 +22,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIB_DIR, "libmts_b200.so")
 SOURCES = ["setup.cpp", "setup_gpu.cu", "kernels.cu", "ring.cu", "mixed.cu", "fast.cu", "diag.cu", "capi.cu"]
-HEADERS = ["setup.h", "device.h", "device_common.cuh"]
+HEADERS = ["setup.h", "device.h", "device_common.cuh", "device_once.h"]
 OBJ_DIR = os.path.join(HERE, "build")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 # device code of these sources may contract a*b+c into one fused multiply-add

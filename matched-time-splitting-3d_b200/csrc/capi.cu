@@ -15,6 +15,7 @@
 
 #include "../../include/mts.h"
 #include "device.h"
+#include "device_once.h"
 #include "setup.h"
 
 namespace {
@@ -273,6 +274,28 @@ cudaError_t ensure_side_stream(mts_problem* h) {
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->side.fork, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->side.join, cudaEventDisableTiming);
   return e;
+}
+
+// The kernels' shared-memory limits, set once per device before a group's
+// first launch there.
+struct Limits {
+  mts::DeviceOnce shape[mts::kTileShapes + mts::kRingShapes], batch[mts::kBatchTiles], mixed, mixed_batch, fast;
+};
+Limits g_limits;
+
+cudaError_t allow_shape(const mts_problem* h, int shape) {
+  return (cudaError_t)g_limits.shape[shape].run(h->device, [&] { return mts::configure_shape(shape); });
+}
+
+// What sweep k of a step may launch in this shape: its kernels, and for a
+// ring the tiles that take the sweep where its data cannot be built.
+cudaError_t allow_sweep(const mts_problem* h, int k, int shape) {
+  const mts::Dev& D = h->dev;
+  const cudaError_t e = allow_shape(h, shape);
+  if (e != cudaSuccess || shape < mts::kTileShapes) return e;
+  const int d = mts::sweep_direction(D.method, k);
+  return allow_shape(h, mts::tile_shape_default(d, d == 0 ? D.nx : d == 1 ? D.ny : D.nz,
+                                                D.method == MTS_ADI && d == 0));
 }
 
 // Gives back block i of the ring sweeps' data (a direction's, or 3: the d'
@@ -609,16 +632,6 @@ mts_status finish_create(mts_problem* h) {
   }
 
   keep_pool(h->device);
-  static bool configured = false;
-  if (!configured) {
-    mts::configure_kernels();
-    mts::configure_ring_kernels();
-    mts::configure_mixed_kernels();
-    mts::configure_batch_kernels();
-    mts::configure_fast_kernels();
-    mts::configure_mixed_batch_kernels();
-    configured = true;
-  }
   int sms = 0;
   CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device));
   D.sweep_blocks = sms > 0 ? sms : 1;
@@ -630,6 +643,7 @@ mts_status finish_create(mts_problem* h) {
     const int d = mts::sweep_direction(p.method, k);
     D.shape[k] = mts::sweep_shape_default(p.method, d, nd[d], line_count(g, d), D.sweep_blocks);
     if (D.shape[k] < 0) return fail(MTS_ERR_ARG, "grid lines too long for the sweep kernels' shared memory");
+    CUDA_TRY(allow_sweep(h, k, D.shape[k]));
   }
   CUDA_TRY(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
   // row slack of the fields that are staged past their last row: kRowPad rows
@@ -1155,7 +1169,8 @@ mts_status mts_batch_advance_steps(const mts_handle* hs, const int32_t* counts, 
       if (method == MTS_ADI && d.nmibnode > 0) add(mib, k, mts::mib_grid(d));
     }
     for (int dd = 0; dd < 3; dd++) {
-      plan.tile[dd] = mts::batch_tile(dd, plan.nmax[dd]);
+      const int tile = plan.tile[dd] = mts::batch_tile(dd, plan.nmax[dd]);
+      BATCH_TRY((cudaError_t)g_limits.batch[tile].run(hs[0]->device, [&] { return mts::configure_batch(tile); }));
       for (int k = 0; k < (int)mem.size(); k++)
         add(sw[dd], k, mts::batch_sweep_grid(hs[mem[(size_t)k]]->dev, plan.tile[dd], dd));
     }
@@ -1190,6 +1205,7 @@ mts_status mts_batch_advance_steps(const mts_handle* hs, const int32_t* counts, 
       cudaStream_t q = nullptr;
       BATCH_TRY(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
       streams.push_back(q);
+      BATCH_TRY((cudaError_t)g_limits.mixed_batch.run(hs[0]->device, mts::configure_mixed_batch_kernels));
       std::vector<mts::Dev> recs;
       mts::MixedBatchPlan plan{};
       plan.n = (int)mem.size();
@@ -1556,6 +1572,7 @@ mts_status mts_set_sweep_shape(mts_handle h, int32_t sweep, int32_t shape) {
   const int d = mts::sweep_direction(h->prm.method, sweep);
   if (!mts::sweep_shape_fits(shape, d, d == 0 ? h->g.nx : d == 1 ? h->g.ny : h->g.nz))
     return fail(MTS_ERR_ARG, "shape needs more shared memory than this grid allows");
+  CUDA_TRY(allow_sweep(h, sweep, shape));
   h->dev.shape[sweep] = shape;
   h->ring_refused = false;
   return MTS_OK;
@@ -1569,6 +1586,7 @@ mts_status mts_set_precision(mts_handle h, int32_t precision) {
     if (h->prm.method != MTS_ADI) return fail(MTS_ERR_ARG, "the fast FP64 form is built for Douglas-ADI only");
     if (!mts::fast_fits(h->g.nx, h->g.ny, h->g.nz))
       return fail(MTS_ERR_ARG, "grid lines too long for the fast FP64 form (at most 544 nodes per axis)");
+    CUDA_TRY((cudaError_t)g_limits.fast.run(h->device, mts::configure_fast_kernels));
     if (!h->fast_built) {
       // row tables, line flags, the crossing lines' coefficients, the block
       // rows' q, once per handle
@@ -1608,6 +1626,7 @@ mts_status mts_set_precision(mts_handle h, int32_t precision) {
     const int nmax = std::max(h->g.nx, std::max(h->g.ny, h->g.nz));
     if (!mts::mixed_shape_fits(nmax))
       return fail(MTS_ERR_ARG, "grid lines too long for the mixed-precision sweeps' shared memory");
+    CUDA_TRY((cudaError_t)g_limits.mixed.run(h->device, mts::configure_mixed_kernels));
     if (mts::mixed_segments_fit(nmax) && !h->mixed_built) {
       // the segmented solves' per-node coefficients, once per handle
       const size_t N = (size_t)h->g.nodes();
@@ -1669,6 +1688,7 @@ mts_status mts_autotune(mts_handle h, int32_t steps, int32_t shapes[3]) {
     for (int k = 0; k < 3; k++) {
       const int d = mts::sweep_direction(h->prm.method, k);
       fits[k] = mts::sweep_shape_fits(s, d, nd[d]);
+      if (fits[k]) CUDA_TRY(allow_sweep(h, k, s));
       h->dev.shape[k] = fits[k] ? s : choice0[k];
     }
     if (!fits[0] && !fits[1] && !fits[2]) continue;

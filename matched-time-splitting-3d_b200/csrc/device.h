@@ -184,12 +184,14 @@ int sweep_direction(int method, int sweep);       // direction of a step's first
 bool sweep_shape_fits(int shape, int d, int n);   // shared memory of the shape for direction-d lines of n nodes
 int sweep_shape_default(int method, int d, int n, long long lines, int sms);  // -1: no shape takes them
 int tile_shape_default(int d, int n, bool adi_x);  // among the tiles; adi_x: the x sweep of Douglas-ADI
-void configure_kernels();
+// Lets the kernels of a shape have its shared memory on the current device
+// (CUDA keeps the limit per device); the others below likewise.
+cudaError_t configure_shape(int shape);
 // The ring sweeps (ring.cu; ring: shape - kTileShapes).
 bool ring_fits(int ring, int n);
 int ring_default(int method, int d, int n, double per_sm);  // lines per SM; -1: none fits
 long long ring_threads(const Dev& P, int ring, int d);  // threads of the launch: columns of Dev::dp
-void configure_ring_kernels();
+cudaError_t configure_ring(int ring);
 void build_ring_factors(const Dev& P, int d, double* fbet, double* fgam, cudaStream_t stream);
 void launch_adi_rhs(const Dev& P, const double* u, double* r, double e_next, cudaStream_t stream);
 void launch_ring_sweep(const Dev& P, int d, int kind, const SweepIO& io, int ring, cudaStream_t stream);
@@ -218,7 +220,7 @@ int launch_step(const Dev& P, const StepTimes& T, double* u0, double* u1, cudaSt
 // The mixed-precision Douglas-ADI step (mixed.cu), in place on u.
 int launch_step_mixed(const Dev& P, const StepTimes& T, double* u, cudaStream_t stream, cudaEvent_t* ev,
                       const SideStream* side);
-void configure_mixed_kernels();
+cudaError_t configure_mixed_kernels();
 int mixed_sweep_threads();            // threads per CTA of the FP32 sweeps
 bool mixed_shape_fits(int nmax);      // their shared memory within the limit
 bool mixed_segments_fit(int n);       // the segmented solves take lines of n rows (else the ring sweeps run)
@@ -229,7 +231,7 @@ int build_mixed_coefs(const Dev& P, cudaStream_t stream);
 // the three launches.
 int launch_step_fast(const Dev& P, const StepTimes& T, double* u, double* d, cudaStream_t stream, cudaEvent_t* ev,
                      const SideStream* side);
-void configure_fast_kernels();
+cudaError_t configure_fast_kernels();
 int fast_rows_per_lane(int n);               // MX of a direction with n rows (0: lines too long)
 bool fast_fits(int nx, int ny, int nz);      // the form takes this grid
 int build_fast_lines(const Dev& P, uint8_t* const fline[3], cudaStream_t stream);  // the line flags
@@ -273,13 +275,13 @@ struct MixedBatchPlan {
 int mixed_batch_class(const Dev& P, int d);          // -1: not batchable
 unsigned mixed_line_ctas(const Dev& P, int d);      // CTAs of the line solves of direction d
 int launch_step_batch_mixed(const MixedBatchPlan& plan, cudaStream_t stream);  // one step + tick
-void configure_mixed_batch_kernels();
+cudaError_t configure_mixed_batch_kernels();
 int launch_batch_tick(const Dev* Ps, int n, cudaStream_t stream);
-constexpr int kBatchClasses = 2;
+constexpr int kBatchClasses = 2, kBatchTiles = 2;
 int batch_tile(int d, int n);              // tiles of the batched sweeps for direction-d lines of up to n nodes; -1: none
 int batch_class(const Dev& P);             // a class is launched together; -1: the problem steps by itself
 unsigned ts_explicit_grid(const Dev& P);
-void configure_batch_kernels();
+cudaError_t configure_batch(int tile);
 int launch_step_batch(const BatchPlan& plan, cudaStream_t stream);  // one step + tick
 unsigned mib_grid(const Dev& P);
 unsigned block_grid(const Dev& P, int d);

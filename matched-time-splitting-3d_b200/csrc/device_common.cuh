@@ -5,6 +5,8 @@
 
 #include <cuda_runtime.h>
 
+#include <initializer_list>
+
 #include "device.h"
 
 namespace mts {
@@ -36,6 +38,15 @@ __device__ __forceinline__ double source(const Dev& P, double E, int out, int ix
   if (P.eq == 0) return 0.0;
   if (out) return -outer_u(P, E, ix, iy, iz) - P.c6bo * E;
   return P.kin * inner_u(P, E, ix, iy, iz);
+}
+
+// Lets each kernel have `bytes` of dynamic shared memory on the current device.
+inline cudaError_t allow_smem(int bytes, std::initializer_list<const void*> kernels) {
+  for (const void* k : kernels) {
+    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
 }
 
 // CTAs of a persistent line sweep: one per SM at most, no more than nl lines

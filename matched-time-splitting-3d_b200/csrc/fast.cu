@@ -1166,23 +1166,25 @@ void launch_dir(const Dev& P, int d, bool crossing, const double* un, double* f,
 }
 
 template <int MX>
-void fast_attr() {
-  cudaFuncSetAttribute(kf_xw<8, MX>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSweepSmem);
-  cudaFuncSetAttribute(kf_xw<4, MX>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSweepSmem);
-  cudaFuncSetAttribute(kf_xc<MX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cross_smem<MX>());
-  cudaFuncSetAttribute(kf_yt<1, MX, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)yt_smem<MX, false>());
-  cudaFuncSetAttribute(kf_yt<2, MX, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)yt_smem<MX, true>());
-  cudaFuncSetAttribute(kf_yc<1, MX, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)yc_smem<MX, false>());
-  cudaFuncSetAttribute(kf_yc<2, MX, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)yc_smem<MX, true>());
+cudaError_t allow_fast() {
+  cudaError_t e = allow_smem(kMaxSweepSmem, {(const void*)kf_xw<8, MX>, (const void*)kf_xw<4, MX>});
+  if (e == cudaSuccess) e = allow_smem((int)cross_smem<MX>(), {(const void*)kf_xc<MX>});
+  if (e == cudaSuccess) e = allow_smem((int)yt_smem<MX, false>(), {(const void*)kf_yt<1, MX, false>});
+  if (e == cudaSuccess) e = allow_smem((int)yt_smem<MX, true>(), {(const void*)kf_yt<2, MX, true>});
+  if (e == cudaSuccess) e = allow_smem((int)yc_smem<MX, false>(), {(const void*)kf_yc<1, MX, false>});
+  if (e == cudaSuccess) e = allow_smem((int)yc_smem<MX, true>(), {(const void*)kf_yc<2, MX, true>});
+  return e;
 }
 
 }  // namespace
 
-void configure_fast_kernels() {
-#define MTS_ATTR(mx) fast_attr<mx>();
-  MTS_FAST_MX(MTS_ATTR)
-#undef MTS_ATTR
+cudaError_t configure_fast_kernels() {
+  cudaError_t e = cudaSuccess;
+#define MTS_ALLOW(mx) \
+  if (e == cudaSuccess) e = allow_fast<mx>();
+  MTS_FAST_MX(MTS_ALLOW)
+#undef MTS_ALLOW
+  return e;
 }
 
 int fast_rows_per_lane(int n) { return fast_mx(n); }

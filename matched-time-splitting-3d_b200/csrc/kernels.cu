@@ -1160,12 +1160,12 @@ void sweep(const Dev& P, const SweepIO& io, int shape, cudaStream_t st) {
   }
 }
 
-template <int D, int KIND>
-void set_smem_attr() {
-#define MTS_ATTR(id, nl, nt) \
-  cudaFuncSetAttribute(k_line<D, KIND, nl, nt>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxTileSmem);
-  MTS_SHAPES(MTS_ATTR)
-#undef MTS_ATTR
+template <int NL, int NT>
+cudaError_t allow_tiles() {
+  return allow_smem(kMaxTileSmem, {(const void*)k_line<0, K_COPY, NL, NT>, (const void*)k_line<1, K_COPY, NL, NT>,
+                                   (const void*)k_line<2, K_COPY, NL, NT>, (const void*)k_line<0, K_STENCIL, NL, NT>,
+                                   (const void*)k_line<1, K_STENCIL, NL, NT>, (const void*)k_line<2, K_STENCIL, NL, NT>,
+                                   (const void*)k_line<0, K_ADI, NL, NT>, (const void*)k_line<2, K_TS_Z, NL, NT>});
 }
 
 }  // namespace
@@ -1242,15 +1242,16 @@ int sweep_shape_default(int method, int d, int n, long long lines, int sms) {
   return k >= 0 && n <= kMaxLineRows ? kTileShapes + k : tile_shape_default(d, n, method == MTS_ADI && d == 0);
 }
 
-void configure_kernels() {
-  set_smem_attr<0, K_COPY>();
-  set_smem_attr<1, K_COPY>();
-  set_smem_attr<2, K_COPY>();
-  set_smem_attr<0, K_STENCIL>();
-  set_smem_attr<0, K_ADI>();
-  set_smem_attr<1, K_STENCIL>();
-  set_smem_attr<2, K_STENCIL>();
-  set_smem_attr<2, K_TS_Z>();
+cudaError_t configure_shape(int shape) {
+  switch (shape) {
+#define MTS_ALLOW(id, nl, nt) \
+  case id:                    \
+    return allow_tiles<nl, nt>();
+    MTS_SHAPES(MTS_ALLOW)
+#undef MTS_ALLOW
+    default:
+      return configure_ring(shape - kTileShapes);
+  }
 }
 
 __global__ void k_tick(int* step) { ++*step; }
@@ -1597,12 +1598,13 @@ void bsweep(const BatchPlan& b, const Roles& r, cudaStream_t st, int& launches) 
   launches++;
 }
 
-template <int D, int KIND>
-void bsweep_attr() {
-#define MTS_ATTR(id, nl, nt) \
-  cudaFuncSetAttribute(kb_line<D, KIND, nl, nt>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxBatchTileSmem);
-  MTS_BATCH_TILES(MTS_ATTR)
-#undef MTS_ATTR
+template <int NL, int NT>
+cudaError_t allow_batch_tiles() {
+  return allow_smem(kMaxBatchTileSmem,
+                    {(const void*)kb_line<0, K_COPY, NL, NT>, (const void*)kb_line<1, K_COPY, NL, NT>,
+                     (const void*)kb_line<2, K_COPY, NL, NT>, (const void*)kb_line<0, K_STENCIL, NL, NT>,
+                     (const void*)kb_line<1, K_STENCIL, NL, NT>, (const void*)kb_line<2, K_STENCIL, NL, NT>,
+                     (const void*)kb_line<0, K_ADI, NL, NT>, (const void*)kb_line<2, K_TS_Z, NL, NT>});
 }
 
 }  // namespace
@@ -1645,16 +1647,7 @@ unsigned batch_sweep_grid(const Dev& P, int tile, int d) {
   return d == 0 ? line_grid<0>(P, nl, faces) : d == 1 ? line_grid<1>(P, nl, faces) : line_grid<2>(P, nl, faces);
 }
 
-void configure_batch_kernels() {
-  bsweep_attr<0, K_COPY>();
-  bsweep_attr<1, K_COPY>();
-  bsweep_attr<2, K_COPY>();
-  bsweep_attr<0, K_STENCIL>();
-  bsweep_attr<0, K_ADI>();
-  bsweep_attr<1, K_STENCIL>();
-  bsweep_attr<2, K_STENCIL>();
-  bsweep_attr<2, K_TS_Z>();
-}
+cudaError_t configure_batch(int tile) { return tile == 0 ? allow_batch_tiles<32, 128>() : allow_batch_tiles<16, 256>(); }
 
 // One step of every problem of the plan, the launch sequence of launch_step.
 int launch_step_batch(const BatchPlan& b, cudaStream_t st) {

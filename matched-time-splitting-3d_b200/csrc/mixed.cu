@@ -934,26 +934,25 @@ void sweep32(const Dev& P, float* f, double* u, cudaStream_t st) {
 }  // namespace
 
 template <int MX>
-void allow_smem() {
-  cudaFuncSetAttribute(k_xline32<MX>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xline_smem<MX>());
-  cudaFuncSetAttribute(k_yzline32<1, MX, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)yzline_smem<MX, false>());
-  cudaFuncSetAttribute(k_yzline32<2, MX, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)yzline_smem<MX, false>());
-  cudaFuncSetAttribute(k_yzline32<2, MX, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)yzline_smem<MX, true>());
+cudaError_t allow_segments() {
+  cudaError_t e = allow_smem((int)xline_smem<MX>(), {(const void*)k_xline32<MX>});
+  if (e == cudaSuccess)
+    e = allow_smem((int)yzline_smem<MX, false>(),
+                   {(const void*)k_yzline32<1, MX, false>, (const void*)k_yzline32<2, MX, false>});
+  if (e == cudaSuccess) e = allow_smem((int)yzline_smem<MX, true>(), {(const void*)k_yzline32<2, MX, true>});
+  return e;
 }
 
-void configure_mixed_kernels() {
-  constexpr int smem = 232448;
-  cudaFuncSetAttribute(k_sweep32<0, S32_CH, S32_NS, S32_NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_sweep32<1, S32_CH, S32_NS, S32_NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaFuncSetAttribute(k_sweep32<2, S32_CH, S32_NS, S32_NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  allow_smem<3>();
-  allow_smem<5>();
-  allow_smem<9>();
-  allow_smem<13>();
-  allow_smem<17>();
+cudaError_t configure_mixed_kernels() {
+  cudaError_t e = allow_smem(232448, {(const void*)k_sweep32<0, S32_CH, S32_NS, S32_NT>,
+                                      (const void*)k_sweep32<1, S32_CH, S32_NS, S32_NT>,
+                                      (const void*)k_sweep32<2, S32_CH, S32_NS, S32_NT>});
+  if (e == cudaSuccess) e = allow_segments<3>();
+  if (e == cudaSuccess) e = allow_segments<5>();
+  if (e == cudaSuccess) e = allow_segments<9>();
+  if (e == cudaSuccess) e = allow_segments<13>();
+  if (e == cudaSuccess) e = allow_segments<17>();
+  return e;
 }
 
 int mixed_sweep_threads() { return S32_NT; }
@@ -989,17 +988,17 @@ unsigned mixed_line_ctas(const Dev& P, int d) {
   return (unsigned)(((d == 1 ? nlines<1>(P) : nlines<2>(P)) + nl - 1) / nl);
 }
 
-void configure_mixed_batch_kernels() {
-  cudaFuncSetAttribute(kbm_xline32<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xline_smem<3>());
-  cudaFuncSetAttribute(kbm_xline32<5>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xline_smem<5>());
-  cudaFuncSetAttribute(kbm_yzline32<1, 3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)yzline_smem<3, false>());
-  cudaFuncSetAttribute(kbm_yzline32<1, 5, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)yzline_smem<5, false>());
-  cudaFuncSetAttribute(kbm_yzline32<2, 3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)yzline_smem<3, true>());
-  cudaFuncSetAttribute(kbm_yzline32<2, 5, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)yzline_smem<5, true>());
+template <int MX>
+cudaError_t allow_batch_segments() {
+  cudaError_t e = allow_smem((int)xline_smem<MX>(), {(const void*)kbm_xline32<MX>});
+  if (e == cudaSuccess) e = allow_smem((int)yzline_smem<MX, false>(), {(const void*)kbm_yzline32<1, MX, false>});
+  if (e == cudaSuccess) e = allow_smem((int)yzline_smem<MX, true>(), {(const void*)kbm_yzline32<2, MX, true>});
+  return e;
+}
+
+cudaError_t configure_mixed_batch_kernels() {
+  const cudaError_t e = allow_batch_segments<3>();
+  return e != cudaSuccess ? e : allow_batch_segments<5>();
 }
 
 int launch_step_batch_mixed(const MixedBatchPlan& b, cudaStream_t st) {

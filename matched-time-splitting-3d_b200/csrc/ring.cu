@@ -664,13 +664,13 @@ void sweep(const Dev& P, const SweepIO& io, int ring, cudaStream_t st) {
   }
 }
 
-template <int D, int KIND>
-void set_smem_attr() {
-#define MTS_ATTR(id, ch, ns, nt)                                                                    \
-  cudaFuncSetAttribute(k_sweep<D, KIND, ch, ns, nt>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                       kMaxSweepSmem);
-  MTS_RINGS(MTS_ATTR)
-#undef MTS_ATTR
+template <int CH, int NS, int NT>
+cudaError_t allow_rings() {
+  return allow_smem(kMaxSweepSmem,
+                    {(const void*)k_sweep<0, K_COPY, CH, NS, NT>, (const void*)k_sweep<1, K_COPY, CH, NS, NT>,
+                     (const void*)k_sweep<2, K_COPY, CH, NS, NT>, (const void*)k_sweep<0, K_STENCIL, CH, NS, NT>,
+                     (const void*)k_sweep<1, K_STENCIL, CH, NS, NT>, (const void*)k_sweep<2, K_STENCIL, CH, NS, NT>,
+                     (const void*)k_sweep<2, K_TS_Z, CH, NS, NT>});
 }
 
 }  // namespace
@@ -710,14 +710,16 @@ long long ring_threads(const Dev& P, int ring, int d) {
   return (long long)nt * sweep_grid(P, d == 0 ? nlines<0>(P) : d == 1 ? nlines<1>(P) : nlines<2>(P), nt);
 }
 
-void configure_ring_kernels() {
-  set_smem_attr<0, K_COPY>();
-  set_smem_attr<1, K_COPY>();
-  set_smem_attr<2, K_COPY>();
-  set_smem_attr<0, K_STENCIL>();
-  set_smem_attr<1, K_STENCIL>();
-  set_smem_attr<2, K_STENCIL>();
-  set_smem_attr<2, K_TS_Z>();
+cudaError_t configure_ring(int ring) {
+  switch (ring) {
+#define MTS_ALLOW(id, ch, ns, nt) \
+  case id:                        \
+    return allow_rings<ch, ns, nt>();
+    MTS_RINGS(MTS_ALLOW)
+#undef MTS_ALLOW
+    default:
+      return cudaErrorInvalidValue;
+  }
 }
 
 void build_ring_factors(const Dev& P, int d, double* fbet, double* fgam, cudaStream_t st) {

@@ -576,29 +576,49 @@ mts_status finish_create(mts_problem* h) {
         }
     }
   }
-  // the lines that cross the interface, in memory order (the fast line index
-  // first), and each line's index in that list
-  std::vector<int32_t> clist[3], cline[3], lperm[3];
+  // the interior lines in the order of the bit-exact sweeps (crossing the
+  // interface, inside, outside; each in memory order, the fast line index
+  // first), the crossing ones among them, and each line's index there
+  // (all of them in one array, which goes up in one copy)
+  std::vector<int32_t> lines;
+  size_t lperm[3], cline[3], clist[3];  // where each begins
+  int ncross[3];
   for (int d = 0; d < 3; d++) {
     const int n1 = d == 0 ? g.ny : g.nx, n2 = d == 2 ? g.ny : g.nz;
-    // (the order of the bit-exact sweeps: crossing, inside, outside)
-    lperm[d].reserve((size_t)(n1 - 2) * (n2 - 2));
-    for (int kind = 0; kind < 3; kind++)
-      for (int i2 = 1; i2 < n2 - 1; i2++)
-        for (int i1 = 1; i1 < n1 - 1; i1++) {
-          const size_t l = (size_t)i1 * n2 + i2;
-          const int kd = bstart[d][l + 1] > bstart[d][l] ? 0 : 1 + ((lside[d][l] >> 1) & 1);
-          if (kd == kind) lperm[d].push_back(i1 + n1 * i2);
+    // a line's kind by its place in memory, turned over in squares that stay
+    // in the cache
+    std::vector<uint8_t> kind((size_t)n1 * n2);
+    size_t at[4] = {0, 0, 0, 0};
+    for (int b1 = 1; b1 < n1 - 1; b1 += 32)
+      for (int b2 = 1; b2 < n2 - 1; b2 += 32)
+        for (int i1 = b1; i1 < std::min(b1 + 32, n1 - 1); i1++)
+          for (int i2 = b2; i2 < std::min(b2 + 32, n2 - 1); i2++) {
+            const size_t l = (size_t)i1 * n2 + i2;
+            const int k = bstart[d][l + 1] > bstart[d][l] ? 0 : 1 + ((lside[d][l] >> 1) & 1);
+            kind[i1 + (size_t)n1 * i2] = (uint8_t)k;
+            at[k + 1]++;
+          }
+    const size_t nc = at[1];
+    at[2] += at[1];
+    ncross[d] = (int)nc;
+    auto part = [&](size_t n, int32_t fill) {
+      const size_t begin = lines.size();
+      lines.resize(begin + (n + kAlign / 4 - 1) / (kAlign / 4) * (kAlign / 4), fill);
+      return begin;
+    };
+    lperm[d] = part((size_t)(n1 - 2) * (n2 - 2), 0);
+    clist[d] = part(nc, 0);
+    cline[d] = part(nc ? (size_t)n1 * n2 : 0, -1);
+    int32_t *const perm = lines.data() + lperm[d], *const list = lines.data() + clist[d],
+                  *const index = lines.data() + cline[d];
+    for (int i2 = 1; i2 < n2 - 1; i2++)
+      for (int i1 = 1; i1 < n1 - 1; i1++) {
+        const int m = i1 + n1 * i2, k = kind[(size_t)m];
+        if (k == 0) {
+          index[m] = (int32_t)at[0];
+          list[at[0]] = i1 * n2 + i2;
         }
-    if (blocks[d].empty()) continue;
-    cline[d].assign((size_t)line_count(g, d), -1);
-    for (int i2 = 0; i2 < n2; i2++)
-      for (int i1 = 0; i1 < n1; i1++) {
-        const size_t l = (size_t)i1 * n2 + i2;
-        if (bstart[d][l + 1] > bstart[d][l]) {
-          cline[d][(size_t)i1 + (size_t)n1 * i2] = (int32_t)clist[d].size();
-          clist[d].push_back((int32_t)l);
-        }
+        perm[at[k]++] = m;
       }
   }
   for (size_t i = 0; i < h->cross.size(); i++) {
@@ -657,7 +677,30 @@ mts_status finish_create(mts_problem* h) {
   h->norm_nb = mts::norms_blocks(D);
   // Every buffer of the handle, placed twice: first only to add up their
   // sizes, then into the one pool block of that size.
+  // The small tables go up in one copy: the sizing pass collects them, the
+  // placing pass points into the copy.
+  std::vector<char> blob;
+  std::vector<size_t> piece;
+  size_t next_piece = 0;
+  char* blob_d = nullptr;
+  auto put_small = [&](auto** dst, const auto& src) -> cudaError_t {
+    using T = std::remove_pointer_t<std::remove_pointer_t<decltype(dst)>>;
+    const size_t bytes = src.size() * sizeof(T);
+    if (bytes == 0 || bytes > 32768) return h->put(dst, (const T*)src.data(), src.size());
+    if (h->sizing) {
+      piece.push_back(blob.size());
+      blob.insert(blob.end(), (const char*)src.data(), (const char*)src.data() + bytes);
+      blob.resize((blob.size() + kAlign - 1) / kAlign * kAlign);
+      *dst = nullptr;
+    } else {
+      *dst = (T*)(blob_d + piece[next_piece++]);
+    }
+    return cudaSuccess;
+  };
   auto place_all = [&]() -> mts_status {
+    if (!h->sizing) CUDA_TRY(h->put(&blob_d, blob.data(), blob.size()));
+    int32_t* dlines = nullptr;
+    CUDA_TRY(h->put(&dlines, lines.data(), lines.size()));
     CUDA_TRY(h->put_padded(&h->u0, (const double*)nullptr, (size_t)N, fpad));
     CUDA_TRY(h->put_padded(&h->u1, (const double*)nullptr, (size_t)N, fpad));
     D.u0 = h->u0;
@@ -666,10 +709,10 @@ mts_status finish_create(mts_problem* h) {
       for (int side = 0; side < 2; side++) {
         double2* pt = nullptr;
         double *pa = nullptr, *pg = nullptr;
-        CUDA_TRY(h->put(&pa, taba[d][side].data(), taba[d][side].size()));
+        CUDA_TRY(put_small(&pa, taba[d][side]));
         D.taba[d][side] = pa;
-        CUDA_TRY(h->put(&pt, tab[d][side].data(), tab[d][side].size()));
-        CUDA_TRY(h->put(&pg, tabg[d][side].data(), tabg[d][side].size()));
+        CUDA_TRY(put_small(&pt, tab[d][side]));
+        CUDA_TRY(put_small(&pg, tabg[d][side]));
         D.tab[d][side] = pt;
         D.tabg[d][side] = pg;
       }
@@ -678,16 +721,14 @@ mts_status finish_create(mts_problem* h) {
       // form's ring sweeps 1/bet and gam per node in FP32 too
       float *fb32 = nullptr, *fg32 = nullptr;
       if (!blocks[d].empty()) {
-        int32_t *dl = nullptr, *dc = nullptr;
         double *ca = nullptr, *cg = nullptr;
         double2* cb = nullptr;
-        CUDA_TRY(h->put(&dl, clist[d].data(), clist[d].size()));
-        CUDA_TRY(h->put(&dc, cline[d].data(), cline[d].size()));
-        CUDA_TRY(h->put(&ca, (const double*)nullptr, clist[d].size() * (size_t)nd[d]));
-        CUDA_TRY(h->put(&cb, (const double2*)nullptr, clist[d].size() * (size_t)nd[d]));
-        CUDA_TRY(h->put(&cg, (const double*)nullptr, clist[d].size() * (size_t)nd[d]));
-        D.fcross[d] = dl;
-        D.cline[d] = dc;
+        const size_t rows = (size_t)ncross[d] * (size_t)nd[d];
+        CUDA_TRY(h->put(&ca, (const double*)nullptr, rows));
+        CUDA_TRY(h->put(&cb, (const double2*)nullptr, rows));
+        CUDA_TRY(h->put(&cg, (const double*)nullptr, rows));
+        D.fcross[d] = dlines + clist[d];
+        D.cline[d] = dlines + cline[d];
         D.ca[d] = ca;
         D.cb[d] = cb;
         D.cg[d] = cg;
@@ -696,7 +737,7 @@ mts_status finish_create(mts_problem* h) {
           CUDA_TRY(h->put_padded(&fg32, (const float*)nullptr, (size_t)N, fpad));
         }
       }
-      D.nfcross[d] = (int)clist[d].size();
+      D.nfcross[d] = ncross[d];
       D.fib32[d] = fb32;
       D.fgam32[d] = fg32;
       // the same factors in FP32 for the mixed-precision sweeps, as 1/bet and gam
@@ -707,7 +748,7 @@ mts_status finish_create(mts_problem* h) {
           p32[2 * j + 1] = (float)(j ? tabg[d][side][j - 1] : 0.0);
         }
         float* pt = nullptr;
-        CUDA_TRY(h->put(&pt, p32.data(), p32.size()));
+        CUDA_TRY(put_small(&pt, p32));
         D.ptab32[d][side] = pt;
       }
       float* rb32 = nullptr;
@@ -728,7 +769,7 @@ mts_status finish_create(mts_problem* h) {
     D.tag = dtag;
     {
       long long* dm = nullptr;
-      CUDA_TRY(h->put(&dm, mibn.empty() ? nullptr : mibn.data(), mibn.size()));
+      CUDA_TRY(put_small(&dm, mibn));
       D.mibnode = dm;
       D.nmibnode = (int)mibn.size();
       int4* ref = nullptr;
@@ -737,29 +778,27 @@ mts_status finish_create(mts_problem* h) {
     }
     for (int d = 0; d < 3; d++) {
       uint8_t* ls = nullptr;
-      CUDA_TRY(h->put(&ls, lside[d].data(), lside[d].size()));
+      CUDA_TRY(put_small(&ls, lside[d]));
       D.lside[d] = ls;
-      int32_t* lp = nullptr;
-      CUDA_TRY(h->put(&lp, lperm[d].data(), lperm[d].size()));
-      D.lperm[d] = lp;
+      D.lperm[d] = dlines + lperm[d];
     }
     for (int d = 0; d < 3; d++) {
       double *a = nullptr, *s = nullptr, *c = nullptr;
-      CUDA_TRY(h->put(&a, axv[d].data(), axv[d].size()));
-      CUDA_TRY(h->put(&s, s2v[d].data(), s2v[d].size()));
-      CUDA_TRY(h->put(&c, c2v[d].data(), c2v[d].size()));
+      CUDA_TRY(put_small(&a, axv[d]));
+      CUDA_TRY(put_small(&s, s2v[d]));
+      CUDA_TRY(put_small(&c, c2v[d]));
       D.ax[d] = a;
       D.s2[d] = s;
       D.c2[d] = c;
       int32_t* bs = nullptr;
       mts::MibBlock* bl = nullptr;
-      CUDA_TRY(h->put(&bs, bstart[d].data(), bstart[d].size()));
-      CUDA_TRY(h->put(&bl, blocks[d].empty() ? nullptr : blocks[d].data(), blocks[d].size()));
+      CUDA_TRY(put_small(&bs, bstart[d]));
+      CUDA_TRY(put_small(&bl, blocks[d]));
       D.bstart[d] = bs;
       D.blk[d] = bl;
     }
     mts::CrossConst* dcc = nullptr;
-    CUDA_TRY(h->put(&dcc, cc.empty() ? nullptr : cc.data(), cc.size()));
+    CUDA_TRY(put_small(&dcc, cc));
     D.cc = dcc;
     CUDA_TRY(h->put(&D.status, (const int*)nullptr, 1));
     CUDA_TRY(h->put(&h->norm_part, (const double*)nullptr, (size_t)3 * h->norm_nb));
@@ -771,7 +810,7 @@ mts_status finish_create(mts_problem* h) {
   mts_status placed = place_all();
   h->sizing = false;
   if (placed) return placed;
-  CUDA_TRY(h->reserve(h->planned));
+  CUDA_TRY(h->reserve(h->planned + std::max(blob.size(), (size_t)kAlign)));
   placed = place_all();
   if (placed) return placed;
   CUDA_TRY(cudaMemsetAsync(D.status, 0, sizeof(int), h->stream));

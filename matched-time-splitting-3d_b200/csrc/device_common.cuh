@@ -15,7 +15,10 @@ namespace {
 constexpr int TPB = 128;                // pointwise kernels and small kernels
 constexpr int kMaxSweepSmem = 232448;  // 227 KB: the sm_100 per-CTA limit
 constexpr int kMaxTileSmem = kMaxSweepSmem - 1024;  // the line tiles keep a few words of static shared memory too
-constexpr int kMaxLineRows = 3245;     // the longest line the bit-exact form takes
+// The longest line the bit-exact form takes: what its smallest ring holds (3 x
+// 16 rows of 132 doubles and 7 doubles a row of the line in 227 KB; 4-line
+// tiles hold 3616).
+constexpr int kMaxLineRows = 3245;
 // The batched line tiles, with their problem's record beside them in static
 // shared memory: three to an SM, and at all.
 constexpr int kBatchTileSmem = 70 * 1024;
@@ -351,18 +354,18 @@ __device__ __forceinline__ MibDir mib_direction(const Dev& P, const double* __re
   return r;
 }
 
-// The listed MIB nodes k0 <= k < k1, shared out over nw warps (this one is
-// w): three lanes a node, one per direction.  done(m, ix, iy, iz, sx, sy,
+// The listed MIB nodes, shared out over nw warps (this one is w): three lanes
+// a node, one per direction.  done(m, ix, iy, iz, sx, sy,
 // sz, src) gets a node's three sums and its source with the jump terms.
 template <class F>
-__device__ __forceinline__ void mib_nodes(const Dev& P, const double* __restrict__ un, double E, int k0, int k1, int w,
-                                          int nw, F done) {
+__device__ __forceinline__ void mib_nodes(const Dev& P, const double* __restrict__ un, double E, int w, int nw,
+                                          F done) {
   constexpr unsigned ALL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int d = lane % 3, g = lane / 3;
-  for (int kb = k0 + 10 * w; kb < k1; kb += 10 * nw) {
+  for (int kb = 10 * w; kb < P.nmibnode; kb += 10 * nw) {
     const int k = kb + g;
-    const bool act = g < 10 && k < k1;
+    const bool act = g < 10 && k < P.nmibnode;
     MibDir r{0.0, 0.0, 0.0, 0};
     long long m = 0;
     int side = 0;

@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(TPB) kf_mib(const __grid_constant__ Dev P, con
                                               double* __restrict__ d, double E) {
   // every MIB row at once, three lanes each (the rows of an x block too:
   // kf_xc applies their block's row operations when it solves the line)
-  mib_nodes(P, un, step_e(P, E, 2), 0, P.nmibnode, blockIdx.x * (TPB / 32) + (threadIdx.x >> 5), gridDim.x * (TPB / 32),
+  mib_nodes(P, un, step_e(P, E, 2), blockIdx.x * (TPB / 32) + (threadIdx.x >> 5), gridDim.x * (TPB / 32),
             [&](long long m, int, int, int, double sx, double sy, double sz, double src) {
               d[m] = P.dt * (((sx + sy) + sz) + src);
             });

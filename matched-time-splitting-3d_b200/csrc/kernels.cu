@@ -41,7 +41,7 @@ namespace {
 __device__ __forceinline__ void k_adi_mib_body(const Dev& P, unsigned cta_, unsigned ncta_,
                                                const double* __restrict__ un, double* __restrict__ R, double E) {
   const double dt = P.dt;
-  mib_nodes(P, un, step_e(P, E, 2), 0, P.nmibnode, cta_ * (TPB / 32) + (threadIdx.x >> 5), ncta_ * (TPB / 32),
+  mib_nodes(P, un, step_e(P, E, 2), cta_ * (TPB / 32) + (threadIdx.x >> 5), ncta_ * (TPB / 32),
             [&](long long m, int, int, int, double, double sy, double sz, double src) {
               double r = sy * dt + sz * dt;
               r += un[m];
@@ -172,15 +172,16 @@ __global__ void __launch_bounds__(TPB) k_ts_explicit(const __grid_constant__ Dev
 // What bounds it: the recurrence is one dependent chain a row, so a tile
 // costs its line's length whatever its width (one warp, B200: 88 clocks a row
 // forward and back, 130 with the lines' own factors), and an SM solves as many
-// lines at once as its shared memory holds (32 lines of 257 rows take 68 KB:
-// 3 tiles); the other tiles' loads and stores overlap the chains.  Up to 4
-// tiles an SM (129^3) the step is one tile's latency; at 257^3 the loads are
-// the longer part, held to about 3.9 TB/s by the small L1 that the tiles
-// leave (a plain tile copy: 5.9 TB/s with 1 KB of shared memory per CTA, 3.9
-// with 36 KB or more).  Against one line per thread over a ring of staged
-// rows with the partial solutions in a global scratch (the form before), us
-// per step: 65^3 Douglas-ADI 158 -> 54, 129^3 LOD-CN 277 -> 84, 113 x 97 x
-// 141 TS 252 -> 99 (92 with the half steps' rows), 257^3 Douglas-ADI 688 -> 680.
+// lines at once as its shared memory holds (32 lines of 257 rows take 72 KB
+// for x, three tiles, and 76 KB for y and z, two); the other tiles' loads and
+// stores overlap the chains.  Up to 4 tiles an SM (129^3) a sweep is one
+// tile's latency; with many more the loads are the longer part, held to about
+// 3.9 TB/s by the small L1 that the tiles leave (a plain tile copy: 5.9 TB/s
+// with 1 KB of shared memory per CTA, 3.9 with 36 KB or more).  Against one
+// line per thread over a ring of staged rows with the partial solutions in a
+// global scratch (ring.cu, which takes the sweeps of many long lines), us per
+// step: 65^3 Douglas-ADI 138 -> 55, 129^3 LOD-CN 256 -> 81, 193^3 LOD-CN 655 ->
+// 241, 225^3 Douglas-ADI 513 -> 463.
 
 // Lines per tile and threads per CTA of each shape (mts_set_sweep_shape).
 #define MTS_SHAPES(X)                                                                           \
@@ -193,8 +194,12 @@ template <int D, int NL>
 __host__ __device__ constexpr int tile_row() { return D == 0 ? NL + 1 : NL; }
 // Rows of a chunk of the lines' own factors while a tile is solved: 8, or 4
 // for x lines, where the smaller buffers let an SM hold three 257-row tiles
-// (257^3: x 229 against 244 us; y and z, whose loads gain from the L1 that two
-// tiles leave, 195 and 213 against 196 and 233).
+// (us with 4 / 8: 257^3 Douglas-ADI x 227 / 240, LOD-IE x 176 / 184, 400 x 129
+// x 129 LOD-IE x 83 / 91; LOD-CN x, whose tiles hold more registers, 225^3 121
+// / 111).  For y and z 8 rows are better at 129 (25 / 27, LOD-IE y), 193 (87 /
+// 92, Douglas-ADI y) and from 257 rows on (LOD-IE z 224 / 210), and 4 where
+// they make room for one more tile, at 161 (48 / 59, Douglas-ADI y) and 225
+// rows (120 / 153).
 template <int D>
 __host__ __device__ constexpr int own_rows() { return D == 0 ? 4 : 8; }
 // Bytes for the factors: those of a side ((bet, 1/bet), gam by row), or two
@@ -286,7 +291,12 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
 // That holds while nothing over- or underflows on the way: |b| in [2^-100,
 // 2^100] (checked where the factors are made, Dev::plain_div) and |q| in
 // [2^-800, 2^800].  A tile with a quotient outside that (zeros, infinities
-// and NaN among them) is built and solved again with the divide.
+// and NaN among them) is built and solved again with the divide: a field that
+// is zero throughout, boundary data and source included, costs 129^3
+// Douglas-ADI 298 against 97 us a step, 257^3 1282 against 623 (rings alone:
+// 386 and 932).  Between boundary values of order one zeros do not last a row.
+// (Letting +0 by a positive factor pass takes the numerator's bits too: 102
+// against 97 us at 129^3 on ordinary fields.)
 // One warp alone (B200): 52 clocks a row of the recurrence against 125 with
 // the divide, whose own reciprocal and tests are on the chain.
 constexpr unsigned kQLo = (1023u - 800u) << 21, kQRange = 1600u << 21;
@@ -540,7 +550,7 @@ struct TileState {
 
 // The MIB rows' right-hand sides (the warps from BW on).
 template <int D, int KIND, int NL, int NT>
-__device__ __forceinline__ void tile_blocks(const Dev& P, const SweepIO& io, const TileState<NL>& T, double* sm, int t0,
+__device__ __forceinline__ void tile_blocks(const Dev& P, const SweepIO& io, const TileState<NL>& T, double* sm,
                                          int nlive) {
   constexpr int RS = tile_row<D, NL>(), NW = NT / 32, BW = NW / 2;
   const int tid = threadIdx.x, w = tid >> 5;
@@ -786,7 +796,7 @@ __device__ __forceinline__ void tile_rows(const Dev& P, const SweepIO& io, TileS
 
 // A tile from its fields to its solution in shared memory.
 template <int D, int KIND, int NL, int NT, bool PLAIN>
-__device__ __forceinline__ void tile_solution(const Dev& P, const SweepIO& io, TileState<NL>& T, double* sm_, int t0,
+__device__ __forceinline__ void tile_solution(const Dev& P, const SweepIO& io, TileState<NL>& T, double* sm_,
                                               int nlive) {
   constexpr int RS = tile_row<D, NL>();
   constexpr int NW = NT / 32;
@@ -813,7 +823,7 @@ __device__ __forceinline__ void tile_solution(const Dev& P, const SweepIO& io, T
     }
   }
   // ---- load
-  if (w >= BW) tile_blocks<D, KIND, NL, NT>(P, io, T, sm, t0, nlive);
+  if (w >= BW) tile_blocks<D, KIND, NL, NT>(P, io, T, sm, nlive);
   tile_rows<D, KIND, NL, NT>(P, io, T, sm, nlive);
   if (w == 0) {
     cp_async_commit();
@@ -856,9 +866,9 @@ __device__ __forceinline__ void tile_solution(const Dev& P, const SweepIO& io, T
 
 // The same with the divide, out of line (rare).
 template <int D, int KIND, int NL, int NT>
-__device__ __noinline__ void tile_solution_plain(const Dev& P, const SweepIO& io, TileState<NL>& T, double* sm_, int t0,
+__device__ __noinline__ void tile_solution_plain(const Dev& P, const SweepIO& io, TileState<NL>& T, double* sm_,
                                                  int nlive) {
-  tile_solution<D, KIND, NL, NT, true>(P, io, T, sm_, t0, nlive);
+  tile_solution<D, KIND, NL, NT, true>(P, io, T, sm_, nlive);
 }
 
 template <int D, int KIND, int NL, int NT>
@@ -891,12 +901,12 @@ __device__ __forceinline__ void k_line_body(const Dev& P, unsigned cta_, unsigne
     T.again = P.plain_div;
   }
   __syncthreads();
-  if (!P.plain_div) tile_solution<D, KIND, NL, NT, false>(P, io, T, sm_, t0, nlive);
+  if (!P.plain_div) tile_solution<D, KIND, NL, NT, false>(P, io, T, sm_, nlive);
   if (T.again) {
     __syncthreads();
     if (tid == 0) T.next_task = 0;
     __syncthreads();
-    tile_solution_plain<D, KIND, NL, NT>(P, io, T, sm_, t0, nlive);
+    tile_solution_plain<D, KIND, NL, NT>(P, io, T, sm_, nlive);
   }
 
   // ---- store
@@ -940,10 +950,13 @@ unsigned line_grid(const Dev& P, int nl, bool faces) {
   return (unsigned)(tiles + (faces ? (fn + 4095) / 4096 : 0));
 }
 
-// CTAs per SM that the registers should allow: four of 256 threads (a 129^3
-// grid's 504 tiles are then all on the chip at once: LOD-CN step 82 against 96
-// us), three for the first right-hand side, which holds more (x sweep of 257^3
-// 229 against 301 us).
+// CTAs per SM that the registers should allow: four of 256 threads, three for
+// the first right-hand side, which holds more.  It pays where the shared memory
+// allows as many, and costs spills where it does not (us with this rule / with
+// one CTA less: LOD-CN x, y, z 129^3 27, 27, 33 / 31, 31, 40, 161^3 43, 47, 58
+// / 46, 46, 58, 241^3 151, 155, 201 / 133, 148, 199; Douglas-ADI x 129^3 39 /
+// 37, 193^3 87 / 111, 257^3 227 / 235, 353^3 690 / 645; 16-line tiles, LOD-IE z
+// 289^3 298 / 350).
 template <int KIND, int NT>
 constexpr int line_min_ctas() { return NT == 256 ? (KIND == K_ADI ? 3 : 4) : NT == 192 ? 4 : NT == 128 ? 5 : 6; }
 

@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(TPB, 8) k_adi_resid(const __grid_constant__ De
 // jumps) and the jump terms of Src_2nd (douglas_adi.cc:1156-1427).
 __device__ __forceinline__ void adi_resid_mib_body(const Dev& P, unsigned cta_, unsigned ncta_,
                                                    const double* __restrict__ un, float* __restrict__ rho, double E) {
-  mib_nodes(P, un, step_e(P, E, 2), 0, P.nmibnode, cta_ * (TPB / 32) + (threadIdx.x >> 5), ncta_ * (TPB / 32),
+  mib_nodes(P, un, step_e(P, E, 2), cta_ * (TPB / 32) + (threadIdx.x >> 5), ncta_ * (TPB / 32),
             [&](long long m, int, int, int, double sx, double sy, double sz, double src) {
               rho[m] = (float)(P.dt * (((sx + sy) + sz) + src));
             });

@@ -112,10 +112,10 @@ def test_gpu_matches_oracle_65(method, surface):
 
 @pytest.mark.parametrize("method", ["adi", "lod-ie", "lod-cn", "ts"])
 def test_every_sweep_shape_gives_the_oracle_bits(method):
-    """Every compiled sweep shape (chunk rows, ring depth, threads per CTA)
-    takes different fast and slow paths through a line; all must give the
-    oracle's bits.  Line lengths 67/61/70 are not multiples of the chunk rows,
-    so every line ends inside a partial chunk."""
+    """Every compiled sweep shape (tiles: lines per tile, threads per CTA; rings:
+    chunk rows, ring depth, threads per CTA) takes different paths through a
+    line; all must give the oracle's bits.  Line lengths 67/61/70 and the line
+    counts between them are multiples of no tile, task or chunk."""
     n = (67, 61, 70)
     spec = M.Spec(n=n, surface="torus", surface_params=(0.5, 0.2), beta_in=1.0, beta_out=1000.0, method=method,
                   mib=2, dt=2.0 / 64)

@@ -268,16 +268,17 @@ mts_status mts_set_profiling(mts_handle h, int32_t on);
 mts_status mts_profile_read(mts_handle h, double ms[8], int64_t launches[8]);
 
 /* Launch shape of the line-sweep kernels (tiles: lines per tile, threads per
- * CTA; then rings: rows per chunk, chunks, threads per CTA), chosen separately for the first, second and third implicit sweep of a step
- * (x, y, z; for TS z, y, x); a shape is refused where its tile does not hold
- * the lines of that sweep's direction.  The ring sweeps' data (16 bytes a node
- * and direction and a scratch of up to 0.53 MB per row of the longest line) is
- * allocated with the first plain step that takes one; where there is no memory
- * for it the tiles take the sweep.  Every shape computes the same bits;
- * they differ only in speed.  mts_autotune times each compiled shape on
- * the handle's own problem for `steps` steps (the solution and time are
- * restored afterwards) and keeps the fastest per sweep; shapes[3] receives
- * the choice.  mts_sweep_shape_count gives the number of shapes. */
+ * CTA; then rings: rows per chunk, chunks, threads per CTA), chosen
+ * separately for the first, second and third implicit sweep of a step (x, y,
+ * z; for TS z, y, x); a shape is refused where its tile does not hold the
+ * lines of that sweep's direction.  Every shape computes the same bits; they
+ * differ only in speed.  The ring sweeps' data (16 bytes a node and direction
+ * and a scratch of up to 0.53 MB per row of the longest line) is allocated
+ * with the first plain step that takes one; where there is no memory for it
+ * the tiles take the sweep.  mts_autotune times each compiled shape on the
+ * handle's own problem for `steps` steps after an unmeasured one (the solution
+ * and time are restored afterwards) and keeps the fastest per sweep; shapes[3]
+ * receives the choice.  mts_sweep_shape_count gives the number of shapes. */
 int32_t mts_sweep_shape_count(void);
 mts_status mts_set_sweep_shape(mts_handle h, int32_t sweep, int32_t shape);
 mts_status mts_autotune(mts_handle h, int32_t steps, int32_t shapes[3]);

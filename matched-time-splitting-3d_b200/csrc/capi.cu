@@ -1727,11 +1727,17 @@ mts_status mts_autotune(mts_handle h, int32_t steps, int32_t shapes[3]) {
     for (int k = 0; k < 3; k++) {
       const int d = mts::sweep_direction(h->prm.method, k);
       fits[k] = mts::sweep_shape_fits(s, d, nd[d]);
-      if (fits[k]) CUDA_TRY(allow_sweep(h, k, s));
+      const cudaError_t e = fits[k] ? allow_sweep(h, k, s) : cudaSuccess;
+      if (e != cudaSuccess) st = fail(MTS_ERR_CUDA, std::string("shared-memory limit: ") + cudaGetErrorString(e));
       h->dev.shape[k] = fits[k] ? s : choice0[k];
     }
+    if (st) break;
     if (!fits[0] && !fits[1] && !fits[2]) continue;
     h->ring_refused = false;
+    // one step unmeasured: the first on a device at rest took 1.1 times as
+    // long, and another shape than the fastest was kept
+    st = advance(h, 1);
+    if (st) break;
     st = mts_profile_read(h, nullptr, nullptr);
     if (st) break;
     st = advance(h, steps);

@@ -10,6 +10,7 @@ import pytest
 
 import mts_b200 as M
 import oracle as O
+from mts_b200 import workloads
 
 
 def _fma(a, b, c):
@@ -257,6 +258,7 @@ def test_grids_of_very_many_lines_take_rings_and_give_the_oracle_bits(method):
         s.initialize()
         assert _ring_default(s)
         many = s.device_bytes()
+        assert many <= workloads.device_bytes_bound(spec, sum(s.counts()["crossings"]))
         s.autotune(1)
         assert s.device_bytes() <= many + 16 * 3 * spec.nodes * 2  # what the kept shapes do not use is given back
     with M.Solver(M.Spec(n=(33, 33, 33), method=method)) as s:
@@ -266,3 +268,53 @@ def test_grids_of_very_many_lines_take_rings_and_give_the_oracle_bits(method):
         shapes = s.autotune(1)
         assert max(shapes) >= 10 or s.device_bytes() == held
     _check(spec, None, 2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("method", ["adi", "ts"])
+def test_a_problem_on_rings_steps_by_itself_in_a_batch(method):
+    specs = [M.Spec(n=(389, 18, 397), method=method, mib=1, beta_out=37.5, dt=0.01, setup="device", **ELL),
+             M.Spec(n=(25, 33, 17), method=method, mib=2, dt=0.05, **ELL)]
+    solvers = [M.Solver(sp) for sp in specs]
+    try:
+        for s in solvers:
+            s.initialize()
+        held = solvers[0].device_bytes()
+        M.batch_advance_steps(solvers, [2, 3])
+        assert solvers[0].device_bytes() > held
+        for sp, s, k in zip(specs, solvers, (2, 3)):
+            _, want = _oracle(sp, None, k)
+            assert _same(s.solution(), want)
+    finally:
+        for s in solvers:
+            s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("method", ["adi", "lod-cn", "ts"])
+def test_a_captured_step_without_ring_data_takes_the_tiles(method):
+    """Ring shapes whose data is not there and cannot be allocated (the stream
+    is being captured): the tiles take the sweeps, with the same bits; the next
+    step outside builds the data and takes the rings."""
+    import torch
+
+    spec = M.Spec(n=(45, 38, 51), method=method, mib=2, beta_out=37.5, dt=0.03, **ELL)
+    u, want = _oracle(spec, None, 1)
+    with M.Solver(spec) as s:
+        for k in range(3):
+            s.set_sweep_shape(k, 10 + k)
+        s.set_solution(u)
+        s.synchronize()
+        held = s.device_bytes()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=torch.cuda.ExternalStream(s.stream()), capture_error_mode="relaxed"):
+            s.advance(1)
+        assert s.device_bytes() == held
+        graph.replay()
+        torch.cuda.synchronize()
+        assert _same(s.solution(), want)
+        s.time = spec.t0
+        s.set_solution(u)
+        s.advance(1)
+        assert s.device_bytes() > held
+        assert _same(s.solution(), want)

@@ -1230,23 +1230,25 @@ int tile_shape_default(int d, int n, bool adi_x) {
 // has threads, whatever their length, but waits for global memory on every
 // step of it and fills an SM with few lines poorly: it pays where an SM has
 // much to do (w: nodes per SM) in long lines, or very many short ones.  The
-// lines lie where the two measured equal (B200, 53 grids of 17 to 1600 rows an
+// lines lie where the two measured equal (B200, 70 grids of 17 to 1600 rows an
 // axis); us per sweep, tiles / ring:
 //   x, LOD-IE                 353^3 465 / 508, 385^3 727 / 620, 449^3 1139 / 955
 //   x, Douglas-ADI, with its first right-hand side (a pass of its own before a
-//   ring)                     321^3 500 / 553, 385^3 922 / 913, 449^3 1468 / 1414
+//   ring)                     321^3 500 / 553, 385 x 298 x 384 689 / 744, 449^3 1468 / 1414
 //   y, z                      ADI y 225^3 142 / 136, 257^3 197 / 190, 385^3 738 / 515;
 //                             LOD-IE y (copied) 249^3 142 / 155, 273^3 201 / 190
 //   z of LOD (adds the source on the way out, row by row in a ring)
-//                             LOD-CN 321^3 429 / 529, 353^3 652 / 593, 385^3 878 / 815
+//                             LOD-CN 345 x 254 x 352 468 / 548, 353^3 652 / 593, 385^3 878
+//                             / 815, 220 x 260 x 640 770 / 642
 //   33 x 700 x 700 x, TS      209 / 169; 500 x 33 x 500 y, ADI 115 / 98
 int sweep_shape_default(int method, int d, int n, long long lines, int sms) {
   const double per_sm = (double)lines / sms, w = per_sm * n;
   bool ring;
   if (d == 0)
-    ring = (n >= 360 && w >= 110e3) || (method != MTS_ADI && n <= 50 && per_sm >= 1500);
+    ring = (n >= (method == MTS_ADI ? 420 : 360) && w >= 110e3) ||
+           (method != MTS_ADI && n <= 50 && per_sm >= 1500);
   else if (d == 2 && (method == MTS_LOD_IE || method == MTS_LOD_CN))
-    ring = (n >= 340 && w >= 180e3) || (n <= 50 && per_sm >= 1500);
+    ring = (n >= 340 && w >= 280e3) || (n >= 600 && w >= 210e3) || (n <= 50 && per_sm >= 1500);
   else if (method == MTS_LOD_IE || (method == MTS_TS && d == 1))
     ring = (n >= 150 && w >= 110e3) || (n <= 82 && per_sm >= 1000);
   else

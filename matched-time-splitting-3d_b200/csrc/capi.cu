@@ -85,7 +85,8 @@ struct mts_problem {
   bool fast_built = false;
   bool mixed_built = false;
   // the ring sweeps' data (ensure_rings): a block per direction, the d'
-  // scratch and its size
+  // scratch, and their sizes
+  mts::RingData ring{};
   void* ring_mem[4] = {nullptr, nullptr, nullptr, nullptr};
   size_t ring_bytes[4] = {0, 0, 0, 0};
   bool ring_refused = false;  // no memory for them: the tiles take those sweeps
@@ -306,10 +307,10 @@ void release_ring(mts_problem* h, int i) {
   h->ring_mem[i] = nullptr;
   h->ring_bytes[i] = 0;
   if (i == 3) {
-    h->dev.dp = nullptr;
+    h->ring.dp = nullptr;
   } else {
-    h->dev.fbet[i] = h->dev.fgam[i] = nullptr;
-    h->dev.rblk[i] = nullptr;
+    h->ring.fbet[i] = h->ring.fgam[i] = nullptr;
+    h->ring.rblk[i] = nullptr;
   }
 }
 
@@ -320,7 +321,8 @@ void release_ring(mts_problem* h, int i) {
 // for them (or the stream is being captured, where memory would be the
 // graph's) the tiles take the sweep (kernels.cu).
 cudaError_t ensure_rings(mts_problem* h) {
-  mts::Dev& D = h->dev;
+  const mts::Dev& D = h->dev;
+  mts::RingData& R = h->ring;
   const int nd[3] = {D.nx, D.ny, D.nz};
   size_t dp = 0;
   bool need[3] = {false, false, false};
@@ -332,7 +334,7 @@ cudaError_t ensure_rings(mts_problem* h) {
                           (size_t)mts::ring_threads(D, D.shape[k] - mts::kTileShapes, d));
   }
   bool missing = dp > h->ring_bytes[3];
-  for (int d = 0; d < 3; d++) missing = missing || (need[d] && !D.rblk[d]);
+  for (int d = 0; d < 3; d++) missing = missing || (need[d] && !R.rblk[d]);
   if (!missing || h->ring_refused) return cudaSuccess;
   cudaStreamCaptureStatus cap;
   cudaError_t e = cudaStreamIsCapturing(h->stream, &cap);
@@ -349,19 +351,19 @@ cudaError_t ensure_rings(mts_problem* h) {
   if (dp > h->ring_bytes[3]) {
     release_ring(h, 3);
     ok = block(3, dp);
-    if (ok) D.dp = (double*)h->ring_mem[3];
+    if (ok) R.dp = (double*)h->ring_mem[3];
   }
   const size_t field = (size_t)(D.nn + (long long)mts::kRowPad * D.nx * D.ny);
   for (int d = 0; d < 3 && ok; d++) {
-    if (!need[d] || D.rblk[d]) continue;
+    if (!need[d] || R.rblk[d]) continue;
     const size_t f = D.nblk[d] > 0 ? field : 0;
     ok = block(d, sizeof(double) * (2 * f + 3 * (size_t)D.nblk[d] + 1));
     if (!ok) break;
     double* const p = (double*)h->ring_mem[d];
     if (f) mts::build_ring_factors(D, d, p, p + f, h->stream);
-    D.fbet[d] = p;
-    D.fgam[d] = p + f;
-    D.rblk[d] = p + 2 * f;
+    R.fbet[d] = p;
+    R.fgam[d] = p + f;
+    R.rblk[d] = p + 2 * f;
   }
   if (!ok) {
     for (int i = 0; i < 4; i++) release_ring(h, i);
@@ -895,7 +897,7 @@ mts_status enqueue_step(mts_problem* h, double t_prev, double t_half, double t_n
     h->launches += mts::launch_step_mixed(h->dev, T, h->u0, h->stream, ev, &h->side);
   else {
     CUDA_TRY(ensure_rings(h));
-    h->launches += mts::launch_step(h->dev, T, h->u0, h->u1, h->stream, ev, &h->side);
+    h->launches += mts::launch_step(h->dev, h->ring, T, h->u0, h->u1, h->stream, ev, &h->side);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(MTS_ERR_CUDA, std::string("step launch: ") + cudaGetErrorString(e));
@@ -1300,7 +1302,7 @@ mts_status mts_batch_advance_steps(const mts_handle* hs, const int32_t* counts, 
       else if (h->dev.precision == 1)
         h->launches += mts::launch_step_mixed(h->dev, T, h->u0, h->stream, nullptr, &h->side);
       else
-        h->launches += mts::launch_step(h->dev, T, h->u0, h->u1, h->stream, nullptr, &h->side);
+        h->launches += mts::launch_step(h->dev, h->ring, T, h->u0, h->u1, h->stream, nullptr, &h->side);
       mts::launch_tick(h->dev, h->stream);
       h->launches++;
     }
@@ -1751,7 +1753,7 @@ mts_status mts_autotune(mts_handle h, int32_t steps, int32_t shapes[3]) {
       // an x ring sweep it has the slot before)
       const double t = ms[first + k] + (k == 0 && h->prm.method == MTS_ADI ? ms[first - 1] : 0.0);
       const int d = mts::sweep_direction(h->prm.method, k);
-      if (fits[k] && (s < mts::kTileShapes || h->dev.rblk[d]) && t < best[k]) {
+      if (fits[k] && (s < mts::kTileShapes || h->ring.rblk[d]) && t < best[k]) {
         best[k] = t;
         choice[k] = s;
       }

@@ -96,15 +96,6 @@ struct Dev {
   const double* ca[3];
   const double2* cb[3];
   const double* cg[3];
-  // The ring sweeps' data (ring.cu), built before a handle's first step that
-  // takes one, for the directions that do (null before): by node bet_j and
-  // gam_j of the crossing lines from their first MIB row on; the block rows'
-  // right-hand sides of the sweep in flight, [3*block + q]; the partial
-  // solutions d'_j, [row][thread].
-  const double* fbet[3];
-  const double* fgam[3];
-  double* rblk[3];
-  double* dp;
   int plain_div;     // a factor is out of the range of the quotients from reciprocals (kernels.cu)
   int nblk[3];
   int sweep_blocks;  // SMs
@@ -157,6 +148,19 @@ struct Dev {
   int* status;       // reserved
 };
 
+// The ring sweeps' data (ring.cu), built before a handle's first step that takes
+// one, for the directions that do (null before): by node bet_j and gam_j of the
+// crossing lines from their first MIB row on; the block rows' right-hand sides
+// of the sweep in flight, [3*block + q]; the partial solutions d'_j,
+// [row][thread].  (Apart from Dev, which every launch carries: its 80 bytes
+// cost a 33^3 step's four launches 1.9 us of host time, 9.6 against 7.7.)
+struct RingData {
+  const double* fbet[3];
+  const double* fgam[3];
+  double* rblk[3];
+  double* dp;
+};
+
 // What a bit-exact line sweep does: its right-hand side (of the copied field,
 // of the line's explicit stencil, of TS's z step, or the whole first
 // right-hand side of Douglas-ADI) and its fields.
@@ -190,11 +194,11 @@ cudaError_t configure_shape(int shape);
 // The ring sweeps (ring.cu; ring: shape - kTileShapes).
 bool ring_fits(int ring, int n);
 int ring_default(int method, int d, int n, double per_sm);  // lines per SM; -1: none fits
-long long ring_threads(const Dev& P, int ring, int d);  // threads of the launch: columns of Dev::dp
+long long ring_threads(const Dev& P, int ring, int d);  // threads of the launch: columns of dp
 cudaError_t configure_ring(int ring);
 void build_ring_factors(const Dev& P, int d, double* fbet, double* fgam, cudaStream_t stream);
 void launch_adi_rhs(const Dev& P, const double* u, double* r, double e_next, cudaStream_t stream);
-void launch_ring_sweep(const Dev& P, int d, int kind, const SweepIO& io, int ring, cudaStream_t stream);
+void launch_ring_sweep(const Dev& P, const RingData& R, int d, int kind, const SweepIO& io, int ring, cudaStream_t stream);
 
 // Per-step exact-solution time factors.
 struct StepTimes {
@@ -215,8 +219,8 @@ struct SideStream {
   cudaStream_t stream;
   cudaEvent_t fork, join;
 };
-int launch_step(const Dev& P, const StepTimes& T, double* u0, double* u1, cudaStream_t stream, cudaEvent_t* ev,
-                const SideStream* side);
+int launch_step(const Dev& P, const RingData& R, const StepTimes& T, double* u0, double* u1, cudaStream_t stream,
+                cudaEvent_t* ev, const SideStream* side);
 // The mixed-precision Douglas-ADI step (mixed.cu), in place on u.
 int launch_step_mixed(const Dev& P, const StepTimes& T, double* u, cudaStream_t stream, cudaEvent_t* ev,
                       const SideStream* side);

@@ -1156,7 +1156,7 @@ void sweep_shape(const Dev& P, const SweepIO& io, cudaStream_t st) {
 
 // One sweep in the shape selected for it (Dev::shape).
 template <int D, int KIND>
-void sweep(const Dev& P, const SweepIO& io, int shape, cudaStream_t st) {
+void sweep(const Dev& P, const RingData& R, const SweepIO& io, int shape, cudaStream_t st) {
   switch (shape) {
 #define MTS_CASE(id, nl, nt)                    \
   case id:                                      \
@@ -1166,10 +1166,10 @@ void sweep(const Dev& P, const SweepIO& io, int shape, cudaStream_t st) {
 #undef MTS_CASE
     default:
       // a ring, where its data could be built
-      if (KIND != K_ADI && P.rblk[D])
-        launch_ring_sweep(P, D, KIND, io, shape - kTileShapes, st);
+      if (KIND != K_ADI && R.rblk[D])
+        launch_ring_sweep(P, R, D, KIND, io, shape - kTileShapes, st);
       else
-        sweep<D, KIND>(P, io, tile_shape_default(D, D == 0 ? P.nx : D == 1 ? P.ny : P.nz, KIND == K_ADI), st);
+        sweep<D, KIND>(P, R, io, tile_shape_default(D, D == 0 ? P.nx : D == 1 ? P.ny : P.nz, KIND == K_ADI), st);
   }
 }
 
@@ -1315,8 +1315,8 @@ int launch_norms(const Dev& P, double E, const double* u, double* partial, int n
 }
 
 // One time step.  u0 holds u^n on entry and u^{n+1} on return; u1 is scratch.
-int launch_step(const Dev& P, const StepTimes& T, double* u0, double* u1, cudaStream_t st, cudaEvent_t* ev,
-                const SideStream* side) {
+int launch_step(const Dev& P, const RingData& R, const StepTimes& T, double* u0, double* u1, cudaStream_t st,
+                cudaEvent_t* ev, const SideStream* side) {
   int launches = 0;
   int slot = 0;
   auto mark = [&](int k) {
@@ -1338,7 +1338,7 @@ int launch_step(const Dev& P, const StepTimes& T, double* u0, double* u1, cudaSt
     // is scratch.  Before an x ring sweep uhs is formed in u1 by passes of its
     // own, the MIB rows on the side stream beside the others (they write
     // disjoint nodes and read only u0).
-    const bool ring_x = P.shape[0] >= kTileShapes && P.rblk[0];
+    const bool ring_x = P.shape[0] >= kTileShapes && R.rblk[0];
     const bool fork = ring_x && side && side->stream && P.nmibnode > 0;
     cudaStream_t sst = fork ? side->stream : st;
     mark(0);
@@ -1369,22 +1369,22 @@ int launch_step(const Dev& P, const StepTimes& T, double* u0, double* u1, cudaSt
       io.stin = u1;
       io.add = u1;
       io.bmode = 0;
-      sweep<0, K_COPY>(P, io, P.shape[0], st);
+      sweep<0, K_COPY>(P, R, io, P.shape[0], st);
       io.stin = u0;
     } else {
-      sweep<0, K_ADI>(P, io, P.shape[0], st);
+      sweep<0, K_ADI>(P, R, io, P.shape[0], st);
     }
     mark(1);
     io.add = u1;
     io.bmode = 0;
     io.k = -P.dt;
     mark(0);
-    sweep<1, K_STENCIL>(P, io, P.shape[1], st);
+    sweep<1, K_STENCIL>(P, R, io, P.shape[1], st);
     mark(1);
     io.out = u0;
     io.bmode = 1;
     mark(0);
-    sweep<2, K_STENCIL>(P, io, P.shape[2], st);
+    sweep<2, K_STENCIL>(P, R, io, P.shape[2], st);
     mark(1);
     launches += 3;
   } else if (P.method == 1 || P.method == 2) {
@@ -1397,23 +1397,23 @@ int launch_step(const Dev& P, const StepTimes& T, double* u0, double* u1, cudaSt
     io.bmode = 1;
     mark(0);
     if (P.method == 2)
-      sweep<0, K_STENCIL>(P, io, P.shape[0], st);
+      sweep<0, K_STENCIL>(P, R, io, P.shape[0], st);
     else
-      sweep<0, K_COPY>(P, io, P.shape[0], st);
+      sweep<0, K_COPY>(P, R, io, P.shape[0], st);
     mark(1);
     mark(0);
     if (P.method == 2)
-      sweep<1, K_STENCIL>(P, io, P.shape[1], st);
+      sweep<1, K_STENCIL>(P, R, io, P.shape[1], st);
     else
-      sweep<1, K_COPY>(P, io, P.shape[1], st);
+      sweep<1, K_COPY>(P, R, io, P.shape[1], st);
     mark(1);
     io.last = 1;
     io.bmode = 2;
     mark(0);
     if (P.method == 2)
-      sweep<2, K_STENCIL>(P, io, P.shape[2], st);
+      sweep<2, K_STENCIL>(P, R, io, P.shape[2], st);
     else
-      sweep<2, K_COPY>(P, io, P.shape[2], st);
+      sweep<2, K_COPY>(P, R, io, P.shape[2], st);
     mark(1);
     launches += 3;
   } else {
@@ -1433,14 +1433,14 @@ int launch_step(const Dev& P, const StepTimes& T, double* u0, double* u1, cudaSt
     io.out = u0;
     io.bmode = 1;
     mark(0);
-    sweep<2, K_TS_Z>(P, io, P.shape[0], st);
+    sweep<2, K_TS_Z>(P, R, io, P.shape[0], st);
     mark(1);
     io.bmode = 0;
     mark(0);
-    sweep<1, K_COPY>(P, io, P.shape[1], st);
+    sweep<1, K_COPY>(P, R, io, P.shape[1], st);
     mark(1);
     mark(0);
-    sweep<0, K_COPY>(P, io, P.shape[2], st);
+    sweep<0, K_COPY>(P, R, io, P.shape[2], st);
     mark(1);
     launches += 5;
   }

@@ -160,7 +160,7 @@ __device__ __forceinline__ void load_head(const MibBlock* blk, const double* rbl
 // Block pre-pass of a sweep: one thread per MIB block of direction D computes
 // the right-hand sides of the block's rows and stores them for the sweep.
 template <int D, int KIND>
-__global__ void __launch_bounds__(TPB) k_block_rhs(const __grid_constant__ Dev P, const SweepIO io) {
+__global__ void __launch_bounds__(TPB) k_block_rhs(const __grid_constant__ Dev P, const SweepIO io, double* rblk) {
   const int k = blockIdx.x * TPB + threadIdx.x;
   if (k >= P.nblk[D]) return;
   const int n2 = D == 2 ? P.ny : P.nz;
@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(TPB) k_block_rhs(const __grid_constant__ Dev P
   decode_line<D>(P, (long long)(line % n2) * (D == 0 ? P.ny : P.nx) + line / n2, L);
   double r[3];
   block_rhs<D, KIND>(P, io, step_e(P, io.e0, 0), step_e(P, io.e1, 2), k, L.base, L.i1, L.i2, r);
-  for (int q = 0; q < 3; q++) P.rblk[D][3 * k + q] = r[q];
+  for (int q = 0; q < 3; q++) rblk[3 * k + q] = r[q];
 }
 
 // Exact-solution parts along a line: the fixed axes are read once per line,
@@ -231,7 +231,8 @@ constexpr size_t ring_smem(int n) {
 
 
 template <int D, int KIND, int CH, int NS, int NT>
-__global__ void __launch_bounds__(NT, 1) k_sweep(const __grid_constant__ Dev P, const SweepIO io) {
+__global__ void __launch_bounds__(NT, 1) k_sweep(const __grid_constant__ Dev P, const __grid_constant__ RingData R,
+                                                 const SweepIO io) {
   static_assert((CH & (CH - 1)) == 0 && (NS & (NS - 1)) == 0 && NS >= 4 && CH >= 4, "shape");
   static_assert(CH <= kRowPad, "chunk rows past a line end must stay within the fields' slack");
   constexpr int RING = NS * CH;    // rows in a field's ring
@@ -250,12 +251,12 @@ __global__ void __launch_bounds__(NT, 1) k_sweep(const __grid_constant__ Dev P, 
 #define SC(j) sC[((j) & (RING - 1)) * RS]
   const long long T = (long long)gridDim.x * NT;
   const long long gt = (long long)blockIdx.x * NT + tid;
-  double* const dp = P.dp + gt;
+  double* const dp = R.dp + gt;
   const long long nl = nlines<D>(P);
   const MibBlock* __restrict__ blk = P.blk[D];
-  const double* __restrict__ fbet = P.fbet[D];
-  const double* __restrict__ fgam = P.fgam[D];
-  const double* __restrict__ rblk = P.rblk[D];
+  const double* __restrict__ fbet = R.fbet[D];
+  const double* __restrict__ fgam = R.fgam[D];
+  const double* __restrict__ rblk = R.rblk[D];
   const double E1 = step_e(P, io.e1, 2);
   const double E0 = step_e(P, io.e0, 0);
   const double kx = io.k;
@@ -651,13 +652,13 @@ __global__ void __launch_bounds__(TPB) k_ring_factors(const __grid_constant__ De
 #define MTS_RINGS(X) X(0, 4, 4, 384) X(1, 4, 4, 448) X(2, 4, 4, 128)
 
 template <int D, int KIND>
-void sweep(const Dev& P, const SweepIO& io, int ring, cudaStream_t st) {
+void sweep(const Dev& P, const RingData& R, const SweepIO& io, int ring, cudaStream_t st) {
   const int nd = D == 0 ? P.nx : D == 1 ? P.ny : P.nz;
-  if (P.nblk[D] > 0) k_block_rhs<D, KIND><<<(P.nblk[D] + TPB - 1) / TPB, TPB, 0, st>>>(P, io);
+  if (P.nblk[D] > 0) k_block_rhs<D, KIND><<<(P.nblk[D] + TPB - 1) / TPB, TPB, 0, st>>>(P, io, R.rblk[D]);
   switch (ring) {
 #define MTS_CASE(id, ch, ns, nt)                                                                               \
   case id:                                                                                                     \
-    k_sweep<D, KIND, ch, ns, nt><<<sweep_grid(P, nlines<D>(P), nt), nt, ring_smem<ch, ns, nt, D>(nd), st>>>(P, io); \
+    k_sweep<D, KIND, ch, ns, nt><<<sweep_grid(P, nlines<D>(P), nt), nt, ring_smem<ch, ns, nt, D>(nd), st>>>(P, R, io); \
     break;
     MTS_RINGS(MTS_CASE)
 #undef MTS_CASE
@@ -738,24 +739,24 @@ void launch_adi_rhs(const Dev& P, const double* u, double* r, double e_next, cud
   k_adi_rhs<2><<<pointwise_rows_grid(P), TPB, 0, st>>>(P, u, r, e_next);
 }
 
-void launch_ring_sweep(const Dev& P, int d, int kind, const SweepIO& io, int ring, cudaStream_t st) {
+void launch_ring_sweep(const Dev& P, const RingData& R, int d, int kind, const SweepIO& io, int ring, cudaStream_t st) {
   if (d == 0) {
     if (kind == K_COPY)
-      sweep<0, K_COPY>(P, io, ring, st);
+      sweep<0, K_COPY>(P, R, io, ring, st);
     else
-      sweep<0, K_STENCIL>(P, io, ring, st);
+      sweep<0, K_STENCIL>(P, R, io, ring, st);
   } else if (d == 1) {
     if (kind == K_COPY)
-      sweep<1, K_COPY>(P, io, ring, st);
+      sweep<1, K_COPY>(P, R, io, ring, st);
     else
-      sweep<1, K_STENCIL>(P, io, ring, st);
+      sweep<1, K_STENCIL>(P, R, io, ring, st);
   } else {
     if (kind == K_COPY)
-      sweep<2, K_COPY>(P, io, ring, st);
+      sweep<2, K_COPY>(P, R, io, ring, st);
     else if (kind == K_TS_Z)
-      sweep<2, K_TS_Z>(P, io, ring, st);
+      sweep<2, K_TS_Z>(P, R, io, ring, st);
     else
-      sweep<2, K_STENCIL>(P, io, ring, st);
+      sweep<2, K_STENCIL>(P, R, io, ring, st);
   }
 }
 
